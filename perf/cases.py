@@ -165,6 +165,9 @@ def _zipf(rows, groups, rg, nulls, seed):
     code = r.perm(groups)[rank]
     once = r.perm(rows)[:groups]  # every group has a row
     code[once] = torch.arange(groups, device="cuda")
+    # codes in first-occurrence order, as the writer gives them out
+    first = torch.full((groups,), rows, device="cuda").scatter_reduce_(0, code, torch.arange(rows, device="cuda"), "amin")
+    code = torch.argsort(torch.argsort(first))[code]
     val = (r.uniform(rows) * 1e7).round_() / 100.0
     vk = vv = None
     if nulls:
