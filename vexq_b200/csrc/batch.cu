@@ -6,9 +6,11 @@
 // holds a body per distinct plan shape: blocks take (plan, chunk range) units
 // from an atomic ticket, largest units first, so uneven plans share the GPU
 // without one launch each. Table init, the class launches (on two forked
-// streams), the partial merge and the table finalize are captured once in a
-// CUDA graph and replayed by each execution, followed by one copy of every
-// output back to pinned host memory. The autotuner picks the shared-memory group
+// streams), the partial merge, the table finalize and the assembly of result
+// columns on the device (assemble.cu: one cluster per table, written straight
+// into a pinned block) are captured once in a CUDA graph and replayed by each
+// execution, followed by one copy of the remaining outputs (register-path
+// rows, joins' groups, error words) back to pinned host memory. The autotuner picks the shared-memory group
 // cache size (the shared-versus-global table cutover), the unit size and the
 // block shape of each class by timing graph replays, and keeps its choice in a
 // JSON file keyed by the batch's shape. A join whose build key range allows a
@@ -28,8 +30,8 @@
 #include <sstream>
 #include <thread>
 
+#include "assemble.h"
 #include "internal.h"
-#include "plan.h"
 
 namespace vq {
 __global__ void k_init_batch(const VQTableDesc* d, int n, long long total);
@@ -61,6 +63,12 @@ struct Item {
     size_t a_keys = 0, a_first = 0, a_acc_i = 0, a_acc_fx = 0, a_special = 0, a_init = 0, a_lsb = 0, a_ngroups = 0;
     size_t o_nout = 0, o_err = 0, o_key = 0, o_first = 0, o_i = 0, o_f = 0;
     size_t a_seg = 0;
+    // group table assembled on the device: its columns' layout, scratch and
+    // place in the output block
+    bool assemble = false;
+    AsmLayout al;
+    size_t a_bits = 0, a_asm = 0, a_acols = 0, o_asm = 0;
+    long long row0 = 0, row1 = 0;
     // join (direct-mapped build): the build side's row ranges, its work units
     // in the build class, its parameter block (bparams[bix]), the key table,
     // the number → key array (GROUP BY the join key) and the build's counts
@@ -96,6 +104,14 @@ struct Batch {
     int njoins = 0;
     int n_tdesc = 0, n_mdesc = 0, merge_entries = 0;
     long long table_slots = 0;
+    // tables finalized by compaction come first among the descriptors
+    int n_fdesc = 0, n_adesc = 0;
+    long long fin_slots = 0;
+    size_t a_adesc = 0, a_outp = 0, asm_bytes = 0;
+    OutPool pool;
+    std::shared_ptr<OutBlock> blk;  // the current execution's block of assembled columns
+    bool blk_lend = true;
+    char* blk_sent = nullptr;       // its device address as last uploaded
     cudaStream_t s = nullptr, s2 = nullptr;
     cudaEvent_t ev[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};  // [4]: kernels done (before the copy back)
     cudaGraph_t graph = nullptr;
@@ -152,8 +168,15 @@ struct Batch {
         a_tdesc = take(n_tdesc * sizeof(VQTableDesc));
         a_mdesc = take(n_mdesc * sizeof(VQMergeDesc));
         a_ticket = take(16);
+        n_adesc = 0;
+        for (int i : ck[1].items) n_adesc += items[i].assemble;
+        n_fdesc = n_tdesc - n_adesc;
+        a_adesc = take(n_adesc * sizeof(VQAsmDesc));
+        a_outp = take(8);
+        blk_sent = nullptr;
+        asm_bytes = 0;
         o_aerr = otake(8);
-        table_slots = 0;
+        table_slots = fin_slots = 0;
         merge_entries = 0;
         // uploaded pieces first, then device scratch (partials, tables)
         for (Item& it : items) {
@@ -165,6 +188,7 @@ struct Batch {
             } else {
                 it.a_init = take((size_t)it.ni * 8);
                 it.a_lsb = take((size_t)std::max(it.nf, 1) * 4);
+                if (it.assemble) it.a_acols = take(it.al.cols.size() * sizeof(VQAsmCol));
             }
         }
         const size_t upload = off;
@@ -192,10 +216,19 @@ struct Batch {
                 it.a_ngroups = take(8);
                 it.o_nout = otake(8);
                 it.o_err = otake(8);
-                it.o_key = otake(it.cap_out * 8);
-                it.o_first = otake(it.cap_out * 8);
-                it.o_i = otake((size_t)it.ni * it.cap_out * 8);
-                it.o_f = otake((size_t)it.nf * it.cap_out * 8);
+                if (it.assemble) {
+                    VQAsmDesc d;
+                    it.a_bits = take(asm_span(*it.p, it.row0, it.row1, d));
+                    it.a_asm = take(asm_scratch(d, ns, nullptr));
+                    it.o_asm = asm_bytes;
+                    asm_bytes += al(it.al.bytes);
+                } else {
+                    it.o_key = otake(it.cap_out * 8);
+                    it.o_first = otake(it.cap_out * 8);
+                    it.o_i = otake((size_t)it.ni * it.cap_out * 8);
+                    it.o_f = otake((size_t)it.nf * it.cap_out * 8);
+                    fin_slots += ns;
+                }
                 table_slots += ns;
             }
         }
@@ -208,12 +241,14 @@ struct Batch {
         // host images of the uploaded part
         std::vector<VQParams> params(items.size()), bparams((size_t)std::max(njoins, 1));
         std::vector<VQUnit> units[3];
-        std::vector<VQTableDesc> td;
+        std::vector<VQTableDesc> td((size_t)n_tdesc);
+        std::vector<VQAsmDesc> ad;
         std::vector<VQMergeDesc> md;
         std::vector<char> blob(upload, 0);
         auto put = [&](size_t at, const void* src, size_t n) { if (n) std::memcpy(blob.data() + at, src, n); };
         int e0 = 0;
-        long long slot0 = 0;
+        long long slot_fin = 0, slot_asm = fin_slots;  // first global slots: compacted tables, then assembled ones
+        int at_fin = 0, at_asm = n_fdesc;
         for (size_t ix = 0; ix < items.size(); ix++) {
             Item& it = items[ix];
             if (it.cls == 2) continue;
@@ -327,9 +362,35 @@ struct Batch {
                 t.o_i = (long long*)(O + it.o_i);
                 t.o_f = (double*)(O + it.o_f);
                 t.cap_out = it.cap_out;
+                long long& slot0 = it.assemble ? slot_asm : slot_fin;
                 t.slot0 = slot0;
                 slot0 += it.nslots;
-                td.push_back(t);
+                if (it.assemble) {
+                    t.o_key = nullptr;
+                    t.o_first = nullptr;
+                    t.o_i = nullptr;
+                    t.o_f = nullptr;
+                    VQAsmDesc d;
+                    std::memset(&d, 0, sizeof d);
+                    asm_span(p, it.row0, it.row1, d);
+                    d.bits = (unsigned*)(D + it.a_bits);
+                    asm_scratch(d, it.nslots, D + it.a_asm);
+                    d.keys = P.keys;
+                    d.first = P.first;
+                    d.acc_i = P.acc_i;
+                    d.acc_fx = P.acc_fx;
+                    d.special = P.special;
+                    d.fx_lsb = t.fx_lsb;
+                    d.error = P.error;
+                    d.cols = (const VQAsmCol*)(D + it.a_acols);
+                    d.nslots = it.nslots;
+                    d.ncols = (int)it.al.cols.size();
+                    d.write = 1;  // the batch's tables fill the GPU together
+                    d.out = (long long)it.o_asm;
+                    put(it.a_acols, it.al.cols.data(), it.al.cols.size() * sizeof(VQAsmCol));
+                    ad.push_back(d);
+                }
+                td[it.assemble ? at_asm++ : at_fin++] = t;
             }
         }
         for (int c = 0; c < 3; c++) {
@@ -355,8 +416,14 @@ struct Batch {
         put(a_params, params.data(), params.size() * sizeof(VQParams));
         put(a_bparams, bparams.data(), (size_t)njoins * sizeof(VQParams));
         put(a_tdesc, td.data(), td.size() * sizeof(VQTableDesc));
+        put(a_adesc, ad.data(), ad.size() * sizeof(VQAsmDesc));
         put(a_mdesc, md.data(), md.size() * sizeof(VQMergeDesc));
         h2d(dev.p, blob.data(), upload, s);
+        for (const Item& it : items)  // the assembly's bitmaps start clear, and each run leaves them so
+            if (it.assemble) {
+                VQAsmDesc d;
+                VQ_CUDA(cudaMemsetAsync(D + it.a_bits, 0, asm_span(*it.p, it.row0, it.row1, d), s));
+            }
         std::ostringstream ex;
         ex << "batch plans=" << items.size() << " regs_plans=" << ck[0].items.size() << " regs_bodies=" << ck[0].nbodies
            << " regs_units=" << ck[0].nunits << " table_plans=" << ck[1].items.size() << " table_bodies=" << ck[1].nbodies
@@ -420,11 +487,15 @@ struct Batch {
             jit_launch(ck[1].k, ck[1].grid, &A, sizeof A, s);
             chk(s, "vq_batch (group tables)");
         }
-        if (table_slots > 0) {
-            int g = (int)std::min<long long>((table_slots + 255) / 256, (long long)sm_count() * 16);
-            k_finalize_batch<<<g, 256, 0, s>>>((const VQTableDesc*)(D + a_tdesc), n_tdesc, table_slots);
+        if (fin_slots > 0) {
+            int g = (int)std::min<long long>((fin_slots + 255) / 256, (long long)sm_count() * 16);
+            k_finalize_batch<<<g, 256, 0, s>>>((const VQTableDesc*)(D + a_tdesc), n_fdesc, fin_slots);
             VQ_CUDA(cudaGetLastError());
             chk(s, "k_finalize_batch");
+        }
+        if (n_adesc > 0) {
+            asm_launch((const VQAsmDesc*)(D + a_adesc), n_adesc, nullptr, (char* const*)(D + a_outp), s);
+            chk(s, "k_assemble");
         }
         VQ_CUDA(cudaEventRecord(ev[3], s2));
         VQ_CUDA(cudaStreamWaitEvent(s, ev[3], 0));
@@ -462,8 +533,36 @@ struct Batch {
         return ms;
     }
 
+    // A HAVING set or removed since the layout moves its plan's table between
+    // the device assembly and the host's results.
+    void follow_having() {
+        bool changed = false;
+        for (Item& it : items) {
+            const bool now = it.cls == 1 && it.nchunks > 0 && asm_run_ok(*it.p, it.nslots, it.row0, it.row1);
+            if (now == it.assemble) continue;
+            it.assemble = now;
+            if (now) it.al = asm_layout(*it.p, it.nslots);
+            changed = true;
+        }
+        if (changed) layout();
+    }
+
+    // The block this execution's columns go to: the last one when its results
+    // are gone (its address is in device memory already), else another.
+    void take_block() {
+        if (n_adesc == 0) return;
+        blk.reset();
+        blk = pool.acquire(asm_bytes, blk_lend);
+        if (!blk) fail(VEXQ_EDEVICE, "pinned host memory has no device address");
+        if (blk->dev == blk_sent) return;
+        h2d((char*)dev.p + a_outp, &blk->dev, 8, s);
+        blk_sent = blk->dev;
+    }
+
     float replay() {
         for (const Item& it : items) check_ranges(*it.p);
+        follow_having();
+        take_block();
         if (!gexec) capture();
         VQ_CUDA(cudaEventRecord(ev[0], s));
         VQ_CUDA(cudaGraphLaunch(gexec, s));
@@ -473,6 +572,7 @@ struct Batch {
     // One execution launched directly, for plan sets that run once.
     float run_direct() {
         for (const Item& it : items) check_ranges(*it.p);
+        take_block();
         VQ_CUDA(cudaEventRecord(ev[0], s));
         enqueue();
         return finish_timing();
@@ -738,6 +838,12 @@ void build_batch(Batch* b, vexq_plan_s* const* handles, int n) {
             }
             it.nslots = it.cap + 1;
             it.cap_out = it.nslots;
+            if (!ss.seg.empty()) {
+                it.row0 = ss.seg.front();
+                it.row1 = ss.seg[ss.seg.size() - 2];
+            }
+            it.assemble = ss.nchunks > 0 && asm_run_ok(*p, it.nslots, it.row0, it.row1);
+            if (it.assemble) it.al = asm_layout(*p, it.nslots);
         }
         b->bytes += it.bytes;
         b->rows += it.rows;
@@ -800,6 +906,19 @@ static void collect(Batch& b, vexq_result_s** out) {
             }
             try {
                 Plan& p = *it.p;
+                if (it.assemble) {
+                    const char* data = (const char*)b.blk->pin.p + it.o_asm;
+                    const VQAsmHdr* h = (const VQAsmHdr*)data;
+                    if (h->err & 1) { plain[i] = 1; continue; }  // hash table overflow: rerun with growth
+                    if (h->err & 2) fail(VEXQ_ENOTSUP, "float sum exceeded its exact accumulation window");
+                    vexq_result_s* r = asm_result(p, it.al, data, (long long)h->n, b.blk_lend ? b.blk : nullptr);
+                    r->kernel_ms = b.kernel_ms;
+                    r->scan_ms = b.kernel_ms;
+                    r->rows_scanned = it.rows + it.brows;
+                    r->bytes_scanned = it.bytes;
+                    out[i] = r;
+                    continue;
+                }
                 Groups g;
                 g.ival.assign(it.ni, {});
                 g.fval.assign(it.nf, {});
@@ -848,7 +967,7 @@ static void collect(Batch& b, vexq_result_s** out) {
     };
     // host threads only pay off when there are many groups to order
     size_t groups = 0;
-    for (const Item& it : b.items) groups += it.cls == 1 ? (size_t)it.cap_out : (size_t)it.G;
+    for (const Item& it : b.items) groups += it.cls == 1 && !it.assemble ? (size_t)it.cap_out : (size_t)it.G;
     const int nt = groups < 200000 ? 1
                    : (int)std::max<size_t>(1, std::min<size_t>({n, (size_t)16, (size_t)std::max(1u, std::thread::hardware_concurrency())}));
     std::vector<std::thread> th;

@@ -96,6 +96,13 @@ struct GlobalDict {
     }
 };
 
+// A column's global dictionary as one run of bytes, shared with the results
+// that show its strings (dictionaries never change after the upload).
+struct FlatDict {
+    std::vector<uint32_t> off;  // entries + 1
+    std::string bytes;
+};
+
 struct Column {
     std::string name;
     int32_t type = 0;
@@ -104,6 +111,7 @@ struct Column {
     DevBuf validity;    // LSB-first bitmap (nullable columns only)
     // STRING
     GlobalDict dict;
+    mutable std::shared_ptr<const FlatDict> flat;  // of dict, made on first use (flat_dict)
     std::vector<std::vector<uint32_t>> rg_remap;   // per RG: local → global code
     std::vector<std::vector<uint8_t>> rg_present;  // per RG: global code present in the RG's dictionary
     bool per_rg_dicts = true;
@@ -114,6 +122,8 @@ struct Column {
     double fmin = 0, fmax = 0;      // FLOAT64
     int64_t imin = 0, imax = 0;     // INT64 / DATE
 };
+
+std::shared_ptr<const FlatDict> flat_dict(const Column& c);
 
 struct Table {
     std::vector<Column> cols;

@@ -114,6 +114,26 @@ struct RegsGraphKey {
     int grid, block, smem, mode;
 };
 
+// Host memory a result's columns lie in: pinned (written by the device) or
+// the result's own copy.
+struct OutBlock {
+    PinnedBuf pin;
+    char* dev = nullptr;             // the pinned block's device address
+    std::unique_ptr<char[]> heap;
+};
+
+// The pinned blocks of one plan or batch. A block goes to one result at a
+// time and comes back when that result (its last holder) is freed; at most two
+// are lent, and a run that finds both with results still alive writes the
+// third, whose rows its result copies.
+struct OutPool {
+    std::vector<std::shared_ptr<OutBlock>> lent;
+    std::shared_ptr<OutBlock> stage;
+    // A block of at least `bytes`, null where pinned memory has no device
+    // address; lend tells whether the result may keep it.
+    std::shared_ptr<OutBlock> acquire(size_t bytes, bool& lend);
+};
+
 struct Plan {
     bool is_join = false;
     Table* t = nullptr;        // aggregate table or probe table
@@ -236,6 +256,11 @@ struct Plan {
     std::vector<unsigned long long> hot_keys;
     mutable std::mutex hot_mu;
     long long hash_rows_seen = 0;          //   and the rows that run scanned
+    // group tables assembled on the device (assemble.cu)
+    OutPool out_pool;
+    DevBuf d_asm, asm_bits, asm_scr;       // descriptor and columns; first-row bitmap; positions
+    std::vector<char> asm_img;             //   as last uploaded
+    long long asm_rows_seen = 0;           // groups of the last run (sizes the next block)
     // GROUP BY exactly the (non-NULL int64) join key on a group-table path:
     // the global join numbers the build's distinct keys (0..nk-1) and the
     // group table is indexed by that number (gid_koff: the key's code offset)
@@ -286,6 +311,12 @@ struct OutColumn {
     std::vector<int64_t> v;      // raw bits (int64 / float64 / date / bool / string code)
     std::vector<uint8_t> valid;
     const GlobalDict* dict = nullptr;
+    // assembled on the device: values in their final width and the validity
+    // bitmap, in the result's block; v and valid stay empty
+    const char* dv = nullptr;
+    const uint8_t* dm = nullptr;
+    std::shared_ptr<const FlatDict> flat;  // STRING: the codes' dictionary
+    bool distinct = false;                 // no two valid rows hold the same value
 };
 
 Plan* compile_agg(Table* t, const vexq_agg_plan_desc* d);
@@ -446,6 +477,7 @@ struct vexq_result_s {
     int32_t settle_code = 0;
     std::string settle_msg;
     std::vector<vq::OutColumn> cols;
+    std::shared_ptr<vq::OutBlock> block;  // holds the device-assembled columns
     int64_t nrows = 0;
     int64_t pos = 0;
     double kernel_ms = 0;

@@ -16,7 +16,7 @@
 #include <numeric>
 #include <set>
 
-#include "plan.h"
+#include "assemble.h"
 #include "device_common.cuh"
 
 namespace vq {
@@ -569,6 +569,18 @@ static void check_distinct_flags(int herr) {
     if (herr & 32) fail(VEXQ_ETIMEDOUT, "COUNT(DISTINCT) set: a slot being written was not published within the wait limit");
 }
 
+// Status of a group-table run from its error word: true when a hash table
+// reached its probe limit (the run repeats with a larger one).
+static bool check_table_flags(int herr, bool hash) {
+    check_spec_flags(herr);
+    check_distinct_flags(herr);
+    if (herr & 8) fail(VEXQ_ETIMEDOUT, "a staged tile copy did not complete within the kernel's wait limit");
+    if (herr & 2) fail(VEXQ_ENOTSUP, "float sum exceeded its exact accumulation window");
+    if (!(herr & 1)) return false;
+    if (!hash) fail(VEXQ_EDEVICE, "dense group table reported a probe failure");
+    return true;
+}
+
 void check_regs_flags(int herr) {
     check_spec_flags(herr);
     check_distinct_flags(herr);
@@ -627,7 +639,36 @@ struct RunCtx {
     int launches = 0;
     const JitKernel* k = nullptr;  // main kernel other than p.k_main (partition join)
     int grid = 0;                  // and its grid
+    long long row0 = 0, row1 = 0;  // rows the main scan's ranges span
 };
+
+std::shared_ptr<OutBlock> OutPool::acquire(size_t bytes, bool& lend) {
+    auto fit = [&](OutBlock& b) {
+        if (b.pin.n >= bytes) return;
+        b.dev = nullptr;
+        b.pin.ensure(bytes + bytes / 4);
+        void* d = nullptr;
+        if (cudaHostGetDevicePointer(&d, b.pin.p, 0) == cudaSuccess) b.dev = (char*)d;
+        else (void)cudaGetLastError();
+    };
+    lend = true;
+    std::shared_ptr<OutBlock> b;
+    for (auto& x : lent)
+        if (x.use_count() == 1 && (!b || x->pin.n > b->pin.n)) b = x;  // the pool is its only holder
+    if (!b && lent.size() < 2) {
+        b = std::make_shared<OutBlock>();
+        lent.push_back(b);
+    }
+    if (!b) {
+        lend = false;
+        if (!stage) stage = std::make_shared<OutBlock>();
+        b = stage;
+    }
+    // the freeing thread's last reads come before the device's next writes
+    std::atomic_thread_fence(std::memory_order_acquire);
+    fit(*b);
+    return b->dev ? b : nullptr;
+}
 
 void ensure_events(Plan& p) {
     for (auto& e : p.ev)
@@ -886,12 +927,87 @@ struct Compacted {
     bool hash = false;             // deferred run on a hash table: its group count sizes the next run
     long long rows = 0;
     bool having_done = false;  // only the groups HAVING keeps
+    vexq_result_s* done = nullptr;  // the finished result, where the device assembled it
 };
+
+// Writes the run's result columns from the group table in P (assemble.cu) and
+// waits for them. Returns null, with the error word, when the kernels raised
+// one or no pinned block is addressable (*ok false).
+static vexq_result_s* run_assemble(RunCtx& rc, const VQParams& P, long long nslots, const int* d_lsb, int* herr, bool* ok) {
+    Plan& p = rc.p;
+    *ok = true;
+    // rows the block holds: every slot of a small table, else a quarter more
+    // than the last run's groups; a run with more groups writes them again
+    // into a larger block (the table is still there)
+    long long cap = nslots <= 65536 ? nslots
+                  : std::min(nslots, p.asm_rows_seen > 0 ? (p.asm_rows_seen + p.asm_rows_seen / 4 + 1023) / 1024 * 1024 : 65536LL);
+    for (;;) {
+        const AsmLayout L = asm_layout(p, cap);
+        bool lend = true;
+        std::shared_ptr<OutBlock> blk = p.out_pool.acquire(L.bytes, lend);
+        if (!blk) {
+            *ok = false;
+            return nullptr;
+        }
+        VQAsmDesc d;
+        std::memset(&d, 0, sizeof d);
+        const size_t nb = asm_span(p, rc.row0, rc.row1, d);
+        if (p.asm_bits.n < nb) {  // cleared once: every run leaves it clear
+            p.asm_bits.ensure(nb);
+            VQ_CUDA(cudaMemsetAsync(p.asm_bits.p, 0, p.asm_bits.n, rc.s));
+        }
+        d.bits = p.asm_bits.as<unsigned>();
+        p.asm_scr.ensure(asm_scratch(d, cap, nullptr));
+        asm_scratch(d, cap, p.asm_scr.as<char>());
+        const size_t at = (sizeof d + 15) & ~(size_t)15, bytes = at + L.cols.size() * sizeof(VQAsmCol);
+        p.d_asm.ensure(bytes);
+        d.keys = P.keys;
+        d.first = P.first;
+        d.acc_i = P.acc_i;
+        d.acc_fx = P.acc_fx;
+        d.special = P.special;
+        d.fx_lsb = d_lsb;
+        d.error = P.error;
+        d.cols = (const VQAsmCol*)(p.d_asm.as<char>() + at);
+        d.nslots = nslots;
+        d.ncols = (int)L.cols.size();
+        d.write = nslots <= kAsmClusterWrites;
+        std::vector<char> img(bytes, 0);
+        std::memcpy(img.data(), &d, sizeof d);
+        std::memcpy(img.data() + at, L.cols.data(), L.cols.size() * sizeof(VQAsmCol));
+        if (img != p.asm_img) {
+            h2d(p.d_asm.p, img.data(), bytes, rc.s);
+            p.asm_img = std::move(img);
+        }
+        asm_launch(p.d_asm.as<VQAsmDesc>(), 1, blk->dev, nullptr, rc.s);
+        launch_check(rc.s, "k_assemble");
+        rc.launches++;
+        if (!d.write) {
+            asm_launch_write(p.d_asm.as<VQAsmDesc>(), blk->dev, rc.s);
+            launch_check(rc.s, "k_asm_write");
+            rc.launches++;
+        }
+        VQ_CUDA(cudaEventRecord(p.ev[3], rc.s));
+        VQ_CUDA(cudaStreamSynchronize(rc.s));
+        const VQAsmHdr* h = (const VQAsmHdr*)blk->pin.p;
+        *herr = h->err;
+        if (h->err) return nullptr;
+        p.asm_rows_seen = (long long)h->n;
+        if ((long long)h->n > cap) {
+            cap = std::min(nslots, ((long long)h->n + 1023) / 1024 * 1024);
+            continue;
+        }
+        return asm_result(p, L, (const char*)blk->pin.p, (long long)h->n, lend ? blk : nullptr);
+    }
+}
 
 // A deferred run (defer set) launches the table kernels and returns without
 // waiting: the caller's top-k launches follow on the stream, and one copy back
 // after them brings the group count and the error word with the results.
-Compacted run_atomic(RunCtx& rc, VQParams& P, long long nchunks, long long estimate, long long rows, bool defer = false) {
+// assemble: the caller wants the finished result (c.done) where the device can
+// write it; where it cannot, the groups come compacted as without it.
+Compacted run_atomic(RunCtx& rc, VQParams& P, long long nchunks, long long estimate, long long rows, bool defer = false,
+                     bool assemble = false) {
     Plan& p = rc.p;
     // a join grouping by its key on the global table: one slot per build key
     // number, no key inserts; the keys come from the build's number→key array
@@ -935,23 +1051,11 @@ Compacted run_atomic(RunCtx& rc, VQParams& P, long long nchunks, long long estim
         tail = (char*)(((uintptr_t)tail + 15) & ~(uintptr_t)15);
         P.ngroups = (unsigned long long*)tail;
         P.error = (int*)(tail + 8);
-        long long* d_init = (long long*)(tail + 16);
+        unsigned long long* n_out = (unsigned long long*)(tail + 16);
         P.cap = (unsigned long long)cap;
         P.cap_mask = hash ? (unsigned long long)(cap - 1) : 0;
         for (int f = 0; f < nf && f < 16; f++) P.fx_lsb[f] = p.fx_lsb[f];
-        // compacted output (upper bound: every slot occupied)
-        long long cap_out = nslots;
-        size_t o_bytes = 16 + cap_out * 16 + (size_t)ni * cap_out * 8 + (size_t)nf * cap_out * 8 + nf * 4 + 64;
-        p.scratch_b.ensure(o_bytes);
-        char* ob = (char*)p.scratch_b.p;
         Compacted c;
-        c.cap_out = cap_out;
-        unsigned long long* n_out = (unsigned long long*)ob;
-        c.key = (unsigned long long*)(ob + 16);
-        c.first = (long long*)(ob + 16 + cap_out * 8);
-        c.ival = (long long*)(ob + 16 + cap_out * 16);
-        c.fval = (double*)(ob + 16 + cap_out * 16 + (size_t)ni * cap_out * 8);
-        (void)d_init;
         // the plan's constant identities and float-sum windows, uploaded once
         const size_t tinit = iv.size() * 8 + (size_t)std::max(nf, 1) * 4;
         if (p.d_tinit.n < tinit) {
@@ -976,6 +1080,37 @@ Compacted run_atomic(RunCtx& rc, VQParams& P, long long nchunks, long long estim
         jit_launch(K, grid, &P, sizeof P, rc.s);
         launch_check(rc.s, "p.k_main");
         VQ_CUDA(cudaEventRecord(p.ev[2], rc.s));
+        if (assemble && asm_run_ok(p, nslots, rc.row0, rc.row1)) {
+            int herr = 0;
+            bool ok = true;
+            c.done = run_assemble(rc, P, nslots, d_lsb, &herr, &ok);
+            if (ok) {
+                rc.scan_ms += elapsed(p.ev[1], p.ev[2]);
+                rc.kernel_ms += elapsed(p.ev[0], p.ev[3]);
+                rc.launches += 2;
+                if (c.done) {
+                    if (hash) {
+                        p.hash_groups_seen = p.asm_rows_seen;
+                        p.hash_rows_seen = rows;
+                    }
+                    return c;
+                }
+                if (check_table_flags(herr, hash)) {
+                    cap = std::max(cap << 1, safe_cap);
+                    continue;
+                }
+            }
+        }
+        // compacted output (upper bound: every slot occupied)
+        long long cap_out = nslots;
+        size_t o_bytes = 16 + cap_out * 16 + (size_t)ni * cap_out * 8 + (size_t)nf * cap_out * 8 + nf * 4 + 64;
+        p.scratch_b.ensure(o_bytes);
+        char* ob = (char*)p.scratch_b.p;
+        c.cap_out = cap_out;
+        c.key = (unsigned long long*)(ob + 16);
+        c.first = (long long*)(ob + 16 + cap_out * 8);
+        c.ival = (long long*)(ob + 16 + cap_out * 16);
+        c.fval = (double*)(ob + 16 + cap_out * 16 + (size_t)ni * cap_out * 8);
         int fg = (int)std::min<long long>((nslots + 255) / 256, (long long)sm_count() * 16);
         k_finalize<<<fg, 256, 0, rc.s>>>(gid ? p.jt_gkey.as<unsigned long long>() : P.keys, P.first, P.acc_i, P.acc_fx, P.special,
                                          nslots, ni, nf, d_lsb, hash || gid, n_out, c.key, c.first, c.ival, c.fval, cap_out);
@@ -1000,12 +1135,7 @@ Compacted run_atomic(RunCtx& rc, VQParams& P, long long nchunks, long long estim
         rc.launches += 3;
         unsigned long long nn = *(unsigned long long*)p.h_stage.p;
         int herr = *(int*)((char*)p.h_stage.p + 8);
-        check_spec_flags(herr);
-        check_distinct_flags(herr);
-        if (herr & 8) fail(VEXQ_ETIMEDOUT, "a staged tile copy did not complete within the kernel's wait limit");
-        if (herr & 2) fail(VEXQ_ENOTSUP, "float sum exceeded its exact accumulation window");
-        if (herr & 1) {  // probe limit: grow the table and rerun
-            if (!hash) fail(VEXQ_EDEVICE, "dense group table reported a probe failure");
+        if (check_table_flags(herr, hash)) {
             cap = std::max(cap << 1, safe_cap);
             continue;
         }
@@ -1159,14 +1289,7 @@ int topk_groups(RunCtx& rc, Compacted& c, Groups& g) {
         rc.kernel_ms += elapsed(p.ev[0], p.ev[3]);
         c.n = (long long)std::min<unsigned long long>(*(const unsigned long long*)hs, (unsigned long long)c.cap_out);
         const int herr = *(const int*)(hs + 8);
-        check_spec_flags(herr);
-        check_distinct_flags(herr);
-        if (herr & 8) fail(VEXQ_ETIMEDOUT, "a staged tile copy did not complete within the kernel's wait limit");
-        if (herr & 2) fail(VEXQ_ENOTSUP, "float sum exceeded its exact accumulation window");
-        if (herr & 1) {
-            if (!c.hash) fail(VEXQ_EDEVICE, "dense group table reported a probe failure");
-            return -1;
-        }
+        if (check_table_flags(herr, c.hash)) return -1;
         if (c.hash) {
             p.hash_groups_seen = c.n;
             p.hash_rows_seen = c.rows;
@@ -1545,7 +1668,13 @@ static vexq_result_s* finish_groups(RunCtx& rc, VQParams& P, long long nchunks, 
         // ORDER BY an aggregate with a LIMIT and no HAVING: the top-k kernels
         // follow the table run without waiting for its count
         const bool defer = !p.partial_out && p.having_root < 0 && p.ndist == 0 && topk_applies(p, false);
-        Compacted c = run_atomic(rc, P, nchunks, estimate, rows, defer);
+        Compacted c = run_atomic(rc, P, nchunks, estimate, rows, defer, !p.partial_out && asm_plan_ok(p));
+        if (c.done) {
+            c.done->kernel_ms = rc.kernel_ms;
+            c.done->scan_ms = rc.scan_ms;
+            c.done->launches = rc.launches;
+            return c.done;
+        }
         if (p.partial_out) {
             g = fetch_groups(rc, c);  // a shard's partial: every group, no HAVING, no LIMIT
         } else {
@@ -2210,6 +2339,10 @@ vexq_result_s* run_plan(Plan& p, int rg_start, int rg_end) {
     P.present = p.d_present.as<unsigned char>();
     for (size_t i = 0, off = 0; i < p.sets.size(); i++) { P.sets[i] = p.d_sets.as<unsigned>() + off; off += p.sets[i].size(); }
 
+    if (!ss.seg.empty()) {
+        rc.row0 = ss.seg.front();
+        rc.row1 = ss.seg[ss.seg.size() - 2];
+    }
     bytes += sm.bytes;
     rows_scanned += ss.rows;
     if (use_radix && ss.nchunks > 0) {
@@ -2289,6 +2422,65 @@ vexq_result_s* run_plan_host(Plan& p, const vexq_column_desc* cols, int32_t ncol
     return run_plan(p, 0, -1);
 }
 
+// A batch's view of a column the device assembled: the block's own bytes, but
+// for strings, whose batch has a dictionary of its own (exec.newStringVector),
+// codes in first-occurrence order.
+static void view_assembled(vexq_result_s& r, size_t c, int64_t n) {
+    const OutColumn& oc = r.cols[c];
+    vexq_vector_view& v = r.views[c];
+    const uint8_t* dm = oc.dm + r.pos / 8;  // batches start at multiples of 1,024 rows
+    v.validity = dm;
+    if (n & 7) {  // bits past the last row are 0 (a LIMIT can cut between rows)
+        std::vector<uint8_t>& bm = r.bbuf[c];
+        bm.assign(dm, dm + (n + 7) / 8);
+        bm.back() &= (uint8_t)((1u << (n & 7)) - 1u);
+        v.validity = bm.data();
+    }
+    if (oc.type != VEXQ_TYPE_STRING) {
+        const int w = (oc.type == VEXQ_TYPE_INT64 || oc.type == VEXQ_TYPE_FLOAT64) ? 8 : oc.type == VEXQ_TYPE_BOOL ? 1 : 4;
+        v.values = oc.dv + r.pos * w;
+        return;
+    }
+    const uint32_t* code = (const uint32_t*)oc.dv + r.pos;
+    const FlatDict& d = *oc.flat;
+    std::vector<char>& vb = r.vbuf[c];
+    vb.resize(n * 4);
+    uint32_t* local = (uint32_t*)vb.data();
+    std::vector<uint32_t>& off = r.doff[c];
+    std::string& bytes = r.dbytes[c];
+    off.reserve(n + 1);
+    off.push_back(0);
+    size_t most = 0;
+    for (int64_t i = 0; i < n; i++)
+        if ((size_t)code[i] + 1 < d.off.size()) most += d.off[code[i] + 1] - d.off[code[i]];
+    bytes.reserve(most);
+    // codes seen in this batch: open addressing over twice the batch's rows
+    constexpr uint32_t kSeen = 2 * VEXQ_BLOCK_ROWS;
+    std::vector<uint64_t> seen(oc.distinct ? 0 : kSeen, 0);  // (code + 1) << 32 | local code
+    for (int64_t i = 0; i < n; i++) {
+        local[i] = 0;
+        if (!((dm[i >> 3] >> (i & 7)) & 1)) continue;
+        const uint32_t g = code[i];
+        if ((size_t)g + 1 >= d.off.size()) fail(VEXQ_EDEVICE, "result string code outside its dictionary");
+        const uint32_t next = (uint32_t)off.size() - 1;
+        uint32_t l = next;
+        if (!oc.distinct) {
+            uint32_t h = (g * 2654435761u) >> 21;  // 11 bits: kSeen slots
+            while (seen[h] && (uint32_t)(seen[h] >> 32) != g + 1) h = (h + 1) & (kSeen - 1);
+            if (seen[h]) l = (uint32_t)seen[h];
+            else seen[h] = (uint64_t)(g + 1) << 32 | next;
+        }
+        local[i] = l;
+        if (l != next) continue;
+        bytes.append(d.bytes, d.off[g], d.off[g + 1] - d.off[g]);
+        off.push_back((uint32_t)bytes.size());
+    }
+    v.values = local;
+    v.dict_str_off = off.data();
+    v.dict_bytes = bytes.data();
+    v.dict_len = (int32_t)off.size() - 1;
+}
+
 // ---- Next(): ≤ 1024-row batches (exec/aggregate.go:209-216) ----------------------------
 int32_t result_next(vexq_result_s* r, vexq_batch_view* out) {
     int64_t n = std::min<int64_t>(VEXQ_BLOCK_ROWS, r->nrows - r->pos);
@@ -2304,6 +2496,10 @@ int32_t result_next(vexq_result_s* r, vexq_batch_view* out) {
         vexq_vector_view& v = r->views[c];
         v.name = oc.name.c_str();
         v.type = oc.type;
+        if (oc.dv) {
+            view_assembled(*r, c, n);
+            continue;
+        }
         std::vector<uint8_t>& bm = r->bbuf[c];
         bm.assign((n + 7) / 8, 0);
         for (int64_t i = 0; i < n; i++) if (oc.valid[r->pos + i]) bm[i >> 3] |= (uint8_t)(1u << (i & 7));

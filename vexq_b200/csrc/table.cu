@@ -70,6 +70,22 @@ uint32_t GlobalDict::add(const std::string& s) {
     return c;
 }
 
+std::shared_ptr<const FlatDict> flat_dict(const Column& c) {
+    static std::mutex mu;
+    std::lock_guard<std::mutex> lk(mu);
+    if (!c.flat) {
+        auto f = std::make_shared<FlatDict>();
+        f->off.reserve(c.dict.keys.size() + 1);
+        f->off.push_back(0);
+        for (const std::string& k : c.dict.keys) {
+            f->bytes += k;
+            f->off.push_back((uint32_t)f->bytes.size());
+        }
+        c.flat = f;
+    }
+    return c.flat;
+}
+
 int sm_count() {
     if (!g_sm_count) {
         int dev = 0;
