@@ -331,6 +331,7 @@ int32_t vexq_filter_run(vexq_table_t t, const vexq_expr* nodes, int32_t nnodes, 
         P.error = (int*)(scal.as<char>() + 16);
         P.seg = dseg.as<long long>();
         P.nseg = seg.empty() ? 0 : 1;
+        set_one_seg(P, seg);
         P.nchunks = chunks;
         cudaStream_t s = plan_stream(*p);
         VQ_CUDA(cudaMemsetAsync(bits.p, 0, bits.n, s));

@@ -248,7 +248,7 @@ bool asm_plan_ok(const Plan& p) {
     // joins order groups by (probe row, chain position), which no row bitmap
     // holds; string MIN/MAX map ranks back to strings on the host; HAVING and
     // ORDER BY take the groups unordered
-    if (p.path == AggPath::Regs || p.is_join || p.keys.empty() || p.hot_n > 0) return false;
+    if (p.path == AggPath::Regs || p.is_join || p.keys.empty()) return false;
     if (p.having_root >= 0 || p.order.sort_col >= 0) return false;
     if (p.keys.size() + p.outs.size() > (size_t)kAsmMaxCols) return false;
     for (const AggOut& a : p.outs)

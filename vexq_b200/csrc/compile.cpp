@@ -1534,385 +1534,249 @@ void emit_atomic_update(std::ostringstream& os, const Plan& p, const std::string
     }
 }
 
-// Block-private shared-memory accumulators for the dense path: groups below
-// smem_groups are updated with shared-memory atomics and flushed to the global
-// table once per block; the layout is [first][int bank][fixed-point digits][flags].
-struct CacheLayout {
-    int C = 0;
-    std::string first, ints, fx, sp;
+// Block-private shared-memory accumulators for the dense path: the groups of
+// the first codes, and the last code (the NULL group of a single nullable
+// key), are updated with 32-bit shared-memory atomics and flushed to the
+// global table once per block. Codes are given out in first-occurrence order,
+// so the frequent groups are among the first; the NULL group has the last code
+// and can be the largest of all (uncached, 5% of 4M rows in it serialised on its
+// global counters: 299 us a scan against 65 us without NULLs).
+//
+// One entry, field by field over all entries (lanes updating different groups
+// spread over the banks): 64-bit MIN/MAX keys, then 32-bit words — first row,
+// row and non-null counts (a block's stay below 2^32), integer sums as two
+// words, float sums as seven limbs (vq_s_fx_add) and, where the input may be
+// NaN or infinite, a flag word.
+//
+// Bound by instruction issue (103 warp instructions a row with one SUM, 153 with
+// SUM COUNT MIN MAX AVG, 60% of the issue slots) and, on small tables, by
+// setting up and flushing the entries: 4M rows over 1,000 groups 39 us (47 with
+// two 512-thread blocks and 68-byte entries whose sums took their carries from
+// returned old values), 1.2M nullable rows over 20,012 groups 31 us (124).
+constexpr int kCacheLimbs = 7;    // VQ_LIMBS
+struct CacheField {
+    int n64 = 0, n32 = 0;         // 8-byte and 4-byte fields of an entry
+    std::vector<int> at;          // per slot: index of its first field in its class
 };
-// The cached group count is the launch-time value P.cache_n (vq_C in the
-// generated code), so plans that differ only in domain share a kernel.
-// Limb form (cache_limbs): the fixed-point region holds, per float sum, sixteen
-// 32-bit limb counters a group (eight positive, eight negative; limb j of
-// every group contiguous) instead of four 64-bit digit counters.
-CacheLayout cache_layout(const Plan& p) {
-    CacheLayout L;
-    L.C = p.smem_groups;
-    L.first = "((long long*)vq_smem)";
-    L.ints = "(((long long*)vq_smem) + vq_C)";
-    L.fx = "(((long long*)vq_smem) + (long long)vq_C * " + std::to_string(1 + p.ni) + ")";
-    const int fx_longs = (p.cache_limbs ? 8 : 4) * p.nf;
-    L.sp = "((unsigned*)(((long long*)vq_smem) + (long long)vq_C * " + std::to_string(1 + p.ni + fx_longs) + "))";
-    return L;
+bool cache_is64(SlotKind k) { return k == S_IMIN || k == S_IMAX || k == S_FMIN || k == S_FMAX; }
+bool slot_finite(const Plan& p, size_t s) { return p.ir[p.slots[s].input].finite; }
+bool slot_signed(const Plan& p, size_t s) {
+    const INode& x = p.ir[p.slots[s].input];
+    return !(x.bounded && x.lo >= 0);
+}
+CacheField cache_fields(const Plan& p) {
+    CacheField F;
+    F.n32 = 1;  // first row
+    F.at.assign(p.slots.size(), -1);
+    for (size_t s = 0; s < p.slots.size(); s++) {
+        const SlotKind k = p.slots[s].kind;
+        if (cache_is64(k)) { F.at[s] = F.n64++; continue; }
+        F.at[s] = F.n32;
+        F.n32 += k == S_ISUM ? 2 : k == S_FSUM ? kCacheLimbs + !slot_finite(p, s) : 1;  // the flag word follows the limbs
+    }
+    return F;
+}
+std::string cache_word(int k) { return "vq_a4 + " + std::to_string(k) + "u * vq_s4"; }
+
+std::string fx_flags(const Plan& p, size_t s) {
+    return std::string("<") + (slot_finite(p, s) ? "true" : "false") + ", " + (slot_signed(p, s) ? "true" : "false") + ">";
 }
 
+// MIN/MAX inputs as unsigned keys in the value's order
+std::string minmax_key(const Plan& p, size_t s) {
+    const std::string SV = "sv" + std::to_string(s);
+    const SlotKind k = p.slots[s].kind;
+    return k == S_FMIN || k == S_FMAX ? "vq_fkey(" + SV + ")" : "((unsigned long long)" + SV + " ^ 0x8000000000000000ull)";
+}
 
-// Opens "if (slot < C) { shared-memory update } else {" — the caller emits the
-// global update and closes the brace.
-void emit_cache_update(std::ostringstream& os, const Plan& p, const std::string& ind) {
-    CacheLayout L = cache_layout(p);
-    const std::string C = "vq_C";
-    os << ind << "if (slot < (unsigned long long)vq_C) {\n";
-    std::string in = ind + "    ";
-    // MIN/MAX and first-row keys only ever move one way, so a plain read that
-    // shows no improvement (possibly stale, never past the true value) skips
-    // the atomic; most rows after the first few of a group skip it
-    os << in << "if (ag_first < " << L.first << "[slot]) atomicMin(" << L.first << " + slot, ag_first);\n";
+// One row's update of the cached entry vq_ci. First row, MIN and MAX only ever
+// move one way, so plain reads that show no improvement (possibly stale, never
+// past the true value) skip their atomics behind one branch; most rows after
+// the first few of a group skip it.
+void emit_cache_update(std::ostringstream& os, const Plan& p, const std::string& in) {
+    const CacheField F = cache_fields(p);
+    os << in << "const unsigned vq_a4 = vq_w4 + vq_ci * 4u;\n";
+    if (F.n64) os << in << "const unsigned vq_a8 = vq_sb + vq_ci * 8u;\n";
+    os << in << "const unsigned vq_gf = vq_s_ld(vq_a4);\n";
+    std::string any = "(unsigned)r < vq_gf";
     for (size_t s = 0; s < p.slots.size(); s++) {
-        std::string S = std::to_string(s), pos = std::to_string(p.slot_pos[s]);
-        std::string ai = L.ints + " + " + pos + " * " + C + " + slot";
-        std::string aiu = "(unsigned long long*)(" + ai + ")";
+        const SlotKind k = p.slots[s].kind;
+        if (!cache_is64(k)) continue;
+        const std::string S = std::to_string(s);
+        const bool nan = (k == S_FMIN || k == S_FMAX) && !slot_finite(p, s), mn = k == S_IMIN || k == S_FMIN;
+        os << in << "const unsigned long long vq_k" << S << " = " << minmax_key(p, s) << ", vq_g" << S << " = vq_s_ld64(vq_a8 + " << F.at[s]
+           << "u * 2u * vq_s4);\n";
+        os << in << "const bool vq_b" << S << " = sok" << S << (nan ? " && !isnan(sv" + S + ")" : std::string()) << " && vq_k" << S
+           << (mn ? " < " : " > ") << "vq_g" << S << ";\n";
+        any += " || vq_b" + S;
+    }
+    os << in << "if (" << any << ") {\n";
+    os << in << "    if ((unsigned)r < vq_gf) vq_s_min(vq_a4, (unsigned)r);\n";
+    for (size_t s = 0; s < p.slots.size(); s++) {
+        const SlotKind k = p.slots[s].kind;
+        if (!cache_is64(k)) continue;
+        const std::string S = std::to_string(s);
+        os << in << "    if (vq_b" << S << ") " << (k == S_IMIN || k == S_FMIN ? "vq_s_min64" : "vq_s_max64") << "(vq_a8 + " << F.at[s]
+           << "u * 2u * vq_s4, vq_k" << S << ");\n";
+    }
+    os << in << "}\n";
+    for (size_t s = 0; s < p.slots.size(); s++) {
+        const std::string S = std::to_string(s), SV = "sv" + S, w = cache_word(F.at[s]), iff = "if (sok" + S + ") ";
         switch (p.slots[s].kind) {
-            case S_CNT:
-            case S_NN:
-                // a block's count stays below 2^32: a 32-bit add on the counter's low word
-                if (p.cache_limbs && s == 0)  // the row count, read back: every 32,768 rows the group's limbs are normalised
-                    os << in << "const unsigned vq_c0 = atomicAdd((unsigned*)(" << ai << "), (unsigned)ag" << S << ");\n";
-                else if (p.cache_cnt32) os << in << "if (ag" << S << ") atomicAdd((unsigned*)(" << ai << "), (unsigned)ag" << S << ");\n";
-                else os << in << "if (ag" << S << ") atomicAdd(" << aiu << ", (unsigned long long)ag" << S << ");\n";
-                break;
-            case S_ISUM:
-                if (p.cache_fx32) os << in << "if (ah" << S << ") vq_add64_as32(" << ai << ", ag" << S << ");\n";
-                else os << in << "if (ah" << S << ") atomicAdd(" << aiu << ", (unsigned long long)ag" << S << ");\n";
-                break;
-            case S_IMIN: os << in << "if (ah" << S << " && ag" << S << " < *(" << ai << ")) atomicMin(" << ai << ", ag" << S << ");\n"; break;
-            case S_IMAX: os << in << "if (ah" << S << " && ag" << S << " > *(" << ai << ")) atomicMax(" << ai << ", ag" << S << ");\n"; break;
-            case S_FMIN: os << in << "if (ah" << S << " && ag" << S << " < *" << aiu << ") atomicMin(" << aiu << ", ag" << S << ");\n"; break;
-            case S_FMAX: os << in << "if (ah" << S << " && ag" << S << " > *" << aiu << ") atomicMax(" << aiu << ", ag" << S << ");\n"; break;
+            case S_CNT: os << in << "vq_s_add(" << w << ", 1u);\n"; break;
+            case S_NN: os << in << iff << "vq_s_add(" << w << ", 1u);\n"; break;
+            case S_ISUM: os << in << iff << "vq_s_add64(" << w << ", " << cache_word(F.at[s] + 1) << ", (unsigned long long)" << SV << ");\n"; break;
             case S_FSUM:
-                if (p.cache_limbs) {
-                    os << in << "if (ah" << S << ") { vq_limbs_add((unsigned*)" << L.fx << " + (long long)" << pos << " * 16 * " << C
-                       << " + (long long)slot, " << C << ", fd" << S << "_0, fd" << S << "_1, fd" << S << "_2, fd" << S << "_3); if (fsp" << S
-                       << ") atomicOr(" << L.sp << " + " << pos << " * " << C << " + slot, fsp" << S << "); }\n";
-                    break;
-                }
-                os << in << "if (ah" << S << ") { " << (p.cache_fx32 ? "vq_fx_add_digits_s32(" : "vq_fx_add_digits_s(") << L.fx << " + (long long)" << pos << " * 4 * " << C
-                   << " + (long long)slot, " << C << ", fd" << S << "_0, fd" << S << "_1, fd" << S << "_2, fd" << S << "_3); if (fsp" << S
-                   << ") atomicOr(" << L.sp << " + " << pos << " * " << C << " + slot, fsp" << S << "); }\n";
+                os << in << iff << "vq_s_fx_add" << fx_flags(p, s) << "(" << w << ", vq_s4, " << SV << ", P.fx_lsb[" << p.slot_pos[s]
+                   << "], P.error);\n";
                 break;
+            default: break;
         }
     }
-    if (p.cache_limbs && p.nf > 0) {
-        os << in << "if (((vq_c0 + (unsigned)ag0) >> 15) != (vq_c0 >> 15)) {\n";
-        for (int f = 0; f < p.nf; f++)
-            os << in << "    vq_limbs_norm((unsigned*)" << L.fx << " + (long long)" << f << " * 16 * " << C << " + (long long)slot, " << C << ");\n";
-        os << in << "}\n";
-    }
-    os << ind << "} else {\n";
 }
 
-void emit_cache_init(std::ostringstream& os, const Plan& p, bool declare_smem = true) {
-    CacheLayout L = cache_layout(p);
-    const std::string C = "vq_C";
-    if (declare_smem) os << "    extern __shared__ __align__(16) unsigned char vq_smem[];\n";
-    os << "    const int vq_C = P.cache_n;\n";
-    os << "    for (int i = threadIdx.x; i < " << C << "; i += blockDim.x) {\n";
-    os << "        " << L.first << "[i] = 0x7FFFFFFFFFFFFFFFLL;\n";
+// Entries that have taken 4,096 rows are normalised each time the block has
+// read 4,096 more, so no limb takes more than VQ_LIMB_ROWS rows in between. The
+// whole block calls it after the same chunk step.
+void emit_cache_norm(std::ostringstream& os, const Plan& p, int block, const std::string& step) {
+    const CacheField F = cache_fields(p);
+    bool any = false;
+    for (size_t s = 0; s < p.slots.size(); s++) any = any || p.slots[s].kind == S_FSUM;
+    if (!any) return;
+    const int steps = std::max(1, 4096 / (block / 32 * 128));
+    os << "        if (" << step << " % " << steps << " == " << steps - 1 << ") {\n";
+    os << "            __syncthreads();\n";
+    os << "            for (unsigned i = threadIdx.x; i < vq_C; i += blockDim.x) {\n";
+    os << "                const unsigned vq_a4 = vq_w4 + i * 4u;\n";
+    os << "                if (vq_s_ld(" << cache_word(F.at[0]) << ") < 4096u) continue;\n";
+    for (size_t s = 0; s < p.slots.size(); s++)
+        if (p.slots[s].kind == S_FSUM)
+            os << "                vq_s_limbs_norm<" << (slot_signed(p, s) ? "true" : "false") << ">(" << cache_word(F.at[s]) << ", vq_s4);\n";
+    os << "            }\n            __syncthreads();\n        }\n";
+}
+
+// One row's update of the global table's slot. Unguarded (fire-and-forget)
+// MIN/MAX and first-row atomics: a read of the current value to skip them
+// measured slower there (4M rows, 65,536 Zipf groups mostly uncached: 118.9
+// against 74.8 us; 200K hash keys: 201.6 against 197.7 us).
+void emit_table_update(std::ostringstream& os, const Plan& p, const std::string& in, const std::string& order) {
+    os << in << "const long long stride = (long long)P.cap + 1;\n";
+    os << in << "atomicMin(&P.first[slot], " << order << ");\n";
     for (size_t s = 0; s < p.slots.size(); s++) {
-        const Slot& sl = p.slots[s];
-        if (sl.kind == S_FSUM) {
-            std::string pos = std::to_string(p.slot_pos[s]);
-            if (p.cache_limbs)
-                os << "        for (int d = 0; d < 16; d++) ((unsigned*)" << L.fx << ")[(" << pos << " * 16 + d) * " << C << " + i] = 0u;\n";
-            else
-                os << "        for (int d = 0; d < 4; d++) " << L.fx << "[(" << pos << " * 4 + d) * " << C << " + i] = 0;\n";
-            os << "        " << L.sp << "[" << pos << " * " << C << " + i] = 0u;\n";
-            continue;
+        const std::string S = std::to_string(s), SV = "sv" + S, pos = std::to_string(p.slot_pos[s]), iff = "if (sok" + S + ") ";
+        const std::string ai = "P.acc_i[" + pos + " * stride + slot]", aiu = "(unsigned long long*)&" + ai;
+        switch (p.slots[s].kind) {
+            case S_CNT: os << in << "atomicAdd(" << aiu << ", 1ull);\n"; break;
+            case S_NN: os << in << iff << "atomicAdd(" << aiu << ", 1ull);\n"; break;
+            case S_ISUM: os << in << iff << "atomicAdd(" << aiu << ", (unsigned long long)" << SV << ");\n"; break;
+            case S_IMIN: os << in << iff << "atomicMin(&" << ai << ", " << SV << ");\n"; break;
+            case S_IMAX: os << in << iff << "atomicMax(&" << ai << ", " << SV << ");\n"; break;
+            case S_FMIN: os << in << "if (sok" << S << " && !isnan(" << SV << ")) atomicMin(" << aiu << ", vq_fkey(" << SV << "));\n"; break;
+            case S_FMAX: os << in << "if (sok" << S << " && !isnan(" << SV << ")) atomicMax(" << aiu << ", vq_fkey(" << SV << "));\n"; break;
+            case S_FSUM:
+                os << in << iff << "vq_g_fx_add" << fx_flags(p, s) << "(P.acc_fx + ((long long)" << pos << " * stride + (long long)slot) * 4, P.special + (long long)"
+                   << pos << " * stride + slot, " << SV << ", P.fx_lsb[" << pos << "], P.error);\n";
+                break;
         }
-        std::string init = "0LL";
-        if (sl.kind == S_IMIN) init = "0x7FFFFFFFFFFFFFFFLL";
-        if (sl.kind == S_IMAX) init = "(-0x7FFFFFFFFFFFFFFFLL - 1LL)";
-        if (sl.kind == S_FMIN) init = "(long long)vq_fkey(1.7976931348623157e308)";
-        if (sl.kind == S_FMAX) init = "(long long)vq_fkey(-1.7976931348623157e308)";
-        os << "        " << L.ints << "[" << p.slot_pos[s] << " * " << C << " + i] = " << init << ";\n";
+    }
+}
+
+// One live row of an aggregate scan on a group-table path.
+void emit_group_update(std::ostringstream& os, const Plan& p, const std::string& ind, const std::string& order, bool cache) {
+    const std::string in = ind + "    ";
+    if (p.path == AggPath::Dense) {
+        os << ind << "if (live) {\n";
+        os << in << "const unsigned slot = (unsigned)key;\n";
+    } else {
+        // lanes leave the probe loop at different steps: the warp meets again
+        // before the atomics
+        os << ind << "unsigned long long slot = VQ_NOSLOT;\n";
+        os << ind << "if (live) slot = vq_insert(P.keys, P.cap_mask, P.cap, key, nullptr, P.error);\n";
+        os << ind << "__syncwarp();\n";
+        os << ind << "if (slot != VQ_NOSLOT) {\n";
+    }
+    if (cache) {
+        os << in << "const unsigned vq_ci = slot == vq_last ? vq_C1 : slot;\n";
+        os << in << "if (vq_ci < vq_C1 || slot == vq_last) {\n";
+        emit_cache_update(os, p, in + "    ");
+        os << in << "} else {\n";
+        emit_table_update(os, p, in + "    ", order);
+        os << in << "}\n";
+    } else {
+        emit_table_update(os, p, in, order);
+    }
+    os << ind << "}\n";
+}
+
+// vq_C cached entries (P.cache_n, a launch-time value, so plans that differ
+// only in domain share a kernel): codes 0 … vq_C1 - 1 and, in entry vq_C1, the
+// last code. No entry: nothing matches vq_last.
+void emit_cache_init(std::ostringstream& os, const Plan& p, bool declare_smem = true) {
+    const CacheField F = cache_fields(p);
+    if (declare_smem) os << "    extern __shared__ __align__(16) unsigned char vq_smem[];\n";
+    os << "    const unsigned vq_C = (unsigned)P.cache_n, vq_C1 = vq_C ? vq_C - 1u : 0u;\n";
+    os << "    const unsigned vq_last = vq_C ? (unsigned)P.cap - 1u : 0xFFFFFFFFu;\n";
+    os << "    const unsigned vq_s4 = vq_C * 4u, vq_sb = vq_smem_addr(vq_smem), vq_w4 = vq_sb + " << 2 * F.n64 << "u * vq_s4;\n";
+    os << "    for (unsigned i = threadIdx.x; i < vq_C; i += blockDim.x) {\n";
+    os << "        const unsigned vq_a4 = vq_w4 + i * 4u;\n";
+    os << "        vq_s_st(vq_a4, 0xFFFFFFFFu);\n";
+    os << "        for (unsigned k = 1; k < " << F.n32 << "u; k++) vq_s_st(vq_a4 + k * vq_s4, 0u);\n";
+    for (size_t s = 0; s < p.slots.size(); s++) {
+        std::string init;
+        switch (p.slots[s].kind) {
+            case S_IMIN: init = "0xFFFFFFFFFFFFFFFFull"; break;  // integer keys: the value with its sign bit flipped
+            case S_IMAX: init = "0ull"; break;
+            case S_FMIN: init = "vq_fkey(1.7976931348623157e308)"; break;
+            case S_FMAX: init = "vq_fkey(-1.7976931348623157e308)"; break;
+            default: continue;
+        }
+        os << "        vq_s_st64(vq_sb + i * 8u + " << F.at[s] << "u * 2u * vq_s4, " << init << ");\n";
     }
     os << "    }\n    __syncthreads();\n";
 }
 
 void emit_cache_flush(std::ostringstream& os, const Plan& p) {
-    CacheLayout L = cache_layout(p);
-    const std::string C = "vq_C";
+    const CacheField F = cache_fields(p);
     os << "    __syncthreads();\n";
-    os << "    for (int i = threadIdx.x; i < " << C << "; i += blockDim.x) {\n";
-    os << "        if (" << L.ints << "[" << p.slot_pos[0] << " * " << C << " + i] == 0) continue;\n";
+    os << "    for (unsigned i = threadIdx.x; i < vq_C; i += blockDim.x) {\n";
+    os << "        const unsigned vq_a4 = vq_w4 + i * 4u;\n";
+    os << "        if (vq_s_ld(" << cache_word(F.at[0]) << ") == 0u) continue;\n";
     os << "        const long long stride = (long long)P.cap + 1;\n";
-    os << "        atomicMin(&P.first[i], " << L.first << "[i]);\n";
+    os << "        const unsigned slot = i == vq_C1 ? vq_last : i;\n";
+    if (p.intkey_order) {
+        // the phase of the group's order key: whether a key column is NULL
+        os << "        bool anynull = false;\n";
+        int64_t stride = 1;
+        for (const KeyCol& k : p.keys) {
+            if (k.nullable)
+                os << "        anynull = anynull || (slot / " << stride << "u) % " << k.domain << "u == " << k.domain - 1 << "u;\n";
+            stride *= k.domain;
+        }
+    }
+    os << "        atomicMin(&P.first[slot], " << order_expr(p, "(long long)vq_s_ld(vq_a4)") << ");\n";
     for (size_t s = 0; s < p.slots.size(); s++) {
-        int pos = p.slot_pos[s];
-        std::string P_ = std::to_string(pos);
-        std::string v = L.ints + "[" + P_ + " * " + C + " + i]";
-        std::string g = "P.acc_i[" + P_ + " * stride + i]";
+        const std::string pos = std::to_string(p.slot_pos[s]), w = cache_word(F.at[s]);
+        const std::string g = "P.acc_i[" + pos + " * stride + slot]", gu = "(unsigned long long*)&" + g;
+        const std::string v8 = "vq_s_ld64(vq_sb + i * 8u + " + std::to_string(F.at[s]) + "u * 2u * vq_s4)";
         switch (p.slots[s].kind) {
             case S_CNT:
-            case S_NN:
-            case S_ISUM: os << "        if (" << v << ") atomicAdd((unsigned long long*)&" << g << ", (unsigned long long)" << v << ");\n"; break;
-            case S_IMIN: os << "        atomicMin(&" << g << ", " << v << ");\n"; break;
-            case S_IMAX: os << "        atomicMax(&" << g << ", " << v << ");\n"; break;
-            case S_FMIN: os << "        atomicMin((unsigned long long*)&" << g << ", (unsigned long long)" << v << ");\n"; break;
-            case S_FMAX: os << "        atomicMax((unsigned long long*)&" << g << ", (unsigned long long)" << v << ");\n"; break;
+            case S_NN: os << "        { const unsigned v = vq_s_ld(" << w << "); if (v) atomicAdd(" << gu << ", (unsigned long long)v); }\n"; break;
+            case S_ISUM:
+                os << "        { const unsigned long long v = ((unsigned long long)vq_s_ld(" << cache_word(F.at[s] + 1) << ") << 32) | vq_s_ld(" << w
+                   << "); if (v) atomicAdd(" << gu << ", v); }\n";
+                break;
+            case S_IMIN: os << "        atomicMin(&" << g << ", (long long)(" << v8 << " ^ 0x8000000000000000ull));\n"; break;
+            case S_IMAX: os << "        atomicMax(&" << g << ", (long long)(" << v8 << " ^ 0x8000000000000000ull));\n"; break;
+            case S_FMIN: os << "        atomicMin(" << gu << ", " << v8 << ");\n"; break;
+            case S_FMAX: os << "        atomicMax(" << gu << ", " << v8 << ");\n"; break;
             case S_FSUM:
-                if (p.cache_limbs)
-                    os << "        for (int d = 0; d < 4; d++) { const long long x = vq_limbs_digit((const unsigned*)" << L.fx << " + (long long)" << P_
-                       << " * 16 * " << C << " + i, " << C << ", d); if (x) atomicAdd((unsigned long long*)&P.acc_fx[(" << P_
-                       << " * stride + i) * 4 + d], (unsigned long long)x); }\n";
-                else
-                    os << "        for (int d = 0; d < 4; d++) { const long long x = " << L.fx << "[(" << P_ << " * 4 + d) * " << C
-                       << " + i]; if (x) atomicAdd((unsigned long long*)&P.acc_fx[(" << P_ << " * stride + i) * 4 + d], (unsigned long long)x); }\n";
-                os << "        if (" << L.sp << "[" << P_ << " * " << C << " + i]) atomicOr(&P.special[" << P_ << " * stride + i], "
-                   << L.sp << "[" << P_ << " * " << C << " + i]);\n";
+                os << "        vq_s_limbs_flush<" << (slot_signed(p, s) ? "true" : "false") << ">(" << w << ", vq_s4, (vq_i64*)P.acc_fx + (" << pos
+                   << " * stride + slot) * 4);\n";
+                if (!slot_finite(p, s))
+                    os << "        { const unsigned f = vq_s_ld(" << cache_word(F.at[s] + kCacheLimbs) << "); if (f) atomicOr(&P.special[" << pos
+                       << " * stride + slot], f); }\n";
                 break;
         }
-    }
-    os << "    }\n";
-}
-
-// Atomic path with warp aggregation: lanes whose rows fall into the same
-// group (__match_any_sync peers) are reduced with redux.sync and only the
-// lowest such lane updates the group table. Every reduction is exact and
-// order-free: counts and integer sums wrap in 64 bits, MIN/MAX compare order
-// keys, and float sums fold 128-bit fixed-point images of the values (the
-// same integers the single-row update would add). When no two lanes of the
-// warp share a group every lane updates its own row without reducing.
-// Whether the dense path's hot-group registers are generated.
-bool hot_on(const Plan& p) { return p.hot_n > 0 && p.path == AggPath::Dense && !p.is_join && !p.warp_agg; }
-
-// One group's update from values in scope (slot, stride, ag_first, ag<s>,
-// ah<s>, fd<s>_<k>, fsp<s>): the block's shared-memory cache when the slot is
-// cached, else the global table.
-void emit_lead_update(std::ostringstream& os, const Plan& p, const std::string& in3, bool cache) {
-    if (cache) emit_cache_update(os, p, in3);
-    // unguarded (fire-and-forget) MIN/MAX and first-row atomics: a read of the
-    // current value to skip them measured slower on the global table (4M rows,
-    // 65,536 Zipf groups mostly uncached: 118.9 against 74.8 us; 200K hash
-    // keys: 201.6 against 197.7 us)
-    os << in3 << "atomicMin(&P.first[slot], ag_first);\n";
-    for (size_t s = 0; s < p.slots.size(); s++) {
-        std::string S = std::to_string(s);
-        int pos = p.slot_pos[s];
-        std::string ai = "P.acc_i[" + std::to_string(pos) + " * stride + slot]";
-        std::string aiu = "(unsigned long long*)&" + ai;
-        switch (p.slots[s].kind) {
-            case S_CNT:
-            case S_NN: os << in3 << "if (ag" << S << ") atomicAdd(" << aiu << ", (unsigned long long)ag" << S << ");\n"; break;
-            case S_ISUM: os << in3 << "if (ah" << S << ") atomicAdd(" << aiu << ", (unsigned long long)ag" << S << ");\n"; break;
-            case S_IMIN: os << in3 << "if (ah" << S << ") atomicMin(&" << ai << ", ag" << S << ");\n"; break;
-            case S_IMAX: os << in3 << "if (ah" << S << ") atomicMax(&" << ai << ", ag" << S << ");\n"; break;
-            case S_FMIN: os << in3 << "if (ah" << S << ") atomicMin(" << aiu << ", ag" << S << ");\n"; break;
-            case S_FMAX: os << in3 << "if (ah" << S << ") atomicMax(" << aiu << ", ag" << S << ");\n"; break;
-            case S_FSUM:
-                os << in3 << "if (ah" << S << ") { vq_fx_add_digits<true>(P.acc_fx + ((long long)" << pos << " * stride + (long long)slot) * 4, fd"
-                   << S << "_0, fd" << S << "_1, fd" << S << "_2, fd" << S << "_3); if (fsp" << S << ") atomicOr(P.special + (long long)" << pos
-                   << " * stride + slot, fsp" << S << "); }\n";
-                break;
-        }
-    }
-    if (cache) os << in3 << "}\n";  // closes the global branch opened by emit_cache_update
-}
-
-void emit_atomic_update_warp(std::ostringstream& os, const Plan& p, const std::string& ind, const std::string& order,
-                             bool cache) {
-    const std::string in = ind + "    ";
-    os << ind << "unsigned long long slot = VQ_NOSLOT;\n";
-    if (p.path == AggPath::Dense) os << ind << "if (live) slot = key;\n";
-    else os << ind << "if (live) slot = vq_insert(P.keys, P.cap_mask, P.cap, key, nullptr, P.error);\n";
-    os << ind << "live = live && slot != VQ_NOSLOT;\n";
-    os << ind << "const unsigned act = __ballot_sync(0xffffffffu, live);\n";
-    os << ind << "if (live) {\n";
-    os << in << "const long long stride = (long long)P.cap + 1;\n";
-    if (p.warp_agg) {
-        os << in << "const unsigned peers = __match_any_sync(act, (unsigned)slot);\n";
-        os << in << "const bool lead = (__ffs(peers) - 1) == lane;\n";
-        os << in << "const bool solo = __all_sync(act, peers == (1u << lane));\n";
-    } else {
-        os << in << "const unsigned peers = 1u << lane; (void)act;\n";
-        os << in << "const bool lead = true, solo = true;\n";
-    }
-    // per-lane fixed-point images of the float-sum inputs
-    for (size_t s = 0; s < p.slots.size(); s++) {
-        if (p.slots[s].kind != S_FSUM) continue;
-        std::string S = std::to_string(s);
-        os << in << "unsigned fw" << S << "[4], fs" << S << " = 0u; fw" << S << "[0] = fw" << S << "[1] = fw" << S << "[2] = fw" << S
-           << "[3] = 0u;\n";
-        os << in << "if (sok" << S << ") vq_fx_words(sv" << S << ", P.fx_lsb[" << p.slot_pos[s] << "], fw" << S << ", fs" << S
-           << ", P.error);\n";
-    }
-    os << in << "long long ag_first;\n";
-    for (size_t s = 0; s < p.slots.size(); s++) {
-        std::string S = std::to_string(s);
-        switch (p.slots[s].kind) {
-            case S_CNT: case S_NN: os << in << "long long ag" << S << ";\n"; break;
-            case S_ISUM: case S_IMIN: case S_IMAX: os << in << "long long ag" << S << "; bool ah" << S << ";\n"; break;
-            case S_FMIN: case S_FMAX: os << in << "unsigned long long ag" << S << "; bool ah" << S << ";\n"; break;
-            case S_FSUM:
-                os << in << "long long fd" << S << "_0, fd" << S << "_1, fd" << S << "_2, fd" << S << "_3; unsigned fsp" << S << "; bool ah" << S
-                   << ";\n";
-                break;
-        }
-    }
-    // single-row values
-    os << in << "if (solo) {\n";
-    std::string i2 = in + "    ";
-    os << i2 << "ag_first = " << order << ";\n";
-    for (size_t s = 0; s < p.slots.size(); s++) {
-        std::string S = std::to_string(s);
-        switch (p.slots[s].kind) {
-            case S_CNT: os << i2 << "ag" << S << " = 1;\n"; break;
-            case S_NN: os << i2 << "ag" << S << " = sok" << S << " ? 1 : 0;\n"; break;
-            case S_ISUM: case S_IMIN: case S_IMAX: os << i2 << "ag" << S << " = sv" << S << "; ah" << S << " = sok" << S << ";\n"; break;
-            case S_FMIN: case S_FMAX:
-                os << i2 << "ah" << S << " = sok" << S << " && !isnan(sv" << S << "); ag" << S << " = vq_fkey(sv" << S << ");\n";
-                break;
-            case S_FSUM:
-                os << i2 << "fd" << S << "_0 = fw" << S << "[0]; fd" << S << "_1 = fw" << S << "[1]; fd" << S << "_2 = fw" << S << "[2]; fd"
-                   << S << "_3 = (long long)(int)fw" << S << "[3]; fsp" << S << " = fs" << S << "; ah" << S << " = sok" << S << ";\n";
-                break;
-        }
-    }
-    if (p.warp_agg) {
-        // peer reductions
-        os << in << "} else {\n";
-        os << i2 << "ag_first = (long long)vq_wmin64(peers, (unsigned long long)(" << order << "));\n";
-        for (size_t s = 0; s < p.slots.size(); s++) {
-            std::string S = std::to_string(s);
-            std::string any = "__ballot_sync(peers, sok" + S + ") != 0u";
-            switch (p.slots[s].kind) {
-                case S_CNT: os << i2 << "ag" << S << " = __popc(peers);\n"; break;
-                case S_NN: os << i2 << "ag" << S << " = __popc(__ballot_sync(peers, sok" << S << "));\n"; break;
-                case S_ISUM:
-                    os << i2 << "ag" << S << " = (long long)vq_wsum64(peers, sok" << S << " ? (unsigned long long)sv" << S << " : 0ull); ah"
-                       << S << " = " << any << ";\n";
-                    break;
-                case S_IMIN:
-                    os << i2 << "ag" << S << " = (long long)(vq_wmin64(peers, (sok" << S << " ? (unsigned long long)sv" << S
-                       << " : 0x7FFFFFFFFFFFFFFFull) ^ 0x8000000000000000ull) ^ 0x8000000000000000ull); ah" << S << " = " << any << ";\n";
-                    break;
-                case S_IMAX:
-                    os << i2 << "ag" << S << " = (long long)(vq_wmax64(peers, (sok" << S << " ? (unsigned long long)sv" << S
-                       << " : 0x8000000000000000ull) ^ 0x8000000000000000ull) ^ 0x8000000000000000ull); ah" << S << " = " << any << ";\n";
-                    break;
-                case S_FMIN:
-                    os << i2 << "{ const bool o = sok" << S << " && !isnan(sv" << S << "); ag" << S << " = vq_wmin64(peers, o ? vq_fkey(sv" << S
-                       << ") : 0xFFFFFFFFFFFFFFFFull); ah" << S << " = __ballot_sync(peers, o) != 0u; }\n";
-                    break;
-                case S_FMAX:
-                    os << i2 << "{ const bool o = sok" << S << " && !isnan(sv" << S << "); ag" << S << " = vq_wmax64(peers, o ? vq_fkey(sv" << S
-                       << ") : 0ull); ah" << S << " = __ballot_sync(peers, o) != 0u; }\n";
-                    break;
-                case S_FSUM:
-                    os << i2 << "fd" << S << "_0 = vq_wsum32(peers, fw" << S << "[0]); fd" << S << "_1 = vq_wsum32(peers, fw" << S << "[1]); fd" << S
-                       << "_2 = vq_wsum32(peers, fw" << S << "[2]);\n";
-                    os << i2 << "fd" << S << "_3 = vq_wsum32(peers, fw" << S << "[3]) - ((long long)__popc(__ballot_sync(peers, (fw" << S
-                       << "[3] >> 31) != 0u)) << 32);\n";
-                    os << i2 << "fsp" << S << " = vq_redux_or(peers, fs" << S << "); ah" << S << " = " << any << ";\n";
-                    break;
-            }
-        }
-    }
-    os << in << "}\n";
-    if (hot_on(p)) {
-        // the plan's hottest groups accumulate in this thread's registers
-        os << in << "int vq_h = -1;\n";
-        for (int h = 0; h < p.hot_n; h++)
-            os << in << (h ? "else " : "") << "if (slot == P.hot[" << h << "]) vq_h = " << h << ";\n";
-        os << in << "if (vq_h >= 0) {\n";
-        os << in << "    switch (vq_h) {\n";
-        for (int h = 0; h < p.hot_n; h++) {
-            std::string H = std::to_string(h), i4 = in + "        ";
-            os << in << "    case " << h << ": {\n";
-            // a lane meets its rows in increasing order: its first row of the group holds the smallest order key
-            os << i4 << "if (!hs" << H << ") { hs" << H << " = true; hf" << H << " = ag_first; }\n";
-            for (size_t s = 0; s < p.slots.size(); s++) {
-                std::string S = std::to_string(s), v = "hv" + H + "_" + S, hh = "hh" + H + "_" + S;
-                switch (p.slots[s].kind) {
-                    case S_CNT: case S_NN: os << i4 << v << " += ag" << S << ";\n"; break;
-                    case S_ISUM:
-                        os << i4 << "if (ah" << S << ") { " << v << " = (long long)((unsigned long long)" << v << " + (unsigned long long)ag" << S
-                           << "); " << hh << " = true; }\n";
-                        break;
-                    case S_IMIN: case S_FMIN:
-                        os << i4 << "if (ah" << S << " && ag" << S << " < " << v << ") " << v << " = ag" << S << "; " << hh << " = " << hh << " || ah" << S << ";\n";
-                        break;
-                    case S_IMAX: case S_FMAX:
-                        os << i4 << "if (ah" << S << " && ag" << S << " > " << v << ") " << v << " = ag" << S << "; " << hh << " = " << hh << " || ah" << S << ";\n";
-                        break;
-                    case S_FSUM: {
-                        std::string d = "hd" + H + "_" + S + "_";
-                        os << i4 << "if (ah" << S << ") { " << d << "0 += fd" << S << "_0; " << d << "1 += fd" << S << "_1; " << d << "2 += fd" << S << "_2; "
-                           << d << "3 += fd" << S << "_3; hp" << H << "_" << S << " |= fsp" << S << "; " << hh << " = true; }\n";
-                        break;
-                    }
-                }
-            }
-            os << i4 << "break;\n" << in << "    }\n";
-        }
-        os << in << "    }\n" << in << "} else if (lead) {\n";
-    } else {
-        os << in << "if (lead) {\n";
-    }
-    emit_lead_update(os, p, in + "    ", cache);
-    os << in << "}\n" << ind << "}\n";
-}
-
-// The dense path's hot groups: register accumulators (declared at kernel or
-// body scope) and their flush into the cache or the table after the scan.
-void emit_hot_decl(std::ostringstream& os, const Plan& p) {
-    for (int h = 0; h < p.hot_n; h++) {
-        std::string H = std::to_string(h);
-        os << "    bool hs" << H << " = false; long long hf" << H << " = 0x7FFFFFFFFFFFFFFFLL;\n";
-        for (size_t s = 0; s < p.slots.size(); s++) {
-            std::string S = std::to_string(s), v = "hv" + H + "_" + S, hh = "bool hh" + H + "_" + S + " = false;";
-            switch (p.slots[s].kind) {
-                case S_CNT: case S_NN: os << "    long long " << v << " = 0;\n"; break;
-                case S_ISUM: os << "    long long " << v << " = 0; " << hh << "\n"; break;
-                case S_IMIN: os << "    long long " << v << " = 0x7FFFFFFFFFFFFFFFLL; " << hh << "\n"; break;
-                case S_IMAX: os << "    long long " << v << " = (-0x7FFFFFFFFFFFFFFFLL - 1LL); " << hh << "\n"; break;
-                case S_FMIN: os << "    unsigned long long " << v << " = 0xFFFFFFFFFFFFFFFFull; " << hh << "\n"; break;
-                case S_FMAX: os << "    unsigned long long " << v << " = 0ull; " << hh << "\n"; break;
-                case S_FSUM: {
-                    std::string d = "hd" + H + "_" + S + "_";
-                    os << "    long long " << d << "0 = 0, " << d << "1 = 0, " << d << "2 = 0, " << d << "3 = 0; unsigned hp" << H << "_" << S
-                       << " = 0u; " << hh << "\n";
-                    break;
-                }
-            }
-        }
-    }
-}
-
-void emit_hot_flush(std::ostringstream& os, const Plan& p, bool cache) {
-    os << "    {\n        const long long stride = (long long)P.cap + 1;\n";
-    for (int h = 0; h < p.hot_n; h++) {
-        std::string H = std::to_string(h), in = "            ";
-        os << "        if (hs" << H << ") {\n";
-        os << in << "const unsigned long long slot = P.hot[" << h << "];\n";
-        os << in << "const long long ag_first = hf" << H << ";\n";
-        for (size_t s = 0; s < p.slots.size(); s++) {
-            std::string S = std::to_string(s), v = "hv" + H + "_" + S, hh = "hh" + H + "_" + S;
-            switch (p.slots[s].kind) {
-                case S_CNT: case S_NN: os << in << "const long long ag" << S << " = " << v << ";\n"; break;
-                case S_ISUM: case S_IMIN: case S_IMAX: os << in << "const long long ag" << S << " = " << v << "; const bool ah" << S << " = " << hh << ";\n"; break;
-                case S_FMIN: case S_FMAX: os << in << "const unsigned long long ag" << S << " = " << v << "; const bool ah" << S << " = " << hh << ";\n"; break;
-                case S_FSUM: {
-                    std::string d = "hd" + H + "_" + S + "_";
-                    os << in << "const long long fd" << S << "_0 = " << d << "0, fd" << S << "_1 = " << d << "1, fd" << S << "_2 = " << d << "2, fd" << S
-                       << "_3 = " << d << "3; const unsigned fsp" << S << " = hp" << H << "_" << S << "; const bool ah" << S << " = " << hh << ";\n";
-                    break;
-                }
-            }
-        }
-        emit_lead_update(os, p, in, cache);
-        os << "        }\n";
     }
     os << "    }\n";
 }
@@ -1932,37 +1796,44 @@ std::string kernel_head(const std::string& name, int block, int min_blocks = 0) 
 // processed, so a warp keeps two chunks of column data in flight.
 std::string seg_lookup(const std::string& c, const std::string& s0, const std::string& s1, const std::string& r0,
                        const std::string& lane_term = "lane * 4") {
-    return "{ int lo = 0, hi = P.nseg - 1;\n"
+    return "if (P.one_seg) { " + s0 + " = P.row_beg; " + s1 + " = P.row_end; " + r0 + " = (P.row_beg & ~127LL) + " + c + " * 128 + " + lane_term + "; }\n"
+           "        else { int lo = 0, hi = P.nseg - 1;\n"
            "          while (lo < hi) { const int mid = (lo + hi + 1) >> 1; if (P.seg[3 * mid + 2] <= " + c +
            ") lo = mid; else hi = mid - 1; }\n"
            "          " + s0 + " = P.seg[3 * lo]; " + s1 + " = P.seg[3 * lo + 1];\n"
            "          " + r0 + " = (" + s0 + " & ~127LL) + (" + c + " - P.seg[3 * lo + 2]) * 128 + " + lane_term + "; }\n";
 }
 
-void chunk_loop_open(std::ostringstream& os, const Plan& p, const Table* t, const std::set<int>& cols) {
+// block_steps (a kernel with the group cache): every warp of the block walks the
+// same number of steps, counted in vq_step, the ones past the last chunk
+// without a row, so the block can meet between them.
+void chunk_loop_open(std::ostringstream& os, const Plan& p, const Table* t, const std::set<int>& cols, bool block_steps = false) {
+    os << "    const int lane = threadIdx.x & 31;\n"
+          "    const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;\n"
+          "    long long c = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;\n";
+    if (block_steps)
+        os << "    int vq_step = 0;\n"
+              "    const long long vq_cb = ((long long)blockIdx.x * blockDim.x) >> 5;\n";
+    const std::string loop = block_steps ? "    for (long long cb = vq_cb; cb < P.nchunks; cb += nw, c += nw, vq_step++) {\n"
+                                         : "    for (; c < P.nchunks; c += nw) {\n";
+    const std::string row = block_steps ? "        if (c < P.nchunks) {\n" : "";
     if (!p.pipeline) {
-        os << "    const int lane = threadIdx.x & 31;\n"
-              "    const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;\n"
-              "    for (long long c = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; c < P.nchunks; c += nw) {\n"
-              "        long long s0 = 0, s1 = 0, r0 = 0;\n        " << seg_lookup("c", "s0", "s1", "r0");
+        os << loop << row << "        long long s0 = 0, s1 = 0, r0 = 0;\n        " << seg_lookup("c", "s0", "s1", "r0");
         emit_loads(os, p, t, cols, "cv", "cm", "r0", "        ", true);
         return;
     }
-    os << "    const int lane = threadIdx.x & 31;\n"
-          "    const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;\n"
-          "    long long c = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;\n"
-          "    long long s0 = 0, s1 = 0, r0 = 0;\n";
+    os << "    long long s0 = 0, s1 = 0, r0 = 0;\n";
     emit_declare_regs(os, t, cols, "cv", "cm", "    ");
     os << "    if (c < P.nchunks) {\n        " << seg_lookup("c", "s0", "s1", "r0");
     emit_loads(os, p, t, cols, "cv", "cm", "r0", "        ", false);
     os << "    }\n";
-    os << "    for (; c < P.nchunks; c += nw) {\n";
+    os << loop;
     os << "        const long long cn = c + nw;\n";
     os << "        long long ns0 = 0, ns1 = 0, nr0 = 0;\n";
     emit_declare_regs(os, t, cols, "nx", "nm", "        ");
     os << "        if (cn < P.nchunks) {\n        " << seg_lookup("cn", "ns0", "ns1", "nr0");
     emit_loads(os, p, t, cols, "nx", "nm", "nr0", "            ", false);
-    os << "        }\n";
+    os << "        }\n" << row;
 }
 
 // ---- TMA-staged tile loop ---------------------------------------------------------------
@@ -2077,14 +1948,16 @@ void staged_loop_close(std::ostringstream& os, const StageLayout& L, const std::
     os << "        }\n    }\n";
 }
 
-// Closes the pipelined loop: the prefetched chunk becomes the current one.
-void chunk_loop_close(std::ostringstream& os, const Plan& p, const Table* t, const std::set<int>& cols) {
-    if (!p.pipeline) {
-        os << "    }\n";
-        return;
+// Closes the chunk loop: in the pipelined one the prefetched chunk becomes the
+// current one. With block_steps the caller emits what the block does between
+// steps and the loop's closing brace.
+void chunk_loop_close(std::ostringstream& os, const Plan& p, const Table* t, const std::set<int>& cols, bool block_steps = false) {
+    if (block_steps) os << "        }\n";
+    if (p.pipeline) {
+        emit_copy_regs(os, t, cols, "        ");
+        os << "        s0 = ns0; s1 = ns1; r0 = nr0;\n";
     }
-    emit_copy_regs(os, t, cols, "        ");
-    os << "        s0 = ns0; s1 = ns1; r0 = nr0;\n    }\n";
+    if (!block_steps) os << "    }\n";
 }
 
 
@@ -2111,9 +1984,12 @@ AsyncLayout async_layout(const Table* t, const std::set<int>& cols) {
 void emit_async_issue_fn(std::ostringstream& os, const Table* t, const std::set<int>& cols, const AsyncLayout& L,
                          const std::string& name) {
     os << "__device__ __forceinline__ void " << name << "(const VQParams& P, unsigned char* dst, long long cc, int lane) {\n";
-    os << "    int lo = 0, hi = P.nseg - 1;\n";
-    os << "    while (lo < hi) { const int mid = (lo + hi + 1) >> 1; if (P.seg[3 * mid + 2] <= cc) lo = mid; else hi = mid - 1; }\n";
-    os << "    const long long base = (P.seg[3 * lo] & ~127LL) + (cc - P.seg[3 * lo + 2]) * 128;\n";
+    os << "    long long base = (P.row_beg & ~127LL) + cc * 128;\n";
+    os << "    if (!P.one_seg) {\n";
+    os << "        int lo = 0, hi = P.nseg - 1;\n";
+    os << "        while (lo < hi) { const int mid = (lo + hi + 1) >> 1; if (P.seg[3 * mid + 2] <= cc) lo = mid; else hi = mid - 1; }\n";
+    os << "        base = (P.seg[3 * lo] & ~127LL) + (cc - P.seg[3 * lo + 2]) * 128;\n";
+    os << "    }\n";
     for (int c : cols) {
         const int w = type_w(t->cols[c].type);
         os << "    { const unsigned char* src = (const unsigned char*)P.col[" << c << "] + base * " << w << ";\n";
@@ -2179,6 +2055,7 @@ struct ScanLoop {
     AsyncLayout A;
     std::string issue;
     bool staged;
+    bool block_steps = false;  // chunk loop of a kernel with the group cache (chunk_loop_open)
     int async_n = 0;
     int warps = 8;
     ScanLoop(const Plan& pp, const Table* tt, const std::set<int>& cc, int block, const std::string& name, bool allow_async = false)
@@ -2203,18 +2080,21 @@ struct ScanLoop {
     void open(std::ostringstream& os) const {
         if (staged) staged_loop_open(os, t, cols, L, issue);
         else if (async_n) async_loop_open(os, t, cols, A, async_n, issue);
-        else chunk_loop_open(os, p, t, cols);
+        else chunk_loop_open(os, p, t, cols, block_steps);
     }
     void close(std::ostringstream& os) const {
         if (staged) staged_loop_close(os, L, issue);
         else if (async_n) async_loop_close(os);
-        else chunk_loop_close(os, p, t, cols);
+        else chunk_loop_close(os, p, t, cols, block_steps);
     }
 };
 
 }  // namespace
 
-int cache_group_bytes(const Plan& p) { return 8 + 8 * p.ni + (p.cache_limbs ? 68 : 36) * p.nf; }
+int cache_group_bytes(const Plan& p) {
+    const CacheField F = cache_fields(p);
+    return 8 * F.n64 + 4 * F.n32;
+}
 int cache_bytes(const Plan& p) { return p.smem_groups * cache_group_bytes(p); }
 
 static std::string gen_kind_tables(const Plan& p, const std::string& prefix = "P_");
@@ -2222,28 +2102,31 @@ static std::string gen_kind_tables(const Plan& p, const std::string& prefix = "P
 // The four rows a lane holds in the current chunk: filter, project, aggregate.
 static void emit_agg_rows(std::ostringstream& os, Plan& p, const std::vector<int>& key_nodes, bool cache,
                           bool strided = false) {
+    // the chunk's rows inside the range, as offsets from the lane's first
+    os << "        const int vq_lo = (int)max(min(s0 - r0, 128LL), -128LL), vq_hi = (int)max(min(s1 - r0, 128LL), -128LL);\n";
     os << "#pragma unroll\n        for (int k = 0; k < 4; k++) {\n";
-    os << "            const long long r = r0 + " << (strided ? "(k << 5)" : "k") << ";\n";
-    bool warp_sync = p.path != AggPath::Regs;  // atomic paths aggregate across the warp
-    if (warp_sync) os << "            bool live = r >= s0 && r < s1;\n";
-    else os << "            if (r < s0 || r >= s1) continue;\n";
+    const std::string off = strided ? "(k << 5)" : "k";
+    os << "            const long long r = r0 + " << off << ";\n";
+    const bool table = p.path != AggPath::Regs;
+    if (table) os << "            bool live = " << off << " >= vq_lo && " << off << " < vq_hi;\n";
+    else os << "            if (" << off << " < vq_lo || " << off << " >= vq_hi) continue;\n";
     Gen g(p, os);
     if (strided) g.kidx = "(k << 5)";
     if (p.pred >= 0) {
         g.emit(p.pred);
-        if (warp_sync) os << "            live = live && x" << p.pred << " && ok" << p.pred << ";\n";
+        if (table) os << "            live = live && x" << p.pred << " && ok" << p.pred << ";\n";
         else os << "            if (!(x" << p.pred << " && ok" << p.pred << ")) continue;\n";
     }
     for (int k : key_nodes) g.emit(k);
     for (auto& s : p.slots) if (s.input >= 0) g.emit(s.input);
     emit_key(os, p, key_nodes, "            ");
-    emit_slot_values(os, p, "            ", warp_sync ? "live" : "true");
+    emit_slot_values(os, p, "            ", table ? "live" : "true");
     std::string order = order_expr(p, "r");
     if (p.path == AggPath::Regs) {
         if (p.regs_pred) emit_regs_update_pred(os, p, "            ", order);
         else emit_regs_update(os, p, "            ", order);
     } else {
-        emit_atomic_update_warp(os, p, "            ", order, cache);
+        emit_group_update(os, p, "            ", order, cache);
     }
     os << "        }\n";
 }
@@ -2263,12 +2146,15 @@ static std::string gen_agg_kernel(Plan& p, const std::vector<int>& key_nodes, in
     os << kernel_head("vq_agg", block, p.min_blocks);
     if (p.path == AggPath::Regs) emit_regs_decl(os, p);
     if (p.smem_groups > 0) emit_cache_init(os, p);
-    if (hot_on(p)) emit_hot_decl(os, p);
+    loop.block_steps = p.smem_groups > 0;
     loop.open(os);
     emit_agg_rows(os, p, key_nodes, p.smem_groups > 0, loop.strided());
     loop.close(os);
+    if (loop.block_steps) {
+        emit_cache_norm(os, p, block, "vq_step");
+        os << "    }\n";
+    }
     if (p.path == AggPath::Regs) emit_regs_flush(os, p, block);
-    if (hot_on(p)) emit_hot_flush(os, p, p.smem_groups > 0);
     if (p.smem_groups > 0) emit_cache_flush(os, p);
     os << "}\n";
     return os.str();
@@ -2290,12 +2176,19 @@ static std::string gen_agg_body(Plan& p, const std::string& name, int block) {
        << "(const VQParams& P, const long long cbeg, const long long cend, const long long pslot, unsigned char* vq_smem) {\n";
     if (p.path == AggPath::Regs) emit_regs_decl(os, p);
     if (cache) emit_cache_init(os, p, false);
-    if (hot_on(p)) emit_hot_decl(os, p);
     os << "    const int lane = threadIdx.x & 31;\n";
-    os << "    for (long long c = cbeg + (threadIdx.x >> 5); c < cend; c += " << block / 32 << ") {\n";
+    if (cache)  // the block's warps walk the same steps (chunk_loop_open)
+        os << "    int vq_step = 0;\n    for (long long cb = cbeg; cb < cend; cb += " << block / 32 << ", vq_step++) {\n"
+           << "        const long long c = cb + (threadIdx.x >> 5);\n        if (c < cend) {\n";
+    else
+        os << "    for (long long c = cbeg + (threadIdx.x >> 5); c < cend; c += " << block / 32 << ") {\n";
     os << "        long long s0 = 0, s1 = 0, r0 = 0;\n        " << seg_lookup("c", "s0", "s1", "r0");
     emit_loads(os, p, p.t, cols, "cv", "cm", "r0", "        ", true);
     emit_agg_rows(os, p, p.key_nodes, cache);
+    if (cache) {
+        os << "        }\n";
+        emit_cache_norm(os, p, block, "vq_step");
+    }
     os << "    }\n";
     if (p.path == AggPath::Regs) {
         FlushCtx fc;
@@ -2304,7 +2197,6 @@ static std::string gen_agg_body(Plan& p, const std::string& name, int block) {
         fc.dyn_smem = true;
         emit_regs_flush(os, p, block, fc);
     }
-    if (hot_on(p)) emit_hot_flush(os, p, cache);
     if (cache) emit_cache_flush(os, p);
     os << "}\n";
     return os.str();
@@ -2460,6 +2352,7 @@ std::string gen_batch_source(const std::vector<Plan*>& plans, int block, std::ve
 
 int dense_cache_groups(const Plan& p, int cache_kb) {
     if (p.path != AggPath::Dense || p.is_join || cache_kb <= 0) return 0;
+    if (p.t->nrows >= 0xFFFFFFFFLL) return 0;  // an entry's first row is a 32-bit word
     int per = cache_group_bytes(p);
     return (int)std::min<int64_t>(p.domain, (int64_t)cache_kb * 1024 / per);
 }
@@ -3012,11 +2905,15 @@ static const int kBlock = 256;
 static void choose_tunables(Plan& p) {
     int64_t acc = p.path == AggPath::Regs ? p.domain * (int64_t)(p.slots.size() + 1) : 0;
     p.block = acc > 24 ? 128 : 256;
-    // dense group tables with the shared-memory cache: two 512-thread blocks
-    // an SM (32 warps) hide the shared-atomic latency better than 256-thread
-    // blocks at the same cache size (4M Zipf(1.1) rows: 46.1-48.2 / 69.6-76.8
-    // us against 54.3-56.3 / 74.8 us at 1,000 / 65,536 groups)
-    if (p.path == AggPath::Dense && !p.is_join) p.block = 512;
+    // dense group tables with the shared-memory cache: one 1,024-thread block
+    // an SM, so a group's rows meet in as few private entries as can be (fewer
+    // first-row, MIN and MAX improvements, half the cache init and flush of two
+    // 512-thread blocks). 4M Zipf(1.1) rows, SUM COUNT MIN MAX AVG, 1,000 /
+    // 4,000 / 20,000 groups: 42.0 / 53.3 / 57.3 us against 47.2 / 57.6 / 61.4.
+    // Tables too small to give every SM such a block take 512 threads (50K
+    // rows, 2,000 groups: 12.3 against 14.5 us; at 400K rows it is 16.5 against
+    // 16.4)
+    if (p.path == AggPath::Dense && !p.is_join) p.block = p.t->nrows >= 300000 ? 1024 : 512;
     // measured: software prefetch costs registers the register-accumulator path
     // needs (6M-row Q1: 74.9 µs without, 87.0 µs with); neutral for Q6
     // joins (measured, 6M-row probe): prefetch helps the register path and
@@ -3024,22 +2921,6 @@ static void choose_tunables(Plan& p) {
     p.pipeline = p.is_join ? p.path == AggPath::Regs : p.path != AggPath::Regs;
     p.staged = false;  // measured: TMA staging is not faster for these scans yet
     p.regs_pred = true;
-    // measured on Zipf(1.1) keys: per-lane shared-memory atomics beat folding
-    // the peers of a warp first (the fold serialises over distinct groups)
-    p.warp_agg = false;
-    // dense path, shared-memory cache: 32-bit atomics (a 64-bit shared atomic
-    // add measured 6x slower than a 32-bit one, 50x with a hot address). 4M
-    // Zipf(1.1) rows, 1,000 / 65,536 groups: 60 / 75 us against 124 / 142 us
-    // with 64-bit adds; the hottest groups in registers (hot=N) then cost more
-    // than they save (67 / 82 us with one)
-    p.cache_cnt32 = p.cache_fx32 = true;
-    p.hot_n = 0;
-    // float sums in the cache as 16-bit limbs with plain adds (no returned
-    // value, no carry) instead of 32-bit word pairs whose carry comes back
-    // from the returned old value: more atomics a row, measured slower (4M
-    // Zipf rows, 1,000 / 65,536 groups: 54.2 / 79.1 against 48.2 / 76.8 us),
-    // so a tunable (limbs=1)
-    p.cache_limbs = false;
     // register path with many accumulators: three 128-thread blocks an SM
     // (~148 registers a thread), too few loads in flight to fill HBM; a
     // two-chunk cp.async pipeline a warp keeps the next chunk's columns in
@@ -3062,8 +2943,7 @@ static void choose_tunables(Plan& p) {
         };
         int b = get("block="), pl = get("pipeline="), st = get("staged="), sb = get("stage_kb="), rp = get("regs_pred=");
         if (rp >= 0) p.regs_pred = rp != 0;
-        int ck = get("cache_kb="), wa = get("warp_agg="), as = get("async="), mb = get("minb="), ho = get("hot=");
-        int c32 = get("cnt32="), f32 = get("fx32="), gs = get("gsm="), cs = get("cs=");
+        int ck = get("cache_kb="), as = get("async="), mb = get("minb="), gs = get("gsm="), cs = get("cs=");
         if (cs >= 0) p.stream_loads = cs != 0;
         const int kt = get("keep=");
         if (kt >= 0) p.keep_tables = kt != 0;
@@ -3080,31 +2960,18 @@ static void choose_tunables(Plan& p) {
         const int gr = get("graph=");
         if (gr == 0) p.graph_off = true;  // register-path runs as direct launches, not a replayed graph
         if (gs >= 0) p.grid_per_sm = gs;
-        const int lb = get("limbs=");
-        if (lb >= 0) p.cache_limbs = lb != 0;
-        if (c32 >= 0) p.cache_cnt32 = c32 != 0;
-        if (f32 >= 0) p.cache_fx32 = f32 != 0;
-        if (ho >= 0 && p.path == AggPath::Dense && !p.is_join) p.hot_n = std::min(ho, VQ_MAXHOT);
         if (as >= 0) p.async_stages = as;
         if (mb >= 0) p.min_blocks = mb;
         if (ck >= 0) cache_kb = ck;
-        if (wa >= 0) p.warp_agg = wa != 0;
-        if (b == 64 || b == 128 || b == 256 || b == 384 || b == 512) p.block = b;
+        if (b == 64 || b == 128 || b == 256 || b == 384 || b == 512 || b == 1024) p.block = b;
         const int ml = get("mlast=");
         if (ml >= 0) p.merge_last = ml != 0;
         if (pl >= 0) p.pipeline = pl != 0;
         if (st >= 0) p.staged = st != 0;
         if (sb > 0) p.stage_budget = sb * 1024;
     }
-    // limbs take one row's canonical image at a time: not with warp folds or
-    // the register hot groups, which add sums of several rows
-    if (p.warp_agg || p.hot_n > 0) p.cache_limbs = false;
-    p.smem_groups = 0;
-    if (p.path == AggPath::Dense && !p.is_join && cache_kb > 0) {
-        int per = cache_group_bytes(p);
-        p.smem_groups = (int)std::min<int64_t>(p.domain, (int64_t)cache_kb * 1024 / per);
-        p.staged = false;  // the cache owns the dynamic shared memory
-    }
+    p.smem_groups = dense_cache_groups(p, cache_kb);
+    if (p.smem_groups > 0) p.staged = false;  // the cache owns the dynamic shared memory
 }
 
 static void finish_compile(Plan& p, const std::vector<int>& key_nodes, bool join, int build_key_node) {
@@ -3209,9 +3076,7 @@ static void finish_compile(Plan& p, const std::vector<int>& key_nodes, bool join
        << (p.staged ? " staged=tma" : (p.async_stages > 1 && p.path == AggPath::Regs) ? " async=" + std::to_string(p.async_stages)
            : p.pipeline ? " pipeline=1" : " pipeline=0")
        << (p.min_blocks > 0 ? " minb=" + std::to_string(p.min_blocks) : std::string())
-       << " tile=" << p.tile << " smem=" << p.smem << " smem_groups=" << p.smem_groups << " warp_agg=" << p.warp_agg;
-    if (hot_on(p)) ex << " hot_groups=" << p.hot_n;
-    if (p.path == AggPath::Dense && !join && !(p.cache_cnt32 && p.cache_fx32)) ex << " atomics64";
+       << " tile=" << p.tile << " smem=" << p.smem << " smem_groups=" << p.smem_groups;
     if (p.join_gid) ex << " groups=build_key_numbers";
     if (p.path == AggPath::Regs && !join) {
         int nx = 0, nm = 0, na = 0;
@@ -3918,10 +3783,6 @@ void check_ranges(const Plan& p) {
 }
 
 void set_plan_constants(const Plan& p, VQParams& P) {
-    {
-        std::lock_guard<std::mutex> lk(p.hot_mu);
-        for (int h = 0; h < VQ_MAXHOT; h++) P.hot[h] = h < (int)p.hot_keys.size() ? p.hot_keys[h] : ~0ull;
-    }
     for (size_t i = 0; i < p.lits.size() && i < VQ_MAXLITS; i++) P.lit[i] = p.lits[i];
     for (size_t f = 0; f < p.fx_lsb.size() && f < 16; f++) P.fx_lsb[f] = p.fx_lsb[f];
     P.cache_n = p.smem_groups;

@@ -134,160 +134,168 @@ __device__ __forceinline__ void vq_fx_add(vq_i64* c, double x, int lsb, unsigned
     }
 }
 
-// The same fixed-point image as a 128-bit two's-complement integer in four
-// 32-bit words (w[0] least significant), for folding the values of several
-// lanes before one accumulator update. Magnitudes above 2^121 (impossible
-// inside the window's bounds) raise err bit 1 so a 32-value fold cannot wrap.
-__device__ __forceinline__ void vq_fx_words(double x, int lsb, unsigned* w, unsigned& special, int* err) {
-    w[0] = w[1] = w[2] = w[3] = 0u;
+// ---- 32-bit shared-memory accesses by address (the block's group cache).
+// A batch body gets the cache's base as an argument, where a pointer would be
+// generic; shared-window addresses keep the accesses native in both. ----
+__device__ __forceinline__ unsigned vq_s_ld(unsigned a) {
+    unsigned v;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ vq_u64 vq_s_ld64(unsigned a) {
+    vq_u64 v;
+    asm volatile("ld.shared.u64 %0, [%1];" : "=l"(v) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ void vq_s_st(unsigned a, unsigned v) { asm volatile("st.shared.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory"); }
+__device__ __forceinline__ void vq_s_st64(unsigned a, vq_u64 v) { asm volatile("st.shared.u64 [%0], %1;" ::"r"(a), "l"(v) : "memory"); }
+__device__ __forceinline__ unsigned vq_s_atom(unsigned a, unsigned v) {
+    unsigned old;
+    asm volatile("atom.shared.add.u32 %0, [%1], %2;" : "=r"(old) : "r"(a), "r"(v));
+    return old;
+}
+__device__ __forceinline__ void vq_s_add(unsigned a, unsigned v) { asm volatile("red.shared.add.u32 [%0], %1;" ::"r"(a), "r"(v)); }
+__device__ __forceinline__ void vq_s_or(unsigned a, unsigned v) { asm volatile("red.shared.or.b32 [%0], %1;" ::"r"(a), "r"(v)); }
+__device__ __forceinline__ void vq_s_min(unsigned a, unsigned v) { asm volatile("red.shared.min.u32 [%0], %1;" ::"r"(a), "r"(v)); }
+__device__ __forceinline__ void vq_s_min64(unsigned a, vq_u64 v) { asm volatile("red.shared.min.u64 [%0], %1;" ::"r"(a), "l"(v)); }
+__device__ __forceinline__ void vq_s_max64(unsigned a, vq_u64 v) { asm volatile("red.shared.max.u64 [%0], %1;" ::"r"(a), "l"(v)); }
+// A 64-bit sum as two words: the low one returns its old value for the carry.
+__device__ __forceinline__ void vq_s_add64(unsigned lo, unsigned hi, vq_u64 v) {
+    const unsigned l = (unsigned)v, old = vq_s_atom(lo, l), h = (unsigned)(v >> 32) + (old + l < old);
+    if (h) vq_s_add(hi, h);
+}
+
+// x as an integer multiple of 2^lsb: its 53-bit magnitude (mh, lo) and the
+// position sh of bit 0 above the window's LSB (the window's bound keeps |x|
+// below 2^(lsb + 97), so sh <= 44). Bits below 2^lsb are truncated. Returns
+// false where nothing is added: NaN and infinities, which set flags instead,
+// and values below the window. kFinite: x is never NaN or infinite.
+template <bool kFinite>
+__device__ __forceinline__ bool vq_fx_image(double x, int lsb, unsigned& mh, unsigned& lo, int& sh, unsigned& special, int* err) {
+    const unsigned hi = (unsigned)__double2hiint(x);
+    lo = (unsigned)__double2loint(x);
+    const int e = (int)((hi >> 20) & 0x7FF);
+    mh = hi & 0xFFFFFu;
     special = 0u;
-    vq_u64 b = (vq_u64)__double_as_longlong(x);
-    int e = (int)((b >> 52) & 0x7FF);
-    if (e == 0x7FF) {
-        special = (b & 0xFFFFFFFFFFFFFull) ? 1u : ((b >> 63) ? 4u : 2u);
+    if (!kFinite && e == 0x7FF) {
+        special = (mh | lo) ? 1u : ((hi >> 31) ? 4u : 2u);
+        return false;
+    }
+    if (e) mh |= 0x100000u;
+    sh = (e ? e : 1) - 1075 - lsb;
+    if ((unsigned)sh <= 44u) return true;
+    if (sh > 44) {  // outside the window's bound
+        atomicOr(reinterpret_cast<unsigned*>(err), 2u);
+        return false;
+    }
+    if (sh <= -53) return false;
+    const vq_u64 m = (((vq_u64)mh << 32) | lo) >> -sh;
+    mh = (unsigned)(m >> 32);
+    lo = (unsigned)m;
+    sh = 0;
+    return true;
+}
+
+// A float sum in the block's group cache: seven 32-bit counters s bytes apart,
+// each the sum of one limb of the values' images (limb j weighs
+// 2^(W j - VQ_LIMB_SHIFT(W)) units of the window's LSB, so that the window's bound
+// lies on a limb boundary and the largest binades take three limbs). Adds that
+// return nothing merge the lanes of one address into one pass (Zipf keys over
+// 1,000 groups: 2.6 cycles a warp, against 6.5 for adds that return the old
+// value, as a carry needs, and 390 for 64-bit adds), so no carry is taken
+// until vq_s_limbs_norm. Unsigned limbs of 19 bits, or signed ones of 18 where
+// x may be negative, hold VQ_LIMB_ROWS rows between two normalisations.
+#define VQ_LIMBS 7
+#define VQ_LIMB_ROWS 8191u
+template <bool kSigned> __device__ __forceinline__ constexpr int vq_limb_bits() { return kSigned ? 18 : 19; }
+template <bool kSigned> __device__ __forceinline__ constexpr int vq_limb_shift() { return 6 * vq_limb_bits<kSigned>() - 97; }
+template <bool kFinite, bool kSigned>
+__device__ __forceinline__ void vq_s_fx_add(unsigned a, unsigned s, double x, int lsb, int* err) {
+    constexpr int W = vq_limb_bits<kSigned>(), kShift = vq_limb_shift<kSigned>();
+    constexpr unsigned M = (1u << W) - 1u;
+    unsigned mh, lo, special;
+    int sh;
+    if (!vq_fx_image<kFinite>(x, lsb, mh, lo, sh, special, err)) {
+        if (!kFinite && special) vq_s_or(a + VQ_LIMBS * s, special);
         return;
     }
-    vq_u64 m = b & 0xFFFFFFFFFFFFFull;
-    if (e == 0) { if (m == 0) return; e = 1; } else m |= 1ull << 52;
-    int sh = e - 1075 - lsb;
-    if (sh < 0) {
-        if (sh <= -53) return;
-        m >>= -sh;
-        sh = 0;
+    sh += kShift;  // 0 … 61
+    const int j = (int)(((unsigned)sh * (65536u / W + 1u)) >> 16), off = sh - j * W;
+    const unsigned t0 = lo << off, t1 = __funnelshift_l(lo, mh, off), t2 = __funnelshift_l(mh, 0u, off);
+    unsigned l0 = t0 & M, l1 = __funnelshift_r(t0, t1, W) & M, l2 = (t1 >> (2 * W - 32)) & M, l3 = __funnelshift_r(t1, t2, 3 * W - 32);
+    if (kSigned && x < 0.0) {
+        l0 = 0u - l0;
+        l1 = 0u - l1;
+        l2 = 0u - l2;
+        l3 = 0u - l3;
     }
-    if (sh > 69) { atomicOr(reinterpret_cast<unsigned*>(err), 2u); return; }
-    vq_u64 lo = sh < 64 ? m << sh : 0ull;
-    vq_u64 hi = sh == 0 ? 0ull : (sh < 64 ? m >> (64 - sh) : m << (sh - 64));
-    if (b >> 63) { lo = ~lo + 1ull; hi = ~hi + (lo == 0ull ? 1ull : 0ull); }
-    w[0] = (unsigned)lo; w[1] = (unsigned)(lo >> 32); w[2] = (unsigned)hi; w[3] = (unsigned)(hi >> 32);
+    a += (unsigned)j * s;
+    vq_s_add(a, l0);
+    vq_s_add(a + s, l1);
+    vq_s_add(a + 2 * s, l2);
+    if (l3) vq_s_add(a + 3 * s, l3);
 }
-
-// Adds carry-save digits (d[k] weighs 2^(32k+lsb)) to the four counters.
-template <bool kAtomic>
-__device__ __forceinline__ void vq_fx_add_digits(vq_i64* c, vq_i64 d0, vq_i64 d1, vq_i64 d2, vq_i64 d3) {
-    if (kAtomic) {
-        if (d0) atomicAdd(reinterpret_cast<unsigned long long*>(c + 0), (unsigned long long)d0);
-        if (d1) atomicAdd(reinterpret_cast<unsigned long long*>(c + 1), (unsigned long long)d1);
-        if (d2) atomicAdd(reinterpret_cast<unsigned long long*>(c + 2), (unsigned long long)d2);
-        if (d3) atomicAdd(reinterpret_cast<unsigned long long*>(c + 3), (unsigned long long)d3);
-    } else {
-        c[0] += d0; c[1] += d1; c[2] += d2; c[3] += d3;
+// Moves what each limb holds above its width into the next one up; no other
+// thread touches the entry meanwhile.
+template <bool kSigned>
+__device__ __forceinline__ void vq_s_limbs_norm(unsigned a, unsigned s) {
+    constexpr int W = vq_limb_bits<kSigned>();
+    unsigned carry = 0u;
+    for (int j = 0; j < VQ_LIMBS - 1; j++) {
+        const unsigned v = vq_s_ld(a + j * s) + carry;
+        carry = kSigned ? (unsigned)((int)v >> W) : v >> W;
+        vq_s_st(a + j * s, v & ((1u << W) - 1u));
     }
+    if (carry) vq_s_st(a + (VQ_LIMBS - 1) * s, vq_s_ld(a + (VQ_LIMBS - 1) * s) + carry);
 }
-
-// The same with the four counters `stride` words apart: the shared-memory
-// group cache keeps digit d of every group contiguous, so the lanes of a warp
-// updating different groups spread over the banks.
-__device__ __forceinline__ void vq_fx_add_digits_s(vq_i64* c, long long stride, vq_i64 d0, vq_i64 d1, vq_i64 d2, vq_i64 d3) {
-    if (d0) atomicAdd(reinterpret_cast<unsigned long long*>(c), (unsigned long long)d0);
-    if (d1) atomicAdd(reinterpret_cast<unsigned long long*>(c + stride), (unsigned long long)d1);
-    if (d2) atomicAdd(reinterpret_cast<unsigned long long*>(c + 2 * stride), (unsigned long long)d2);
-    if (d3) atomicAdd(reinterpret_cast<unsigned long long*>(c + 3 * stride), (unsigned long long)d3);
-}
-
-// The four digits with 32-bit shared-memory atomics (vq_add64_as32).
-__device__ __forceinline__ void vq_fx_add_digits_s32(vq_i64* c, long long stride, vq_i64 d0, vq_i64 d1, vq_i64 d2, vq_i64 d3) {
-    vq_add64_as32(c, d0);
-    vq_add64_as32(c + stride, d1);
-    vq_add64_as32(c + 2 * stride, d2);
-    vq_add64_as32(c + 3 * stride, d3);
-}
-
-// The shared-memory group cache in limb form: a float sum's 128-bit fixed-point
-// image as eight 16-bit limbs of its magnitude, each added with a plain 32-bit
-// atomic (no returned value, no carry) into its own counter, positive and
-// negative values in separate sets of eight (L[j * C], L[(8 + j) * C]). A
-// counter takes at most 0xFFFF a row, so 32,768 rows of a group between two
-// normalisations (vq_limbs_norm) keep every counter below 2^31. d0..d3 are
-// the canonical 32-bit words of the two's-complement image (d3 signed).
-__device__ __forceinline__ void vq_limbs_add(unsigned* L, long long C, long long d0, long long d1, long long d2, long long d3) {
-    unsigned m0 = (unsigned)d0, m1 = (unsigned)d1, m2 = (unsigned)d2, m3 = (unsigned)d3;
-    if (d3 < 0) {  // magnitude of a negative image: ~x + 1 over 128 bits
-        m0 = ~m0; m1 = ~m1; m2 = ~m2; m3 = ~m3;
-        m0 += 1u;
-        const unsigned c0 = m0 == 0u;
-        m1 += c0;
-        const unsigned c1 = c0 & (m1 == 0u);
-        m2 += c1;
-        m3 += c1 & (m2 == 0u);
-        L += 8 * C;
-    }
-    const unsigned m[4] = {m0, m1, m2, m3};
+// The entry's sum in units of the window's LSB, added to the global table's
+// four 64-bit counters of 32-bit digits.
+template <bool kSigned>
+__device__ __forceinline__ void vq_s_limbs_flush(unsigned a, unsigned s, vq_i64* c) {
+    constexpr int W = vq_limb_bits<kSigned>(), kShift = vq_limb_shift<kSigned>();
+    vq_i64 d[VQ_FX_DIGITS] = {0, 0, 0, 0};
+    vq_i64 carry = 0;  // of the limbs below, in units of the limb at hand
 #pragma unroll
-    for (int j = 0; j < 8; j++) {
-        const unsigned limb = (m[j >> 1] >> (16 * (j & 1))) & 0xFFFFu;
-        if (limb) atomicAdd(L + j * C, limb);
-    }
-}
-// Moves every counter's bits above 16 into the next limb up (both sets; the
-// top limb keeps its high bits): atomic, so adds landing meanwhile are kept.
-__device__ __forceinline__ void vq_limbs_norm(unsigned* L, long long C) {
-#pragma unroll
-    for (int s = 0; s < 2; s++)
-#pragma unroll
-        for (int j = 0; j < 7; j++) {
-            const unsigned old = atomicAnd(L + (8 * s + j) * C, 0xFFFFu);
-            if (old >> 16) atomicAdd(L + (8 * s + j + 1) * C, old >> 16);
+    for (int j = 0; j < VQ_LIMBS; j++) {
+        const unsigned raw = vq_s_ld(a + j * s);
+        vq_i64 v = (kSigned ? (vq_i64)(int)raw : (vq_i64)raw) + carry;
+        if (j < VQ_LIMBS - 1) {
+            carry = v >> W;
+            v &= (1 << W) - 1;
         }
-}
-// The block's limbs as the global table's carry-save digit d (weight 2^(32d)).
-__device__ __forceinline__ long long vq_limbs_digit(const unsigned* L, long long C, int d) {
-    return (long long)L[(2 * d) * C] + ((long long)L[(2 * d + 1) * C] << 16) - (long long)L[(8 + 2 * d) * C] -
-           ((long long)L[(8 + 2 * d + 1) * C] << 16);
+        // bits [W j - kShift, …) of the sum: values hold no bit below the LSB
+        const int at = W * j - kShift;
+        if (at < 0) {
+            d[0] += v >> -at;
+        } else {
+            d[at >> 5] += (vq_i64)((vq_u64)v << (at & 31));
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < VQ_FX_DIGITS; k++)
+        if (d[k]) atomicAdd(reinterpret_cast<unsigned long long*>(c + k), (unsigned long long)d[k]);
 }
 
-// ---- warp reductions over a peer mask (redux.sync; every lane named in the
-// mask executes the same call with the same mask) ----
-__device__ __forceinline__ unsigned vq_redux_add(unsigned mask, unsigned v) {
-    unsigned r;
-    asm volatile("redux.sync.add.u32 %0, %1, %2;" : "=r"(r) : "r"(v), "r"(mask));
-    return r;
-}
-__device__ __forceinline__ unsigned vq_redux_min(unsigned mask, unsigned v) {
-    unsigned r;
-    asm volatile("redux.sync.min.u32 %0, %1, %2;" : "=r"(r) : "r"(v), "r"(mask));
-    return r;
-}
-__device__ __forceinline__ unsigned vq_redux_max(unsigned mask, unsigned v) {
-    unsigned r;
-    asm volatile("redux.sync.max.u32 %0, %1, %2;" : "=r"(r) : "r"(v), "r"(mask));
-    return r;
-}
-__device__ __forceinline__ unsigned vq_redux_or(unsigned mask, unsigned v) {
-    unsigned r;
-    asm volatile("redux.sync.or.b32 %0, %1, %2;" : "=r"(r) : "r"(v), "r"(mask));
-    return r;
-}
-// Sum of one 32-bit word over the peers, exact in 64 bits (two 16-bit halves).
-__device__ __forceinline__ vq_i64 vq_wsum32(unsigned mask, unsigned v) {
-    return (vq_i64)vq_redux_add(mask, v & 0xFFFFu) + ((vq_i64)vq_redux_add(mask, v >> 16) << 16);
-}
-// Wrapping 64-bit sum over the peers (four 16-bit quarters).
-__device__ __forceinline__ vq_u64 vq_wsum64(unsigned mask, vq_u64 v) {
-    vq_u64 r = 0;
+// The same sum in the global table: four 64-bit counters of signed 32-bit
+// digits (vq_fx_add's), at most three of them touched by a value.
+template <bool kFinite, bool kSigned>
+__device__ __forceinline__ void vq_g_fx_add(vq_i64* c, unsigned* sp, double x, int lsb, int* err) {
+    unsigned mh, lo, special;
+    int sh;
+    if (!vq_fx_image<kFinite>(x, lsb, mh, lo, sh, special, err)) {
+        if (!kFinite && special) atomicOr(sp, special);
+        return;
+    }
+    const int off = sh & 31;
+    const unsigned t[3] = {lo << off, __funnelshift_l(lo, mh, off), __funnelshift_l(mh, 0u, off)};
+    unsigned long long* p = reinterpret_cast<unsigned long long*>(c + (sh >> 5));
 #pragma unroll
-    for (int q = 0; q < 4; q++) r += (vq_u64)vq_redux_add(mask, (unsigned)(v >> (16 * q)) & 0xFFFFu) << (16 * q);
-    return r;
-}
-// Unsigned 64-bit min / max over the peers: the high words first, then the
-// low words among the lanes holding the extreme high word.
-__device__ __forceinline__ vq_u64 vq_wmin64(unsigned mask, vq_u64 v) {
-    const unsigned h = (unsigned)(v >> 32);
-    const unsigned mh = vq_redux_min(mask, h);
-    const unsigned m2 = __ballot_sync(mask, h == mh);
-    unsigned ml = 0u;
-    if (h == mh) ml = vq_redux_min(m2, (unsigned)v);
-    ml = __shfl_sync(mask, ml, __ffs(m2) - 1);
-    return ((vq_u64)mh << 32) | ml;
-}
-__device__ __forceinline__ vq_u64 vq_wmax64(unsigned mask, vq_u64 v) {
-    const unsigned h = (unsigned)(v >> 32);
-    const unsigned mh = vq_redux_max(mask, h);
-    const unsigned m2 = __ballot_sync(mask, h == mh);
-    unsigned ml = 0u;
-    if (h == mh) ml = vq_redux_max(m2, (unsigned)v);
-    ml = __shfl_sync(mask, ml, __ffs(m2) - 1);
-    return ((vq_u64)mh << 32) | ml;
+    for (int k = 0; k < 3; k++) {
+        if (!t[k]) continue;
+        unsigned long long v = t[k];
+        if (kSigned && x < 0.0) v = 0ull - v;
+        atomicAdd(p + k, v);
+    }
 }
 
 __device__ __host__ inline int vq_clz64(vq_u64 x) {

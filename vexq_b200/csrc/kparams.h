@@ -7,7 +7,6 @@
 #define VQ_MAXSETS 16
 #define VQ_FX_DIGITS 4  // 32-bit digits of the exact fixed-point float sums
 #define VQ_MAXLITS 32   // numeric literals passed at launch (raw 8-byte images)
-#define VQ_MAXHOT 4     // dense path: hottest groups accumulated in registers
 #define VQ_RADIX_CAP 4096      // radix join: build entries of one partition held in shared memory
 #define VQ_RADIX_MAX_BITS 12   // radix join: at most 4,096 partitions
 #define VQ_MAXDIST 4    // COUNT(DISTINCT) aggregates of one plan
@@ -106,16 +105,17 @@ struct VQParams {
     long long lit[VQ_MAXLITS];
     // ---- 8-byte scalars ----
     long long nchunks;
+    long long row_beg, row_end;    // one_seg: the only row range (its chunks start at 0)
     long long rg_rows;
     unsigned long long cap_mask;   // atomic path: capacity - 1 (hash) or unused (dense)
     unsigned long long cap;        // slots (hash: power of two; dense: domain)
     unsigned long long jmask;      // join table capacity - 1
-    unsigned long long hot[VQ_MAXHOT];  // dense path: groups a thread accumulates in registers (~0 = none)
     // ---- 4-byte scalars ----
     int nseg;
+    int one_seg;               // 1: a single row range, read from here instead of seg
     int n_rg;
     int mode;                  // join build: 0 = insert/count, 1 = fill, 2 = unique keys into jslot, 3 = unique keys into dmap
-    int cache_n;               // dense path: groups held in the block's shared-memory cache
+    int cache_n;               // dense path: groups held in the block's shared-memory cache (the first codes and the last)
     int nparts;                // radix join: partitions (a power of two)
     int pbits;                 // radix join: partition = top pbits bits of the key hash
     int fx_lsb[16];            // per float-sum slot: exponent of the window's LSB

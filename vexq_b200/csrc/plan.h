@@ -182,7 +182,6 @@ struct Plan {
     bool pipeline = true;
     bool staged = true;        // TMA bulk-copy staging of row tiles into shared memory
     bool regs_pred = true;     // register path: branch-free predicated updates
-    bool warp_agg = true;      // atomic path: fold lanes of one group before updating
     int smem_groups = 0;       // dense path: groups cached in block-private shared memory
     int stage_budget = 0;      // bytes of the stage ring per block (0: default)
     int tile = 128, smem = 0;  // main kernel: rows per loop unit, dynamic shared memory
@@ -245,16 +244,6 @@ struct Plan {
     ScanMemo scan_memo;                    // main-table pruning of the last run's row-group range
     ScanMemo build_memo;                   // join build side's pruning (whole table), until its zone maps change
     long long hash_groups_seen = -1;       // hash path: groups the last run found (sizes the next table)
-    // dense path: the kernel accumulates hot_n groups per thread in registers;
-    // which groups is a launch value, the largest-count groups of the last run
-    int hot_n = 0;
-    // dense path, shared-memory cache: counts added as 32-bit atomics on the
-    // counter's low word; fixed-point digits as 32-bit atomics with the carry
-    // (from the returned old value) added to the high word
-    bool cache_cnt32 = false, cache_fx32 = false;
-    bool cache_limbs = false;      // cached float sums as 16-bit limbs (plain adds, normalised every 32,768 rows)
-    std::vector<unsigned long long> hot_keys;
-    mutable std::mutex hot_mu;
     long long hash_rows_seen = 0;          //   and the rows that run scanned
     // group tables assembled on the device (assemble.cu)
     OutPool out_pool;
@@ -359,9 +348,6 @@ vexq_result_s* build_result(Plan& p, Groups& g);
 // Gives the result's STRING columns dictionaries of their own (the strings
 // they use, codes renumbered), so the result outlives the tables it read.
 void own_dictionaries(vexq_result_s* r);
-// Dense path: the groups with the largest counts of a finished run become the
-// groups the next run accumulates in registers.
-void note_hot_groups(Plan& p, const Groups& g);
 int64_t scanned_bytes(const Plan& p, const Table& t, long long rows, bool build);
 long long estimate_groups(const Plan& p, long long rows, long long join_keys);
 void set_columns(VQParams& P, const Table& t, bool build_side);
@@ -452,6 +438,13 @@ long long walk_segments(const Table& t, Keep&& keep, int rg_start, int rg_end, i
         rg = e;
     }
     return chunks;
+}
+// A scan over one row range finds it in the parameter block: no search and no
+// loads ahead of the column loads (the usual case: no row group pruned).
+inline void set_one_seg(VQParams& P, const std::vector<long long>& seg) {
+    P.one_seg = seg.size() == 3;
+    P.row_beg = P.one_seg ? seg[0] : 0;
+    P.row_end = P.one_seg ? seg[1] : 0;
 }
 // Grid of a scan kernel: every SM filled to its occupancy (at most cap_per_sm
 // blocks an SM when > 0), never more blocks than loop units.

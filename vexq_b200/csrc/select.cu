@@ -214,6 +214,7 @@ VQParams select_params(Plan& p, const Table& t, const DevBuf& seg, const ScanSeg
     set_columns(P, t, false);
     P.seg = seg.as<long long>();
     P.nseg = (int)ss.seg.size() / 3;
+    set_one_seg(P, ss.seg);
     P.nchunks = ss.nchunks;
     P.rg_rows = t.rg_rows;
     P.n_rg = t.n_rg;
