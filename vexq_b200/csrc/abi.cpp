@@ -305,7 +305,8 @@ int32_t vexq_filter_run(vexq_table_t t, const vexq_expr* nodes, int32_t nnodes, 
         Table& tb = *t->t;
         if (row_end < 0 || row_end > tb.nrows) row_end = tb.nrows;
         if (row_start < 0 || row_start > row_end) fail(VEXQ_EINVAL, "row range out of bounds");
-        std::unique_ptr<Plan> p(compile_filter(&tb, nodes, nnodes, children, nchildren, predicate));
+        SelectLease lease(tb, 'f', nodes, nnodes, children, nchildren, predicate, nullptr, 0);
+        Plan* p = lease.p.get();
         // one segment [row_start, row_end)
         std::vector<long long> seg;
         long long chunks = 0;
@@ -314,8 +315,10 @@ int32_t vexq_filter_run(vexq_table_t t, const vexq_expr* nodes, int32_t nnodes, 
             seg = {row_start, row_end, 0};
             chunks = (row_end - (row_start & ~(U - 1)) + U - 1) / U;
         }
-        size_t words = (size_t)(tb.nrows + kPadRows) / 32 + 8;
-        DevBuf bits(words * 4), dseg(24), scal(32);
+        // count and error word, then the bitmap (bit r = table row r)
+        const size_t words = (size_t)(tb.nrows + kPadRows) / 32 + 8;
+        p->scratch_a.ensure(64 + words * 4);
+        char* base = p->scratch_a.as<char>();
         VQParams P;
         std::memset(&P, 0, sizeof P);
         for (size_t c = 0; c < tb.cols.size(); c++) {
@@ -326,42 +329,42 @@ int32_t vexq_filter_run(vexq_table_t t, const vexq_expr* nodes, int32_t nnodes, 
         P.present = p->d_present.as<unsigned char>();
         P.rg_rows = tb.rg_rows;
         P.n_rg = tb.n_rg;
-        P.acc_i = bits.as<long long>();
-        P.ngroups = scal.as<unsigned long long>();
-        P.error = (int*)(scal.as<char>() + 16);
-        P.seg = dseg.as<long long>();
+        P.acc_i = (long long*)(base + 64);
+        P.ngroups = (unsigned long long*)base;
+        P.error = (int*)(base + 16);
         P.nseg = seg.empty() ? 0 : 1;
         set_one_seg(P, seg);
         P.nchunks = chunks;
         cudaStream_t s = plan_stream(*p);
-        VQ_CUDA(cudaMemsetAsync(bits.p, 0, bits.n, s));
-        VQ_CUDA(cudaMemsetAsync(scal.p, 0, 32, s));
-        if (!seg.empty()) VQ_CUDA(cudaMemcpyAsync(dseg.p, seg.data(), 24, cudaMemcpyHostToDevice, s));
+        // the bytes of the range: cleared, filled and copied back
+        const int64_t n = row_end - row_start, b0 = row_start >> 3, nb = (n + 7) / 8;
+        const int sh = (int)(row_start & 7);
+        const size_t w0 = (size_t)(row_start >> 5), w1 = std::min(words, (size_t)(row_end >> 5) + 2);
+        VQ_CUDA(cudaMemsetAsync(base, 0, 64, s));
+        VQ_CUDA(cudaMemsetAsync(base + 64 + w0 * 4, 0, (w1 - w0) * 4, s));
         if (chunks > 0) {
             int per_sm = std::max(1, p->k_main.max_blocks_per_sm);
             long long want = p->staged ? chunks : (chunks + 7) / 8;
             int grid = (int)std::max<long long>(1, std::min<long long>((long long)sm_count() * per_sm, want));
             jit_launch(p->k_main, grid, &P, sizeof P, s);
         }
-        std::vector<uint32_t> h(words);
-        unsigned long long sc[4] = {0, 0, 0, 0};
-        VQ_CUDA(cudaMemcpyAsync(h.data(), bits.p, words * 4, cudaMemcpyDeviceToHost, s));
-        VQ_CUDA(cudaMemcpyAsync(sc, scal.p, 32, cudaMemcpyDeviceToHost, s));
+        p->h_stage.ensure(32 + (size_t)nb + 1);
+        VQ_CUDA(cudaMemcpyAsync(p->h_stage.p, base, 32, cudaMemcpyDeviceToHost, s));
+        if (nb > 0) VQ_CUDA(cudaMemcpyAsync((char*)p->h_stage.p + 32, base + 64 + b0, (size_t)nb + 1, cudaMemcpyDeviceToHost, s));
         VQ_CUDA(cudaStreamSynchronize(s));
-        unsigned long long cnt = sc[0];
-        if ((int)(sc[2] & 0xFFFFFFFF) & 8) fail(VEXQ_ETIMEDOUT, "a staged tile copy did not complete within the kernel's wait limit");
+        unsigned long long cnt = *(const unsigned long long*)p->h_stage.p;
+        const int herr = *(const int*)((const char*)p->h_stage.p + 16);
+        if (herr & 8) fail(VEXQ_ETIMEDOUT, "a staged tile copy did not complete within the kernel's wait limit");
         // the device words are LSB-first, so byte k of the (little-endian)
-        // word array holds rows 8k..8k+7: shift bytes by row_start's bit offset
-        int64_t n = row_end - row_start;
-        const uint8_t* hb = (const uint8_t*)h.data();
-        const int64_t b0 = row_start >> 3, nb = (n + 7) / 8;
-        const int sh = (int)(row_start & 7);
-        for (int64_t i = 0; i < nb; i++) {
-            unsigned v = (unsigned)hb[b0 + i] >> sh;
-            if (sh) v |= (unsigned)hb[b0 + i + 1] << (8 - sh);  // the word array has 8 words of padding
-            out_bits[i] = (uint8_t)v;
+        // word array holds rows 8k..8k+7: bytes, or shifted by row_start's bit offset
+        const uint8_t* hb = (const uint8_t*)p->h_stage.p + 32;
+        if (sh == 0) {
+            std::memcpy(out_bits, hb, (size_t)nb);
+        } else {
+            for (int64_t i = 0; i < nb; i++) out_bits[i] = (uint8_t)(((unsigned)hb[i] >> sh) | ((unsigned)hb[i + 1] << (8 - sh)));
         }
         if (n & 7) out_bits[nb - 1] &= (uint8_t)((1u << (n & 7)) - 1u);
+        lease.done();
         *count = (int64_t)cnt;
         return VEXQ_OK;
     });

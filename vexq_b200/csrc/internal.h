@@ -81,8 +81,9 @@ struct PinnedBuf {
     PinnedBuf() = default;
     PinnedBuf(const PinnedBuf&) = delete;
     PinnedBuf& operator=(const PinnedBuf&) = delete;
-    ~PinnedBuf();
+    ~PinnedBuf() { release(); }
     void ensure(size_t bytes);
+    void release();
 };
 
 // ---- tables ----------------------------------------------------------------------------
@@ -125,8 +126,11 @@ struct Column {
 
 std::shared_ptr<const FlatDict> flat_dict(const Column& c);
 
+struct SelectPlans;  // compiled Filter and Project plans of a table (select.cu)
+
 struct Table {
     std::vector<Column> cols;
+    std::shared_ptr<SelectPlans> selects;
     int64_t nrows = 0;
     int32_t rg_rows = 65536;
     int32_t n_rg = 0;

@@ -132,6 +132,7 @@ struct OutPool {
     // A block of at least `bytes`, null where pinned memory has no device
     // address; lend tells whether the result may keep it.
     std::shared_ptr<OutBlock> acquire(size_t bytes, bool& lend);
+    void trim(size_t most);  // drops blocks of more than `most` bytes (a result that holds one keeps it)
 };
 
 struct Plan {
@@ -318,6 +319,20 @@ Plan* compile_select(Table* t, const vexq_expr* nodes, int nnodes, const int32_t
                      const int32_t* roots, int nroots);
 void set_having(Plan& p, const vexq_expr* nodes, int nnodes, const int32_t* children, int nchildren, int root, int visible);
 bool zone_eval(const Plan& p, int root, const Table& t, int rg);
+// A compiled Filter (kind 'f') or Project (kind 'p') plan of a table, taken for
+// one call: compile_filter / compile_select's plan with its stream and buffers.
+// done() puts it back among the table's few kept plans, keyed by the whole
+// expression, for the next call with the same expression; a lease that ends
+// without it (an error) drops the plan. A call must have synchronised before.
+struct SelectLease {
+    Table& t;
+    std::string key;
+    std::unique_ptr<Plan> p;
+    SelectLease(Table& t, char kind, const vexq_expr* nodes, int nnodes, const int32_t* children, int nchildren, int pred,
+                const int32_t* roots, int nroots);
+    void done();
+};
+void ensure_events(Plan& p);
 // Copies the plan's launch-time constants (literals, float-sum windows, cache size) into P.
 void set_plan_constants(const Plan& p, VQParams& P);
 // Fails when a table the plan reads was re-filled with values outside the

@@ -670,6 +670,12 @@ std::shared_ptr<OutBlock> OutPool::acquire(size_t bytes, bool& lend) {
     return b->dev ? b : nullptr;
 }
 
+void OutPool::trim(size_t most) {
+    for (size_t i = lent.size(); i-- > 0;)
+        if (lent[i]->pin.n > most) lent.erase(lent.begin() + i);
+    if (stage && stage->pin.n > most) stage.reset();
+}
+
 void ensure_events(Plan& p) {
     for (auto& e : p.ev)
         if (!e) VQ_CUDA(cudaEventCreate(&e));

@@ -20,7 +20,7 @@
 #include <algorithm>
 #include <cstring>
 
-#include "plan.h"
+#include "assemble.h"
 
 namespace vq {
 cudaStream_t plan_stream(Plan& p);
@@ -150,6 +150,36 @@ void scan64(long long* a, long long n, long long* tiles, long long* total, cudaS
     VQ_CUDA(cudaGetLastError());
 }
 
+// Projected rows from raw 8-byte images and validity bytes to the result's
+// block: each column in its final width with its validity bitmap. One warp an
+// item of 32 rows of one column; bound by the block's PCIe writes.
+struct ProjectCols {
+    int n;
+    struct {
+        const unsigned long long* v;
+        const unsigned char* ok;
+        long long vals, valid;
+        int width;
+    } c[8];
+};
+__global__ void __launch_bounds__(256) k_project_out(const __grid_constant__ ProjectCols p, long long rows, char* out) {
+    const int lane = threadIdx.x & 31;
+    const long long items = (rows + 31) / 32 * p.n, nw = ((long long)gridDim.x * blockDim.x) >> 5;
+    for (long long i = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < items; i += nw) {
+        const int j = (int)(i % p.n);
+        const long long r = i / p.n * 32 + lane;
+        const bool in = r < rows;
+        const unsigned long long v = in ? p.c[j].v[r] : 0ull;
+        const unsigned word = __ballot_sync(0xffffffffu, in && p.c[j].ok[r]);
+        if (in) {
+            if (p.c[j].width == 8) reinterpret_cast<unsigned long long*>(out + p.c[j].vals)[r] = v;
+            else if (p.c[j].width == 4) reinterpret_cast<unsigned*>(out + p.c[j].vals)[r] = (unsigned)v;
+            else reinterpret_cast<unsigned char*>(out + p.c[j].vals)[r] = (unsigned char)v;
+        }
+        if (lane == 0) reinterpret_cast<unsigned*>(out + p.c[j].valid)[r >> 5] = word;
+    }
+}
+
 int type_width(int t) { return (t == VEXQ_TYPE_INT64 || t == VEXQ_TYPE_FLOAT64) ? 8 : t == VEXQ_TYPE_BOOL ? 1 : 4; }
 
 // The table's columns in pinned host memory, copied from HBM (the columns'
@@ -162,6 +192,83 @@ std::mutex g_mirror_mu;
 std::map<const Table*, std::unique_ptr<HostMirror>> g_mirrors;
 
 }  // namespace
+
+// Plans kept per table: the most recent kKept, each holding at most kKeptBytes
+// of device and of pinned memory between calls (larger buffers are freed with
+// the call that grew them). A call used to compile its plan, create a stream
+// and allocate every buffer: about 450 us of a 6M-row selection bitmap's 655.
+struct SelectPlans {
+    std::mutex mu;
+    struct Kept {
+        std::string key;
+        std::unique_ptr<Plan> p;
+    };
+    std::vector<Kept> kept;  // oldest first
+};
+static std::mutex g_selects_mu;
+constexpr size_t kKept = 8, kKeptBytes = 32u << 20;
+
+static std::shared_ptr<SelectPlans> selects_of(Table& t) {
+    std::lock_guard<std::mutex> lk(g_selects_mu);
+    if (!t.selects) t.selects = std::make_shared<SelectPlans>();
+    return t.selects;
+}
+
+SelectLease::SelectLease(Table& tb, char kind, const vexq_expr* nodes, int nnodes, const int32_t* children, int nchildren, int pred,
+                         const int32_t* roots, int nroots)
+    : t(tb) {
+    // the expression, whole: a plan is reused only for the same one
+    auto raw = [&](const void* q, size_t n) { key.append((const char*)q, n); };
+    key.push_back(kind);
+    raw(&pred, sizeof pred);
+    raw(&nroots, sizeof nroots);
+    if (nroots > 0 && roots) raw(roots, (size_t)nroots * 4);
+    raw(&nchildren, sizeof nchildren);
+    if (nchildren > 0 && children) raw(children, (size_t)nchildren * 4);
+    for (int i = 0; i < nnodes; i++) {
+        const vexq_expr& e = nodes[i];
+        const int32_t head[6] = {e.kind, e.op, e.column, e.lit_kind, e.child0, e.nchildren};
+        raw(head, sizeof head);
+        raw(&e.lit_int, 8);
+        raw(&e.lit_float, 8);
+        const int64_t len = e.lit_str ? (int64_t)std::strlen(e.lit_str) : -1;
+        raw(&len, 8);
+        if (len > 0) raw(e.lit_str, (size_t)len);
+    }
+    {
+        const std::shared_ptr<SelectPlans> sp = selects_of(t);
+        std::lock_guard<std::mutex> lk(sp->mu);
+        for (size_t i = sp->kept.size(); i-- > 0;) {
+            // a refill that widened a column's range changes what is generated
+            if (sp->kept[i].p->range_epoch != t.range_epoch) {
+                sp->kept.erase(sp->kept.begin() + i);
+            } else if (!p && sp->kept[i].key == key) {
+                p = std::move(sp->kept[i].p);
+                sp->kept.erase(sp->kept.begin() + i);
+            }
+        }
+    }
+    if (!p) p.reset(kind == 'f' ? compile_filter(&t, nodes, nnodes, children, nchildren, pred)
+                                : compile_select(&t, nodes, nnodes, children, nchildren, pred, roots, nroots));
+}
+
+void SelectLease::done() {
+    DevBuf* bufs[] = {&p->scratch_a, &p->scratch_b, &p->scratch_c, &p->scratch_d};
+    size_t held = 0;
+    for (DevBuf* b : bufs) held += b->n;
+    if (held > kKeptBytes)
+        for (DevBuf* b : bufs) b->release();
+    if (p->h_stage.n > kKeptBytes) p->h_stage.release();
+    p->out_pool.trim(kKeptBytes / 2);
+    const std::shared_ptr<SelectPlans> sp = selects_of(t);
+    std::unique_ptr<Plan> old;
+    std::lock_guard<std::mutex> lk(sp->mu);
+    if (sp->kept.size() >= kKept) {
+        old = std::move(sp->kept.front().p);
+        sp->kept.erase(sp->kept.begin());
+    }
+    sp->kept.push_back({std::move(key), std::move(p)});
+}
 
 void drop_host_mirror(const Table* t) {
     std::lock_guard<std::mutex> lk(g_mirror_mu);
@@ -296,8 +403,10 @@ struct Events {
 void mark_rows(Plan& p, const Table& t, const ScanSegs& ss, DevBuf& words, DevBuf& seg, cudaStream_t s) {
     words.ensure(((size_t)(t.nrows + kPadRows) / 32 + 8) * 4);
     VQ_CUDA(cudaMemsetAsync(words.p, 0, words.n, s));
-    seg.ensure(std::max<size_t>(ss.seg.size(), 3) * 8);
-    h2d(seg.p, ss.seg.data(), ss.seg.size() * 8, s);
+    if (ss.seg.size() != 3) {  // one range travels in the parameter block
+        seg.ensure(std::max<size_t>(ss.seg.size(), 3) * 8);
+        h2d(seg.p, ss.seg.data(), ss.seg.size() * 8, s);
+    }
     if (ss.nchunks <= 0) return;
     VQParams P = select_params(p, t, seg, ss);
     P.acc_i = words.as<long long>();
@@ -457,8 +566,8 @@ int32_t vexq_project_run(vexq_table_t table, const vexq_expr* nodes, int32_t nno
         Table& t = *table->t;
         int rgs = rg_start, rge = rg_end;
         check_range_args(t, rgs, rge);
-        std::unique_ptr<Plan> pp(compile_select(&t, nodes, nnodes, children, nchildren, predicate, roots, nexprs));
-        Plan& p = *pp;
+        SelectLease lease(t, 'p', nodes, nnodes, children, nchildren, predicate, roots, nexprs);
+        Plan& p = *lease.p;
         cudaStream_t s = plan_stream(p);
         const ScanSegs ss = kept_segments(p, t, rgs, rge);
         std::unique_ptr<vexq_result_s> r(new vexq_result_s);
@@ -471,60 +580,120 @@ int32_t vexq_project_run(vexq_table_t table, const vexq_expr* nodes, int32_t nno
             if (n.type == VEXQ_TYPE_STRING) oc.dict = &t.cols[n.col].dict;
         }
         long long total = 0;
-        Events e;
-        VQ_CUDA(cudaEventRecord(e.a, s));
+        ensure_events(p);
+        VQ_CUDA(cudaEventRecord(p.ev[0], s));
         int launches = 0;
+        bool direct = false;  // columns written by the device into the result's block
         if (ss.nchunks > 0) {
-            DevBuf words, seg;
+            DevBuf &words = p.scratch_a, &seg = p.d_seg, &scr = p.scratch_b;
             mark_rows(p, t, ss, words, seg, s);
             const long long nck = (t.nrows + 127) / 128 + 1;
-            DevBuf d_off((size_t)(nck + 1) * 8), d_tiles((size_t)((nck + 1023) / 1024 + 1) * 8), d_total(8);
+            // chunk offsets | tile totals | grand total
+            const size_t b_off = (size_t)(nck + 1) * 8, b_tiles = (size_t)((nck + 1023) / 1024 + 1) * 8;
+            scr.ensure(b_off + b_tiles + 8);
+            long long* d_off = scr.as<long long>();
+            long long* d_tiles = (long long*)(scr.as<char>() + b_off);
+            long long* d_total = (long long*)(scr.as<char>() + b_off + b_tiles);
             const int cg = (int)std::min<long long>((nck + 255) / 256, (long long)sm_count() * 8);
-            k_chunk_count<<<cg, 256, 0, s>>>(words.as<unsigned>(), nck, d_off.as<long long>());
+            k_chunk_count<<<cg, 256, 0, s>>>(words.as<unsigned>(), nck, d_off);
             launch_check(s, "k_chunk_count");
-            scan64(d_off.as<long long>(), nck, d_tiles.as<long long>(), d_total.as<long long>(), s);
-            VQ_CUDA(cudaMemcpyAsync(&total, d_total.p, 8, cudaMemcpyDeviceToHost, s));
+            scan64(d_off, nck, d_tiles, d_total, s);
+            p.h_stage.ensure(8);
+            VQ_CUDA(cudaMemcpyAsync(p.h_stage.p, d_total, 8, cudaMemcpyDeviceToHost, s));
             VQ_CUDA(cudaStreamSynchronize(s));
+            total = *(const long long*)p.h_stage.p;
             launches = 5;
             if (total > 0) {
-                const int ng = (nexprs + 7) / 8;
-                std::vector<DevBuf> dv, dm;
-                for (int j = 0; j < std::min(nexprs, 8); j++) {
-                    dv.emplace_back((size_t)total * 8);
-                    dm.emplace_back((size_t)total);
-                }
-                for (auto& oc : r->cols) {
-                    oc.v.resize(total);
-                    oc.valid.resize(total);
-                }
+                const int ng = (nexprs + 7) / 8, nb = std::min(nexprs, 8);
+                // eight expressions' images and validity bytes at a time
+                const size_t b_v = ((size_t)total * 8 + 255) & ~(size_t)255, b_m = ((size_t)total + 255) & ~(size_t)255;
+                p.scratch_c.ensure((b_v + b_m) * nb);
+                char* dv = p.scratch_c.as<char>();
+                char* dm = dv + b_v * nb;
                 VQParams P = select_params(p, t, seg, ss);
                 P.acc_i = words.as<long long>();
-                P.first = d_off.as<long long>();
-                for (size_t j = 0; j < dv.size(); j++) {
-                    P.qpay[j] = dv[j].as<unsigned long long>();
-                    P.qpayv[j] = dm[j].as<unsigned char>();
+                P.first = d_off;
+                for (int j = 0; j < nb; j++) {
+                    P.qpay[j] = (unsigned long long*)(dv + b_v * j);
+                    P.qpayv[j] = (unsigned char*)(dm + b_m * j);
                 }
+                // the result's block: every column's values and bitmap. Up to
+                // 64 MB pinned (larger results come back column by column)
+                std::vector<std::pair<size_t, size_t>> at(nexprs);
+                size_t bytes = 0;
+                for (int j = 0; j < nexprs; j++) {
+                    at[j].first = bytes;
+                    bytes += ((size_t)total * type_width(r->cols[j].type) + 127) & ~(size_t)127;
+                    at[j].second = bytes;
+                    bytes += ((size_t)(total + 31) / 32 * 4 + 127) & ~(size_t)127;
+                }
+                bool lend = true;
+                std::shared_ptr<OutBlock> blk;
+                if (bytes <= (64u << 20)) blk = p.out_pool.acquire(bytes, lend);
+                direct = blk != nullptr;
+                if (!direct)
+                    for (auto& oc : r->cols) {
+                        oc.v.resize(total);
+                        oc.valid.resize(total);
+                    }
                 for (int g = 0; g < ng; g++) {
                     P.mode = g;
                     jit_launch(p.k_build, grid_for(p.k_build, ss.nchunks, false, 0), &P, sizeof P, s);
                     launch_check(s, "vq_pwrite");
                     launches++;
-                    for (int j = g * 8; j < std::min(nexprs, g * 8 + 8); j++) {
-                        VQ_CUDA(cudaMemcpyAsync(r->cols[j].v.data(), dv[j % 8].p, (size_t)total * 8, cudaMemcpyDeviceToHost, s));
-                        VQ_CUDA(cudaMemcpyAsync(r->cols[j].valid.data(), dm[j % 8].p, (size_t)total, cudaMemcpyDeviceToHost, s));
+                    const int j0 = g * 8, j1 = std::min(nexprs, g * 8 + 8);
+                    if (direct) {
+                        ProjectCols pc;
+                        std::memset(&pc, 0, sizeof pc);
+                        pc.n = j1 - j0;
+                        for (int j = j0; j < j1; j++)
+                            pc.c[j - j0] = {P.qpay[j - j0], P.qpayv[j - j0], (long long)at[j].first, (long long)at[j].second,
+                                            type_width(r->cols[j].type)};
+                        k_project_out<<<2 * sm_count(), 256, 0, s>>>(pc, total, blk->dev);
+                        VQ_CUDA(cudaGetLastError());
+                        launch_check(s, "k_project_out");
+                        launches++;
+                        continue;
+                    }
+                    for (int j = j0; j < j1; j++) {
+                        VQ_CUDA(cudaMemcpyAsync(r->cols[j].v.data(), P.qpay[j % 8], (size_t)total * 8, cudaMemcpyDeviceToHost, s));
+                        VQ_CUDA(cudaMemcpyAsync(r->cols[j].valid.data(), P.qpayv[j % 8], (size_t)total, cudaMemcpyDeviceToHost, s));
                     }
                     VQ_CUDA(cudaStreamSynchronize(s));
                 }
+                if (direct) {
+                    VQ_CUDA(cudaEventRecord(p.ev[2], s));
+                    VQ_CUDA(cudaStreamSynchronize(s));
+                    const char* data = (const char*)blk->pin.p;
+                    if (!lend) {  // the pool's blocks are with earlier results: a copy of its own
+                        auto own = std::make_shared<OutBlock>();
+                        own->heap.reset(new char[bytes]);
+                        std::memcpy(own->heap.get(), data, bytes);
+                        data = own->heap.get();
+                        blk = own;
+                    }
+                    r->block = blk;
+                    for (int j = 0; j < nexprs; j++) {
+                        OutColumn& oc = r->cols[j];
+                        oc.dv = data + at[j].first;
+                        oc.dm = (const uint8_t*)data + at[j].second;
+                        if (oc.type == VEXQ_TYPE_STRING) oc.flat = flat_dict(t.cols[p.ir[p.key_nodes[j]].col]);
+                        oc.dict = nullptr;
+                    }
+                }
             }
         }
-        VQ_CUDA(cudaEventRecord(e.b, s));
-        VQ_CUDA(cudaStreamSynchronize(s));
+        if (!direct) {
+            VQ_CUDA(cudaEventRecord(p.ev[2], s));
+            VQ_CUDA(cudaStreamSynchronize(s));
+        }
         r->nrows = total;
         own_dictionaries(r.get());
-        r->kernel_ms = ev_ms(e.a, e.b);
+        r->kernel_ms = ev_ms(p.ev[0], p.ev[2]);
         r->scan_ms = r->kernel_ms;
         r->launches = launches;
         r->rows_scanned = ss.rows;
+        lease.done();
         *out = r.release();
         return VEXQ_OK;
     });

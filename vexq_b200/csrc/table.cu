@@ -52,11 +52,14 @@ void DevBuf::release() {
     n = 0;
 }
 
-PinnedBuf::~PinnedBuf() { if (p) cudaFreeHost(p); }
-void PinnedBuf::ensure(size_t bytes) {
-    if (bytes <= n) return;
+void PinnedBuf::release() {
     if (p) cudaFreeHost(p);
     p = nullptr;
+    n = 0;
+}
+void PinnedBuf::ensure(size_t bytes) {
+    if (bytes <= n) return;
+    release();
     VQ_CUDA(cudaMallocHost(&p, bytes));
     n = bytes;
 }

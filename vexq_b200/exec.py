@@ -34,6 +34,11 @@ from .table import HostTable
 
 _initialised = False
 
+# PyBytes_FromStringAndSize(NULL, n): a new bytes object whose contents the
+# caller fills before anyone else sees it
+_new_bytes = C.pythonapi.PyBytes_FromStringAndSize
+_new_bytes.restype, _new_bytes.argtypes = C.py_object, [C.c_void_p, C.c_ssize_t]
+
 
 def init(device: int = 0) -> None:
     global _initialised
@@ -405,11 +410,12 @@ class GpuFilter:
 
     def bitmap(self, row_start: int = 0, row_end: int = -1):
         n = (self.table.host.nrows if row_end < 0 else row_end) - row_start
-        out = (C.c_uint8 * max((n + 7) // 8, 1))()
+        # the library fills the bytes object itself: no cleared array, no copy
+        out = _new_bytes(None, max(0, (n + 7) // 8))
         cnt = C.c_int64()
         abi.check(abi.load().vexq_filter_run(self.table.h, self.nodes, self.nn, self.ch, self.nc, self.root,
-                                             row_start, row_end, out, C.byref(cnt)))
-        return bytes(out)[:(n + 7) // 8], cnt.value
+                                             row_start, row_end, C.cast(C.c_char_p(out), C.POINTER(C.c_uint8)), C.byref(cnt)))
+        return out, cnt.value
 
     @staticmethod
     def selvec(bits: bytes, nrows: int, block: int) -> List[int]:
