@@ -126,6 +126,7 @@ struct Batch {
     std::string explain;
 
     ~Batch() {
+        if (s) (void)cudaStreamSynchronize(s);  // before its pinned blocks go back to the pool
         if (gexec) cudaGraphExecDestroy(gexec);
         if (graph) cudaGraphDestroy(graph);
         for (auto& e : ev)

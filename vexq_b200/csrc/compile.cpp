@@ -3158,6 +3158,9 @@ Plan::~Plan() {
         std::lock_guard<std::mutex> lk(g_zone_mu);
         g_zone_strings.erase(this);
     }
+    // a run that ended in an error may have left work on the stream: its pinned
+    // blocks go back to the pool only after it
+    if (stream) (void)cudaStreamSynchronize(stream);
     if (rg_exec) cudaGraphExecDestroy(rg_exec);
     for (auto& e : ev)
         if (e) cudaEventDestroy(e);

@@ -646,7 +646,7 @@ std::shared_ptr<OutBlock> OutPool::acquire(size_t bytes, bool& lend) {
     auto fit = [&](OutBlock& b) {
         if (b.pin.n >= bytes) return;
         b.dev = nullptr;
-        b.pin.ensure(bytes + bytes / 4);
+        b.pin.ensure(bytes);
         void* d = nullptr;
         if (cudaHostGetDevicePointer(&d, b.pin.p, 0) == cudaSuccess) b.dev = (char*)d;
         else (void)cudaGetLastError();

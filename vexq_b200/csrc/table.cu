@@ -52,16 +52,54 @@ void DevBuf::release() {
     n = 0;
 }
 
+// Pinned blocks given back, by power-of-two size, for the next buffer of that
+// size: pinning costs milliseconds a call, which the first run of every new plan
+// paid. At most kPinnedKept bytes are kept; a block serves one buffer at a time
+// and comes back only when no copy or kernel uses it any more (its owner has
+// synchronised). Never freed at exit: the driver may be gone by then.
+namespace {
+constexpr size_t kPinnedKept = 128u << 20, kPinnedMin = 4096;
+std::mutex g_pinned_mu;
+std::map<size_t, std::vector<void*>>& pinned_free() {
+    static auto* m = new std::map<size_t, std::vector<void*>>;
+    return *m;
+}
+size_t g_pinned_bytes = 0;
+}  // namespace
+
 void PinnedBuf::release() {
-    if (p) cudaFreeHost(p);
+    if (p) {
+        std::unique_lock<std::mutex> lk(g_pinned_mu);
+        if (n <= kPinnedKept / 4 && g_pinned_bytes + n <= kPinnedKept) {
+            pinned_free()[n].push_back(p);
+            g_pinned_bytes += n;
+        } else {
+            lk.unlock();
+            cudaFreeHost(p);
+        }
+    }
     p = nullptr;
     n = 0;
 }
 void PinnedBuf::ensure(size_t bytes) {
     if (bytes <= n) return;
     release();
-    VQ_CUDA(cudaMallocHost(&p, bytes));
-    n = bytes;
+    size_t want = kPinnedMin;
+    while (want < bytes && want < kPinnedKept / 4) want <<= 1;
+    want = std::max(want, bytes);  // above the kept sizes: as asked
+    {
+        std::lock_guard<std::mutex> lk(g_pinned_mu);
+        auto it = pinned_free().find(want);
+        if (it != pinned_free().end() && !it->second.empty()) {
+            p = it->second.back();
+            it->second.pop_back();
+            g_pinned_bytes -= want;
+            n = want;
+            return;
+        }
+    }
+    VQ_CUDA(cudaMallocHost(&p, want));
+    n = want;
 }
 
 uint32_t GlobalDict::add(const std::string& s) {
