@@ -72,7 +72,7 @@ __global__ void k_init_table(unsigned long long* keys, long long* first, long lo
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         *ngroups = 0ull;
         *error = 0;
-        *n_out = 0ull;
+        n_out[0] = n_out[1] = n_out[2] = 0ull;  // groups, and the top-k's counters
     }
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < nslots; i += (long long)gridDim.x * blockDim.x) {
         if (hash) keys[i] = (i == nslots - 1) ? 0ull : VQ_EMPTY_KEY;
@@ -396,42 +396,90 @@ __device__ __forceinline__ unsigned long long vq_rank(long long bits, bool isnul
     u = desc ? u : ~u;
     return u == 0xFFFFFFFFFFFFFFFFull ? u - 1 : u;
 }
-// The top-k kernels read the group count from the device (*np, written by
-// the finalize or HAVING compaction), so they follow it without a copy back.
-// One block samples S evenly spaced group ranks (S <= 16384) and finds the
-// q-th largest of them (q < S) by radix select, most significant byte first: each round counts, in shared memory,
-// the next byte of the samples that match the bytes chosen so far, and one
-// warp walks the 256 counts from the top to the byte holding the q-th largest.
-// The result is the selection threshold, so the host needs no copy of the
-// samples.
-__global__ void __launch_bounds__(1024) k_threshold(const unsigned long long* rank, int S, const unsigned long long* np, long long nmax,
-                                                    int limit, unsigned long long* thr) {
-    const long long n = (long long)min(*np, (unsigned long long)nmax);
-    // few groups (at most 4·LIMIT + 4096): every group is a candidate
-    if (n <= 4LL * limit + 4096) {
-        if (threadIdx.x == 0) *thr = 0ull;
-        return;
+// The groups a top-k selects from: a group table as the scan left it (np null:
+// every slot with a row count), or compacted groups (*np of them).
+struct VQTop {
+    const unsigned long long* keys;
+    const long long* first;
+    const long long* ival;
+    const long long* fx;
+    const unsigned* special;
+    const double* fval;            // compacted: the float sums
+    const int* fx_lsb;
+    const unsigned long long* np;
+    long long n, stride;           // slots (or the most groups); distance between banks
+    int ni, nf, hash;              // hash: keys[] holds the keys (else the slot is the key)
+    int kind, vbank, vpos, nnpos, fmin_key, desc, limit;
+    unsigned long long* rank;      // [n] sort rank, 0 where there is no group
+    unsigned long long* wmax;      // [(n + 31) / 32] largest rank of every 32
+    unsigned long long* cnt;       // groups, selected groups, blocks done: 0 before k_rank
+    const int* error;
+    long long R, cap;              // rows that fit the host block, and at all
+    long long* host;               // header (groups, error word, selected), rows [0, R)
+    long long* rest;               // rows [R, cap)
+};
+
+__device__ __forceinline__ double top_float(const VQTop& t, int f, long long i) {
+    const long long at = (long long)f * t.stride + i;
+    return t.np ? t.fval[at] : vq_fx_result(t.fx + at * 4, t.fx_lsb[f], t.special[at]);
+}
+
+// Rank of the ORDER BY output of every group: its raw bits (NULL flag) mapped by
+// vq_rank so that a larger rank sorts first, and the largest rank of each 32
+// slots. The table is read where it lies (one pass over the occupied counts,
+// the sort column's bank and 8 bytes written a slot), not compacted first: 720K
+// slots 9 us, against 17 + 5 for the compaction and the ranks of its output.
+__global__ void __launch_bounds__(256) k_rank(const __grid_constant__ VQTop t) {
+    __shared__ unsigned warp_groups[8];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const long long n = t.np ? (long long)min(*t.np, (unsigned long long)t.n) : t.n;
+    const long long stride = (long long)gridDim.x * blockDim.x;
+    unsigned groups = 0u;
+    for (long long b = (long long)blockIdx.x * blockDim.x + warp * 32; b < t.n; b += stride) {
+        const long long i = b + lane;
+        const bool occ = i < n && (t.np || t.ival[i] != 0);
+        unsigned long long rank = 0ull;
+        if (occ) {
+            const long long nn = t.ival[(long long)t.nnpos * t.stride + i];
+            const bool isnull = t.kind != VEXQ_AGG_COUNT && nn == 0;
+            long long bits;
+            if (t.vbank == 1) {  // float sum bank
+                double v = top_float(t, t.vpos, i);
+                if (t.kind == VEXQ_AGG_AVG) v = v / (double)nn;
+                bits = __double_as_longlong(v);
+            } else {
+                bits = t.ival[(long long)t.vpos * t.stride + i];
+                if (t.fmin_key) bits = __double_as_longlong(vq_fkey_inv((unsigned long long)bits));
+            }
+            rank = vq_rank(bits, isnull, t.desc);
+        }
+        if (i < t.n) t.rank[i] = rank;
+        groups += __popc(__ballot_sync(0xffffffffu, occ));
+        unsigned long long m = rank;
+        for (int o = 16; o > 0; o >>= 1) {
+            const unsigned long long x = __shfl_xor_sync(0xffffffffu, m, o);
+            m = x > m ? x : m;
+        }
+        if (lane == 0) t.wmax[b >> 5] = m;
     }
-    // expected (q+1)·n/S groups at or above the q-th largest sample: about
-    // 4·LIMIT + 64 (n above 4·LIMIT + 4096 keeps q below S), and q at least 3:
-    // the count above the q-th largest sample spreads like a Gamma(q+1)
-    // variable, so with q = 0 about one run in 20 kept fewer than LIMIT groups
-    // and fetched every group instead; from q = 3 (about 4·n/S candidates)
-    // that is about one run in 10,000 at LIMIT 10
-    const int q = max((int)ceil((4.0 * limit + 64.0) * S / (double)n) - 1, min(3, S - 1));
+    if (lane == 0) warp_groups[warp] = groups;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        unsigned sum = 0u;
+        for (int w = 0; w < 8; w++) sum += warp_groups[w];
+        if (sum) atomicAdd(t.cnt, (unsigned long long)sum);
+    }
+}
+
+// q-th largest (from 0) of the block's 16 values a thread by radix select, most
+// significant byte first: each round counts, in shared memory, the next byte of
+// the values that match the bytes chosen so far, and one warp walks the 256
+// counts from the top to the byte holding the q-th largest.
+__device__ __forceinline__ unsigned long long block_kth16(const unsigned long long (&v)[16], unsigned q) {
     __shared__ unsigned hist[256];
     __shared__ unsigned long long prefix;
     __shared__ unsigned need;
-    // 16 samples a thread in registers (blockDim × 16 ≥ S), valid bits in a mask
-    unsigned long long v[16];
-    unsigned valid = 0u;
-#pragma unroll
-    for (int k = 0; k < 16; k++) {
-        const int i = (int)threadIdx.x + k * (int)blockDim.x;
-        v[k] = i < S ? rank[(long long)i * n / S] : 0ull;  // the sample: S evenly spaced groups
-        if (i < S) valid |= 1u << k;
-    }
-    if (threadIdx.x == 0) { prefix = 0ull; need = (unsigned)q; }
+    if (threadIdx.x == 0) { prefix = 0ull; need = q; }
     for (int shift = 56; shift >= 0; shift -= 8) {
         for (int i = threadIdx.x; i < 256; i += blockDim.x) hist[i] = 0u;
         __syncthreads();
@@ -440,7 +488,7 @@ __global__ void __launch_bounds__(1024) k_threshold(const unsigned long long* ra
         const unsigned nd = need;  // both rewritten only after the next barrier
 #pragma unroll
         for (int k = 0; k < 16; k++)
-            if (((valid >> k) & 1u) && (v[k] & hi_mask) == pre) atomicAdd(&hist[(v[k] >> shift) & 255u], 1u);
+            if ((v[k] & hi_mask) == pre) atomicAdd(&hist[(v[k] >> shift) & 255u], 1u);
         __syncthreads();
         if (threadIdx.x < 32) {
             const int lane = threadIdx.x;
@@ -467,50 +515,90 @@ __global__ void __launch_bounds__(1024) k_threshold(const unsigned long long* ra
         }
         __syncthreads();
     }
-    if (threadIdx.x == 0) *thr = q < S ? prefix : 0ull;
-}
-// The groups at or above the threshold, each gathered straight into its
-// claimed row of the staging block (key, first-row key, integer bank, float
-// bank as raw bits).
-__global__ void k_select(const unsigned long long* rank, const unsigned long long* np, long long nmax, const unsigned long long* thrp,
-                         unsigned long long* nsel, long long cap, const unsigned long long* key, const long long* first,
-                         const long long* ival, const double* fval, long long cap_out, int ni, int nf, long long* out) {
-    const long long n = (long long)min(*np, (unsigned long long)nmax);
-    const unsigned long long thr = *thrp;
-    const long long w = 2 + ni + nf;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        if (rank[i] >= thr) {
-            const unsigned long long p = atomicAdd(nsel, 1ull);
-            if ((long long)p >= cap) continue;
-            long long* o = out + (long long)p * w;
-            o[0] = (long long)key[i];
-            o[1] = first[i];
-            for (int s = 0; s < ni; s++) o[2 + s] = ival[(long long)s * cap_out + i];
-            for (int f = 0; f < nf; f++) o[2 + ni + f] = __double_as_longlong(fval[(long long)f * cap_out + i]);
-        }
-    }
-}
-// Rank of one aggregate output per compacted group: its sort key's raw bits
-// (NULL flag) mapped by vq_rank so that a larger rank sorts first.
-__global__ void k_sortrank(const long long* o_i, const double* o_f, long long cap_out, const unsigned long long* np, int kind,
-                           int vbank, int vpos, int nnpos, int fmin_key, int desc, unsigned long long* rank) {
-    const long long n = (long long)min(*np, (unsigned long long)cap_out);
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        long long nn = o_i[(long long)nnpos * cap_out + i];
-        bool isnull = kind != VEXQ_AGG_COUNT && nn == 0;
-        long long bits;
-        if (vbank == 1) {  // float sum bank
-            double v = o_f[(long long)vpos * cap_out + i];
-            if (kind == VEXQ_AGG_AVG) v = v / (double)nn;
-            bits = __double_as_longlong(v);
-        } else {
-            bits = o_i[(long long)vpos * cap_out + i];
-            if (fmin_key) bits = __double_as_longlong(vq_fkey_inv((unsigned long long)bits));
-        }
-        rank[i] = vq_rank(bits, isnull, desc);
-    }
+    return prefix;
 }
 
+// The block's 1,024 values, one a thread, sorted descending (bitonic; strides
+// below 32 in registers).
+__device__ __forceinline__ unsigned long long block_sort1024(unsigned long long v) {
+    __shared__ unsigned long long sh[1024];
+    const int t = threadIdx.x;
+    for (int k = 2; k <= 1024; k <<= 1)
+        for (int j = k >> 1; j > 0; j >>= 1) {
+            unsigned long long o;
+            if (j >= 32) {
+                __syncthreads();
+                sh[t] = v;
+                __syncthreads();
+                o = sh[t ^ j];
+            } else {
+                o = __shfl_xor_sync(0xffffffffu, v, j);
+            }
+            const bool keep_max = ((t & j) == 0) == ((t & k) == 0);
+            v = keep_max ? (v > o ? v : o) : (v < o ? v : o);
+        }
+    return v;
+}
+
+// The groups ORDER BY … LIMIT can need. The slots are parted into at least
+// 1,024 parts; the LIMIT-th largest of the parts' largest ranks is a threshold
+// that at least LIMIT groups reach, and few others (LIMIT 100 of 200K groups in
+// 1,024 parts: about 105). Every block finds it for itself from the 32-slot
+// maxima (180 KB for 720K slots), then takes its share of the ranks; the groups
+// at or above it (ties included; every group when fewer parts than LIMIT hold
+// one) are written as rows (key, first-row key, integer bank, float bank as raw
+// bits) straight into pinned host memory. One launch of one block an SM, 5 us,
+// against 25 + 5 us for a one-block select over 16,384 samples and the gather,
+// with four copies back.
+__global__ void __launch_bounds__(1024) k_select(const __grid_constant__ VQTop t) {
+    __shared__ unsigned long long threshold;
+    const long long m = (t.n + 31) / 32;
+    const unsigned q = (unsigned)max(t.limit, 1) - 1u;
+    if (q < 256u) {
+        unsigned long long v = 0ull;
+        for (long long i = threadIdx.x; i < m; i += 1024) {
+            const unsigned long long x = t.wmax[i];
+            v = x > v ? x : v;
+        }
+        v = block_sort1024(v);
+        if (threadIdx.x == q) threshold = v;
+        __syncthreads();
+    } else {
+        unsigned long long v[16];
+#pragma unroll
+        for (int k = 0; k < 16; k++) {
+            v[k] = 0ull;
+            for (long long i = threadIdx.x + k * 1024; i < m; i += 16384) {
+                const unsigned long long x = t.wmax[i];
+                v[k] = x > v[k] ? x : v[k];
+            }
+        }
+        const unsigned long long kth = block_kth16(v, q);
+        if (threadIdx.x == 0) threshold = kth;
+        __syncthreads();
+    }
+    const unsigned long long thr = threshold;
+    const long long w = 2 + t.ni + t.nf;
+    const long long n = t.np ? (long long)min(*t.np, (unsigned long long)t.n) : t.n;
+    for (long long i = (long long)blockIdx.x * 1024 + threadIdx.x; i < n; i += (long long)gridDim.x * 1024) {
+        if (t.rank[i] < thr || (thr == 0ull && !t.np && t.ival[i] == 0)) continue;
+        const long long p = (long long)atomicAdd(t.cnt + 1, 1ull);
+        if (p >= t.cap) continue;
+        long long* o = p < t.R ? t.host + 4 + p * w : t.rest + (p - t.R) * w;
+        o[0] = (long long)(!t.hash ? (unsigned long long)i : !t.np && i == t.n - 1 ? VQ_EMPTY_KEY : t.keys[i]);
+        o[1] = t.first[i];
+        for (int s = 0; s < t.ni; s++) o[2 + s] = t.ival[(long long)s * t.stride + i];
+        for (int f = 0; f < t.nf; f++) o[2 + t.ni + f] = __double_as_longlong(top_float(t, f, i));
+    }
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0 && atomicAdd(t.cnt + 2, 1ull) == gridDim.x - 1) {  // the last block
+        __threadfence();
+        t.host[0] = (long long)(t.np ? (unsigned long long)n : t.cnt[0]);
+        t.host[1] = t.error ? *t.error : 0;
+        t.host[2] = (long long)*(volatile unsigned long long*)(t.cnt + 1);
+    }
+}
 
 }  // namespace vq
 
@@ -928,9 +1016,13 @@ struct Compacted {
     long long* first = nullptr;
     long long* ival = nullptr;
     double* fval = nullptr;
-    const unsigned long long* n_dev = nullptr;  // the group count on the device
-    const int* err_dev = nullptr;  // deferred run: the kernels' error word, read with the results
-    bool hash = false;             // deferred run on a hash table: its group count sizes the next run
+    unsigned long long* n_dev = nullptr;  // the group count on the device (and two counters of the top-k)
+    // deferred run: the table as the scan left it, not compacted yet
+    const unsigned long long* t_keys = nullptr;
+    const VQParams* P = nullptr;
+    const int* d_lsb = nullptr;
+    bool keyed = false;            // t_keys holds the groups' keys
+    bool hash = false;             // a hash table: its group count sizes the next run
     long long rows = 0;
     bool having_done = false;  // only the groups HAVING keeps
     vexq_result_s* done = nullptr;  // the finished result, where the device assembled it
@@ -1007,9 +1099,29 @@ static vexq_result_s* run_assemble(RunCtx& rc, const VQParams& P, long long nslo
     }
 }
 
-// A deferred run (defer set) launches the table kernels and returns without
-// waiting: the caller's top-k launches follow on the stream, and one copy back
-// after them brings the group count and the error word with the results.
+// Compacts a table the scan has filled into scratch_b (at most every slot is a group).
+static void compact_table(RunCtx& rc, Compacted& c) {
+    Plan& p = rc.p;
+    const VQParams& P = *c.P;
+    const long long nslots = c.cap_out, cap_out = nslots;
+    const int ni = p.ni, nf = p.nf;
+    p.scratch_b.ensure(16 + cap_out * 16 + (size_t)ni * cap_out * 8 + (size_t)nf * cap_out * 8 + nf * 4 + 64);
+    char* ob = (char*)p.scratch_b.p;
+    c.key = (unsigned long long*)(ob + 16);
+    c.first = (long long*)(ob + 16 + cap_out * 8);
+    c.ival = (long long*)(ob + 16 + cap_out * 16);
+    c.fval = (double*)(ob + 16 + cap_out * 16 + (size_t)ni * cap_out * 8);
+    const int fg = (int)std::min<long long>((nslots + 255) / 256, (long long)sm_count() * 16);
+    k_finalize<<<fg, 256, 0, rc.s>>>(c.t_keys, P.first, P.acc_i, P.acc_fx, P.special, nslots, ni, nf, c.d_lsb, c.keyed, c.n_dev, c.key,
+                                     c.first, c.ival, c.fval, cap_out);
+    launch_check(rc.s, "k_finalize");
+    VQ_CUDA(cudaGetLastError());
+    VQ_CUDA(cudaEventRecord(p.ev[3], rc.s));
+}
+
+// A deferred run (defer set) launches the scan and returns without waiting or
+// compacting: the caller's top-k launches read the table where it lies, and
+// their output brings the group count and the error word.
 // assemble: the caller wants the finished result (c.done) where the device can
 // write it; where it cannot, the groups come compacted as without it.
 Compacted run_atomic(RunCtx& rc, VQParams& P, long long nchunks, long long estimate, long long rows, bool defer = false,
@@ -1107,31 +1219,20 @@ Compacted run_atomic(RunCtx& rc, VQParams& P, long long nchunks, long long estim
                 }
             }
         }
-        // compacted output (upper bound: every slot occupied)
-        long long cap_out = nslots;
-        size_t o_bytes = 16 + cap_out * 16 + (size_t)ni * cap_out * 8 + (size_t)nf * cap_out * 8 + nf * 4 + 64;
-        p.scratch_b.ensure(o_bytes);
-        char* ob = (char*)p.scratch_b.p;
-        c.cap_out = cap_out;
-        c.key = (unsigned long long*)(ob + 16);
-        c.first = (long long*)(ob + 16 + cap_out * 8);
-        c.ival = (long long*)(ob + 16 + cap_out * 16);
-        c.fval = (double*)(ob + 16 + cap_out * 16 + (size_t)ni * cap_out * 8);
-        int fg = (int)std::min<long long>((nslots + 255) / 256, (long long)sm_count() * 16);
-        k_finalize<<<fg, 256, 0, rc.s>>>(gid ? p.jt_gkey.as<unsigned long long>() : P.keys, P.first, P.acc_i, P.acc_fx, P.special,
-                                         nslots, ni, nf, d_lsb, hash || gid, n_out, c.key, c.first, c.ival, c.fval, cap_out);
-        launch_check(rc.s, "k_finalize");
-        VQ_CUDA(cudaGetLastError());
-        VQ_CUDA(cudaEventRecord(p.ev[3], rc.s));
         c.n_dev = n_out;
+        c.cap_out = nslots;
+        c.t_keys = gid ? p.jt_gkey.as<unsigned long long>() : P.keys;
+        c.P = &P;
+        c.d_lsb = d_lsb;
+        c.keyed = hash || gid;
+        c.hash = hash;
+        c.rows = rows;
         if (defer) {
             c.n = -1;
-            c.err_dev = P.error;
-            c.hash = hash;
-            c.rows = rows;
-            rc.launches += 3;
+            rc.launches += 2;
             return c;
         }
+        compact_table(rc, c);
         p.h_stage.ensure(32);
         VQ_CUDA(cudaMemcpyAsync(p.h_stage.p, n_out, 8, cudaMemcpyDeviceToHost, rc.s));
         VQ_CUDA(cudaMemcpyAsync((char*)p.h_stage.p + 8, P.error, 4, cudaMemcpyDeviceToHost, rc.s));
@@ -1145,7 +1246,7 @@ Compacted run_atomic(RunCtx& rc, VQParams& P, long long nchunks, long long estim
             cap = std::max(cap << 1, safe_cap);
             continue;
         }
-        c.n = (long long)std::min<unsigned long long>(nn, (unsigned long long)cap_out);
+        c.n = (long long)std::min<unsigned long long>(nn, (unsigned long long)nslots);
         if (hash) {
             p.hash_groups_seen = c.n;
             p.hash_rows_seen = rows;
@@ -1218,17 +1319,13 @@ Compacted having_device(RunCtx& rc, const Compacted& c) {
     return o;
 }
 
-// Device top-k candidates for ORDER BY <aggregate> LIMIT k: every group's sort
-// rank (raw int64 bits in the ExternalSort order, NULLs first) is computed on
-// the device; the q-th largest of a 4096-point sample, found on the device,
-// is a threshold that keeps about 4·LIMIT + 64 groups (every group when there
-// are at most 4·LIMIT + 4096); the groups at or above it (ties included) are
-// gathered, and the host finishes the stable sort on them. The kernels read
-// the group count on the device, so they follow a deferred table run without
-// a copy back; one copy brings the count, the error word, the selected count
-// and the first gathered rows. Returns 1 with g filled; 0 when the caller
-// fetches every group instead (the plan has no such ORDER BY, the groups are
-// few and already counted, or the sample was unlucky; c.n is set); -1 when a
+// Device top-k candidates for ORDER BY <aggregate> LIMIT k (k_rank, k_select):
+// the groups that can be among the first LIMIT come back, ties included, and
+// the host finishes the stable sort on them. They read the group table (a
+// deferred run) or the compacted groups (after HAVING). Returns 1 with g
+// filled; 0 when the caller fetches every group instead (the plan has no such
+// ORDER BY, the groups are few and already counted, or more than 65,536 groups
+// reach the threshold; c.n is set and the groups are compacted); -1 when a
 // deferred run hit its table's probe limit and must run again.
 bool topk_applies(const Plan& p, bool having_done) {
     const vexq_order_desc& o = p.order;
@@ -1248,78 +1345,97 @@ int topk_groups(RunCtx& rc, Compacted& c, Groups& g) {
     int vbank = (p.slots[vslot].kind == S_FSUM) ? 1 : 0;
     int fmin_key = (p.slots[vslot].kind == S_FMIN || p.slots[vslot].kind == S_FMAX) ? 1 : 0;
     if (a.kind == VEXQ_AGG_COUNT) vbank = 0;
-    // 16,384 samples: with q at least 3 about 4·n/S ≈ 175 candidates for
-    // Q3's ~700K groups (4,096 samples with q at least 7 kept ~1,400, whose
-    // host sort cost more)
-    const int S = 16384;
-    const long long w = 2 + p.ni + p.nf;
-    const long long nmax = c.n >= 0 ? c.n : c.cap_out;
-    // rank | threshold, count | gathered rows
-    size_t need = (size_t)nmax * 8 + 16 + (size_t)kCap * w * 8 + 64;
-    p.scratch_d.ensure(need);
-    unsigned long long* rank = p.scratch_d.as<unsigned long long>();
-    unsigned long long* thr = rank + nmax;
-    unsigned long long* nsel = thr + 1;
-    long long* dout = (long long*)(nsel + 1);
-    int gr = (int)std::min<long long>((nmax + 255) / 256, (long long)sm_count() * 8);
-    k_sortrank<<<std::max(gr, 1), 256, 0, rc.s>>>(c.ival, c.fval, c.cap_out, c.n_dev, a.kind, vbank, p.slot_pos[vslot],
-                                                  p.slot_pos[a.nn_slot], fmin_key, o.descending, rank);
-    launch_check(rc.s, "k_sortrank");
-    k_threshold<<<1, 1024, 0, rc.s>>>(rank, S, c.n_dev, nmax, (int)o.limit, thr);
-    launch_check(rc.s, "k_threshold");
-    VQ_CUDA(cudaMemsetAsync(nsel, 0, 8, rc.s));
-    k_select<<<std::max(gr, 1), 256, 0, rc.s>>>(rank, c.n_dev, nmax, thr, nsel, kCap, c.key, c.first, c.ival, c.fval, c.cap_out,
-                                                p.ni, p.nf, dout);
+    const bool table = c.n < 0;  // a deferred run
+    const long long w = 2 + p.ni + p.nf, nmax = table ? c.cap_out : c.n;
+    const size_t b_rank = (size_t)nmax * 8, b_max = (size_t)(nmax + 31) / 32 * 8;
+    // rank | maxima | counters (compacted groups) | rows past the host block's
+    // R: the last run's candidates and as many again, at least 1,024
+    long long R = 1024;
+    while (R < 2 * p.topk_seen && R < kCap) R <<= 1;
+    p.scratch_d.ensure(b_rank + b_max + 32 + (size_t)(kCap - R) * w * 8);
+    p.h_stage.ensure(32 + (size_t)R * w * 8);
+    void* mapped = nullptr;
+    if (cudaHostGetDevicePointer(&mapped, p.h_stage.p, 0) != cudaSuccess) fail(VEXQ_EDEVICE, "pinned host memory has no device address");
+    VQTop t;
+    std::memset(&t, 0, sizeof t);
+    t.rank = p.scratch_d.as<unsigned long long>();
+    t.wmax = t.rank + nmax;
+    t.cnt = table ? c.n_dev : t.wmax + (nmax + 31) / 32;
+    t.rest = (long long*)(p.scratch_d.as<char>() + b_rank + b_max + 32);
+    t.host = (long long*)mapped;
+    t.R = R;
+    t.cap = kCap;
+    t.n = nmax;
+    t.stride = c.cap_out;
+    t.ni = p.ni;
+    t.nf = p.nf;
+    t.kind = a.kind;
+    t.vbank = vbank;
+    t.vpos = p.slot_pos[vslot];
+    t.nnpos = p.slot_pos[a.nn_slot];
+    t.fmin_key = fmin_key;
+    t.desc = o.descending;
+    t.limit = (int)o.limit;
+    if (table) {
+        t.keys = c.t_keys;
+        t.first = c.P->first;
+        t.ival = c.P->acc_i;
+        t.fx = c.P->acc_fx;
+        t.special = c.P->special;
+        t.fx_lsb = c.d_lsb;
+        t.hash = c.keyed;
+        t.error = c.P->error;
+    } else {
+        t.keys = c.key;
+        t.first = c.first;
+        t.ival = c.ival;
+        t.fval = c.fval;
+        t.hash = 1;
+        t.np = c.n_dev;
+        VQ_CUDA(cudaMemsetAsync(t.cnt, 0, 24, rc.s));
+    }
+    const int gr = (int)std::max<long long>(1, std::min<long long>((nmax + 255) / 256, (long long)sm_count() * 8));
+    k_rank<<<gr, 256, 0, rc.s>>>(t);
+    launch_check(rc.s, "k_rank");
+    k_select<<<(int)std::max<long long>(1, std::min<long long>((nmax + 1023) / 1024, sm_count())), 1024, 0, rc.s>>>(t);
     launch_check(rc.s, "k_select");
     VQ_CUDA(cudaGetLastError());
-    rc.launches += 3;
-    // one copy back: group count, error word, selected count, and the first
-    // R gathered rows (twice the last run's candidates and 256 more, at least
-    // twice the expected 4·LIMIT + 64), rounded up to a power of two so the
-    // pinned staging buffer grows only at doublings
-    const long long want = std::max<long long>(2 * (4LL * o.limit + 64), p.topk_seen * 2 + 256);
-    long long R = 1024;
-    while (R < want) R <<= 1;
-    R = std::min(R, kCap);
-    p.h_stage.ensure(32 + (size_t)R * w * 8);
-    char* hs = (char*)p.h_stage.p;
-    std::memset(hs, 0, 32);
-    VQ_CUDA(cudaMemcpyAsync(hs, c.n_dev, 8, cudaMemcpyDeviceToHost, rc.s));
-    if (c.err_dev) VQ_CUDA(cudaMemcpyAsync(hs + 8, c.err_dev, 4, cudaMemcpyDeviceToHost, rc.s));
-    VQ_CUDA(cudaMemcpyAsync(hs + 16, nsel, 8, cudaMemcpyDeviceToHost, rc.s));
-    VQ_CUDA(cudaMemcpyAsync(hs + 32, dout, (size_t)R * w * 8, cudaMemcpyDeviceToHost, rc.s));
-    if (c.n < 0) VQ_CUDA(cudaEventRecord(p.ev[3], rc.s));
+    rc.launches += 2;
+    if (table) VQ_CUDA(cudaEventRecord(p.ev[3], rc.s));
     VQ_CUDA(cudaStreamSynchronize(rc.s));
-    if (c.n < 0) {  // a deferred table run: its time, count and error word
+    const long long* hs = (const long long*)p.h_stage.p;
+    if (table) {  // its time, count and error word
         rc.scan_ms += elapsed(p.ev[1], p.ev[2]);
         rc.kernel_ms += elapsed(p.ev[0], p.ev[3]);
-        c.n = (long long)std::min<unsigned long long>(*(const unsigned long long*)hs, (unsigned long long)c.cap_out);
-        const int herr = *(const int*)(hs + 8);
-        if (check_table_flags(herr, c.hash)) return -1;
+        c.n = std::min<long long>(hs[0], c.cap_out);
+        if (check_table_flags((int)hs[1], c.hash)) return -1;
         if (c.hash) {
             p.hash_groups_seen = c.n;
             p.hash_rows_seen = c.rows;
         }
     }
-    const long long ns = (long long)*(const unsigned long long*)(hs + 16);
+    const long long ns = hs[2];
     p.topk_seen = std::min(ns, kCap);
-    // few groups: all of them were selected; otherwise an unlucky sample (fewer
-    // than LIMIT selected) or too many ties at the threshold: the caller
-    // fetches every group
-    if (c.n > 4 * o.limit + 4096 && (ns < o.limit || ns > kCap)) return 0;
-    if (ns > kCap) return 0;
+    // too many ties at the threshold: the caller fetches every group
+    if (ns > kCap) {
+        if (table) {
+            VQ_CUDA(cudaMemsetAsync(c.n_dev, 0, 8, rc.s));
+            compact_table(rc, c);
+        }
+        return 0;
+    }
     g.having_done = c.having_done;
     std::vector<long long> rest;
     if (ns > R) {
         rest.resize((size_t)(ns - R) * w);
-        VQ_CUDA(cudaMemcpyAsync(rest.data(), dout + R * w, rest.size() * 8, cudaMemcpyDeviceToHost, rc.s));
+        VQ_CUDA(cudaMemcpyAsync(rest.data(), t.rest, rest.size() * 8, cudaMemcpyDeviceToHost, rc.s));
         VQ_CUDA(cudaStreamSynchronize(rc.s));
     }
     g.key.resize(ns);
     g.first.resize(ns);
     g.ival.assign(p.ni, std::vector<int64_t>(ns));
     g.fval.assign(p.nf, std::vector<double>(ns));
-    const long long* head = (const long long*)(hs + 32);
+    const long long* head = hs + 4;
     for (long long j = 0; j < ns; j++) {
         const long long* r = j < R ? head + j * w : rest.data() + (j - R) * w;
         g.key[j] = (uint64_t)r[0];
