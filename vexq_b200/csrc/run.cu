@@ -62,10 +62,24 @@ __global__ void __launch_bounds__(256) k_merge_batch(const VQMergeDesc* d, int n
     merge_entry(w - m.e0, m.part_f, m.part_i, m.nblocks, m.G, m.nf, m.ni, m.fkind, m.ikind, m.out_f, m.out_i);
 }
 
-// Atomic path: per-slot initial values (counts 0, MIN/MAX identities).
-// Every slot at its identities in one pass (keys empty, first-row keys max,
+// n words of v from p on (8-byte aligned), by all threads of the grid: whole
+// 16-byte stores, consecutive threads consecutive addresses.
+__device__ __forceinline__ void fill64(void* p, long long n, unsigned long long v) {
+    unsigned long long* q = (unsigned long long*)p;
+    const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x, all = (long long)gridDim.x * blockDim.x;
+    const long long head = ((uintptr_t)q & 15) ? 1 : 0, pairs = (n - head) >> 1;
+    if (n <= 0) return;
+    if (tid == 0 && head) q[0] = v;
+    ulonglong2* w = (ulonglong2*)(q + head);
+    for (long long i = tid; i < pairs; i += all) w[i] = make_ulonglong2(v, v);
+    if (tid == 0 && ((n - head) & 1)) q[n - 1] = v;
+}
+
+// Atomic path: every slot at its identities (keys empty, first-row keys max,
 // integer accumulators at their kind's identity, fixed-point digits and
-// special flags 0), and the run's counters and error word cleared.
+// special flags 0), and the run's counters and error word cleared. Bound by L2
+// writes: field by field, so a warp's stores are whole lines (slot by slot, a
+// thread's 32 bytes of digits at a time, 720K slots took 12.5 us).
 __global__ void k_init_table(unsigned long long* keys, long long* first, long long* acc_i, int ni, const long long* init_i,
                              long long* acc_fx, unsigned* special, int nf, long long nslots, int hash,
                              unsigned long long* ngroups, int* error, unsigned long long* n_out) {
@@ -73,20 +87,15 @@ __global__ void k_init_table(unsigned long long* keys, long long* first, long lo
         *ngroups = 0ull;
         *error = 0;
         n_out[0] = n_out[1] = n_out[2] = 0ull;  // groups, and the top-k's counters
+        if (hash) keys[nslots - 1] = 0ull;      // used flag of the key equal to the empty sentinel
     }
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < nslots; i += (long long)gridDim.x * blockDim.x) {
-        if (hash) keys[i] = (i == nslots - 1) ? 0ull : VQ_EMPTY_KEY;
-        first[i] = 0x7FFFFFFFFFFFFFFFLL;
-        for (int s = 0; s < ni; s++) acc_i[(long long)s * nslots + i] = init_i[s];
-        for (int f = 0; f < nf; f++) {
-            long long* d = acc_fx + ((long long)f * nslots + i) * 4;  // 8-byte aligned only (odd slot counts)
-            d[0] = 0;
-            d[1] = 0;
-            d[2] = 0;
-            d[3] = 0;
-            special[(long long)f * nslots + i] = 0u;
-        }
-    }
+    if (hash) fill64(keys, nslots - 1, VQ_EMPTY_KEY);
+    fill64(first, nslots, 0x7FFFFFFFFFFFFFFFull);
+    for (int s = 0; s < ni; s++) fill64(acc_i + (long long)s * nslots, nslots, (unsigned long long)init_i[s]);
+    fill64(acc_fx, (long long)nf * nslots * 4, 0ull);
+    const long long nsp = (long long)nf * nslots;  // 4-byte flags, from an 8-byte boundary
+    fill64(special, nsp >> 1, 0ull);
+    if (blockIdx.x == 0 && threadIdx.x == 0 && (nsp & 1)) special[nsp - 1] = 0u;
 }
 
 // Compacts occupied slots (count > 0) and turns exact fixed-point sums into
@@ -398,6 +407,7 @@ __device__ __forceinline__ unsigned long long vq_rank(long long bits, bool isnul
 }
 // The groups a top-k selects from: a group table as the scan left it (np null:
 // every slot with a row count), or compacted groups (*np of them).
+constexpr long long kTopDouble = -1;
 struct VQTop {
     const unsigned long long* keys;
     const long long* first;
@@ -410,8 +420,10 @@ struct VQTop {
     long long n, stride;           // slots (or the most groups); distance between banks
     int ni, nf, hash;              // hash: keys[] holds the keys (else the slot is the key)
     int kind, vbank, vpos, nnpos, fmin_key, desc, limit;
-    unsigned long long* rank;      // [n] sort rank, 0 where there is no group
-    unsigned long long* wmax;      // [(n + 31) / 32] largest rank of every 32
+    unsigned long long* rank;      // [n] sort rank of every slot, 0 without a group
+    unsigned long long* wmax;      // [parts] largest sort rank of every 32 slots, 0 without a group
+    unsigned long long* bmax;      // [(parts + 7) / 8] the same of every 256
+    long long parts;
     unsigned long long* cnt;       // groups, selected groups, blocks done: 0 before k_rank
     const int* error;
     long long R, cap;              // rows that fit the host block, and at all
@@ -424,43 +436,57 @@ __device__ __forceinline__ double top_float(const VQTop& t, int f, long long i) 
     return t.np ? t.fval[at] : vq_fx_result(t.fx + at * 4, t.fx_lsb[f], t.special[at]);
 }
 
-// Rank of the ORDER BY output of every group: its raw bits (NULL flag) mapped by
-// vq_rank so that a larger rank sorts first, and the largest rank of each 32
-// slots. The table is read where it lies (one pass over the occupied counts,
-// the sort column's bank and 8 bytes written a slot), not compacted first: 720K
-// slots 9 us, against 17 + 5 for the compaction and the ranks of its output.
+__device__ __forceinline__ bool top_occupied(const VQTop& t, long long n, long long i) {
+    return i < n && (t.np || t.ival[i] != 0);
+}
+
+// Sort rank of group i: its ORDER BY output's raw bits (NULL flag) mapped by
+// vq_rank so that a larger rank sorts first.
+__device__ __forceinline__ unsigned long long top_rank(const VQTop& t, long long i) {
+    const long long nn = t.ival[(long long)t.nnpos * t.stride + i];
+    const bool isnull = t.kind != VEXQ_AGG_COUNT && nn == 0;
+    long long bits;
+    if (t.vbank == 1) {  // float sum bank
+        double v = top_float(t, t.vpos, i);
+        if (t.kind == VEXQ_AGG_AVG) v = v / (double)nn;
+        bits = __double_as_longlong(v);
+    } else {
+        bits = t.ival[(long long)t.vpos * t.stride + i];
+        if (t.fmin_key) bits = __double_as_longlong(vq_fkey_inv((unsigned long long)bits));
+    }
+    return vq_rank(bits, isnull, t.desc);
+}
+
+// The largest rank of every 32 slots (a warp's) and of every 256 (the block's),
+// and the number of groups. The table is read where it lies (the row counts and
+// the sort column's bank), not compacted first; 8 bytes a slot are written.
 __global__ void __launch_bounds__(256) k_rank(const __grid_constant__ VQTop t) {
     __shared__ unsigned warp_groups[8];
+    __shared__ unsigned long long warp_max[2][8];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const long long n = t.np ? (long long)min(*t.np, (unsigned long long)t.n) : t.n;
-    const long long stride = (long long)gridDim.x * blockDim.x;
     unsigned groups = 0u;
-    for (long long b = (long long)blockIdx.x * blockDim.x + warp * 32; b < t.n; b += stride) {
-        const long long i = b + lane;
-        const bool occ = i < n && (t.np || t.ival[i] != 0);
-        unsigned long long rank = 0ull;
-        if (occ) {
-            const long long nn = t.ival[(long long)t.nnpos * t.stride + i];
-            const bool isnull = t.kind != VEXQ_AGG_COUNT && nn == 0;
-            long long bits;
-            if (t.vbank == 1) {  // float sum bank
-                double v = top_float(t, t.vpos, i);
-                if (t.kind == VEXQ_AGG_AVG) v = v / (double)nn;
-                bits = __double_as_longlong(v);
-            } else {
-                bits = t.ival[(long long)t.vpos * t.stride + i];
-                if (t.fmin_key) bits = __double_as_longlong(vq_fkey_inv((unsigned long long)bits));
-            }
-            rank = vq_rank(bits, isnull, t.desc);
-        }
-        if (i < t.n) t.rank[i] = rank;
+    int turn = 0;
+    for (long long b = blockIdx.x; b * 8 < t.parts; b += gridDim.x, turn ^= 1) {
+        const long long part = b * 8 + warp;
+        const bool occ = top_occupied(t, n, part * 32 + lane);
+        const unsigned long long rank = occ ? top_rank(t, part * 32 + lane) : 0ull;
+        if (part * 32 + lane < t.n) t.rank[part * 32 + lane] = rank;
         groups += __popc(__ballot_sync(0xffffffffu, occ));
-        unsigned long long m = rank;
-        for (int o = 16; o > 0; o >>= 1) {
-            const unsigned long long x = __shfl_xor_sync(0xffffffffu, m, o);
-            m = x > m ? x : m;
+        // the warp's maximum: the high words, then the low words of the lanes that hold it
+        const unsigned hi = __reduce_max_sync(0xffffffffu, (unsigned)(rank >> 32));
+        const unsigned lo = __reduce_max_sync(0xffffffffu, (unsigned)(rank >> 32) == hi ? (unsigned)rank : 0u);
+        if (lane == 0) {
+            const unsigned long long m = (unsigned long long)hi << 32 | lo;
+            if (part < t.parts) t.wmax[part] = m;
+            warp_max[turn][warp] = m;
         }
-        if (lane == 0) t.wmax[b >> 5] = m;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            unsigned long long m = 0ull;
+            for (int w = 0; w < 8; w++) m = max(m, warp_max[turn][w]);
+            t.bmax[b] = m;
+        }
     }
     if (lane == 0) warp_groups[warp] = groups;
     __syncthreads();
@@ -471,30 +497,37 @@ __global__ void __launch_bounds__(256) k_rank(const __grid_constant__ VQTop t) {
     }
 }
 
-// q-th largest (from 0) of the block's 16 values a thread by radix select, most
-// significant byte first: each round counts, in shared memory, the next byte of
-// the values that match the bytes chosen so far, and one warp walks the 256
-// counts from the top to the byte holding the q-th largest.
-__device__ __forceinline__ unsigned long long block_kth16(const unsigned long long (&v)[16], unsigned q) {
+// A value that q + 1 of the block's kValues values a thread reach, and few more:
+// the q-th largest (from 0) but for low bits. Radix select, most significant
+// byte first: each round counts, in shared memory, the next byte of the values
+// that match the bytes chosen so far, and one warp walks the 256 counts from
+// the top to the byte holding the q-th largest; a byte that no other value shares
+// ends it.
+template <int kValues>
+__device__ __forceinline__ unsigned long long block_kth(const unsigned long long (&v)[kValues], unsigned q) {
     __shared__ unsigned hist[256];
     __shared__ unsigned long long prefix;
-    __shared__ unsigned need;
-    if (threadIdx.x == 0) { prefix = 0ull; need = q; }
+    __shared__ unsigned need, alone;
+    if (threadIdx.x == 0) { prefix = 0ull; need = q; alone = 0u; }
+    if (threadIdx.x < 256) hist[threadIdx.x] = 0u;
+    __syncthreads();
     for (int shift = 56; shift >= 0; shift -= 8) {
-        for (int i = threadIdx.x; i < 256; i += blockDim.x) hist[i] = 0u;
-        __syncthreads();
         const unsigned long long hi_mask = shift == 56 ? 0ull : (~0ull << (shift + 8));
         const unsigned long long pre = prefix;
         const unsigned nd = need;  // both rewritten only after the next barrier
 #pragma unroll
-        for (int k = 0; k < 16; k++)
+        for (int k = 0; k < kValues; k++)
             if ((v[k] & hi_mask) == pre) atomicAdd(&hist[(v[k] >> shift) & 255u], 1u);
         __syncthreads();
         if (threadIdx.x < 32) {
             const int lane = threadIdx.x;
             unsigned c[8], sum = 0u;
 #pragma unroll
-            for (int k = 0; k < 8; k++) { c[k] = hist[255 - (8 * lane + k)]; sum += c[k]; }
+            for (int k = 0; k < 8; k++) {
+                c[k] = hist[255 - (8 * lane + k)];
+                hist[255 - (8 * lane + k)] = 0u;
+                sum += c[k];
+            }
             unsigned incl = sum;
             for (int o = 1; o < 32; o <<= 1) {
                 const unsigned t = __shfl_up_sync(0xffffffffu, incl, o);
@@ -507,6 +540,7 @@ __device__ __forceinline__ unsigned long long block_kth16(const unsigned long lo
                     if (nd < acc + c[k]) {
                         prefix = pre | ((unsigned long long)(255 - (8 * lane + k)) << shift);
                         need = nd - acc;
+                        alone = c[k] == 1u;
                         break;
                     }
                     acc += c[k];
@@ -514,89 +548,84 @@ __device__ __forceinline__ unsigned long long block_kth16(const unsigned long lo
             }
         }
         __syncthreads();
+        if (alone) break;
     }
     return prefix;
 }
 
-// The block's 1,024 values, one a thread, sorted descending (bitonic; strides
-// below 32 in registers).
-__device__ __forceinline__ unsigned long long block_sort1024(unsigned long long v) {
-    __shared__ unsigned long long sh[1024];
-    const int t = threadIdx.x;
-    for (int k = 2; k <= 1024; k <<= 1)
-        for (int j = k >> 1; j > 0; j >>= 1) {
-            unsigned long long o;
-            if (j >= 32) {
-                __syncthreads();
-                sh[t] = v;
-                __syncthreads();
-                o = sh[t ^ j];
-            } else {
-                o = __shfl_xor_sync(0xffffffffu, v, j);
-            }
-            const bool keep_max = ((t & j) == 0) == ((t & k) == 0);
-            v = keep_max ? (v > o ? v : o) : (v < o ? v : o);
-        }
-    return v;
-}
-
-// The groups ORDER BY … LIMIT can need. The slots are parted into at least
-// 1,024 parts; the LIMIT-th largest of the parts' largest ranks is a threshold
-// that at least LIMIT groups reach, and few others (LIMIT 100 of 200K groups in
-// 1,024 parts: about 105). Every block finds it for itself from the 32-slot
-// maxima (180 KB for 720K slots), then takes its share of the ranks; the groups
-// at or above it (ties included; every group when fewer parts than LIMIT hold
-// one) are written as rows (key, first-row key, integer bank, float bank as raw
-// bits) straight into pinned host memory. One launch of one block an SM, 5 us,
-// against 25 + 5 us for a one-block select over 16,384 samples and the gather,
-// with four copies back.
+// The groups ORDER BY … LIMIT can need. The LIMIT-th largest of the parts'
+// largest ranks is a threshold that at least LIMIT groups reach, and few others
+// (LIMIT 100 of 200K groups: about 105). Every block finds it for itself from
+// the maxima, then takes its share of the parts that reach it; their groups at
+// or above it (ties included; every group when fewer parts than LIMIT hold one)
+// are written straight into pinned host memory as rows: key, first-row key,
+// integer bank, and per float sum its four digits and special flags (compacted
+// groups: the sum's bits, 0, 0, 0 and kTopDouble), which the host turns into
+// doubles. Bound by latency: the dependent reads, and fetching the kernel's code,
+// of which the conversion would be the larger part.
 __global__ void __launch_bounds__(1024) k_select(const __grid_constant__ VQTop t) {
-    __shared__ unsigned long long threshold;
-    const long long m = (t.n + 31) / 32;
     const unsigned q = (unsigned)max(t.limit, 1) - 1u;
+    unsigned long long thr;
     if (q < 256u) {
-        unsigned long long v = 0ull;
-        for (long long i = threadIdx.x; i < m; i += 1024) {
-            const unsigned long long x = t.wmax[i];
-            v = x > v ? x : v;
-        }
-        v = block_sort1024(v);
-        if (threadIdx.x == q) threshold = v;
-        __syncthreads();
+        // the maxima of 256 slots where there are 1,024 of them
+        const long long blocks = (t.parts + 7) / 8, m = blocks >= 1024 ? blocks : t.parts;
+        const unsigned long long* a = blocks >= 1024 ? t.bmax : t.wmax;
+        unsigned long long v[1] = {0ull};
+#pragma unroll 8
+        for (long long i = threadIdx.x; i < m; i += 1024) v[0] = max(v[0], a[i]);
+        thr = block_kth(v, q);
     } else {
         unsigned long long v[16];
 #pragma unroll
         for (int k = 0; k < 16; k++) {
             v[k] = 0ull;
-            for (long long i = threadIdx.x + k * 1024; i < m; i += 16384) {
-                const unsigned long long x = t.wmax[i];
-                v[k] = x > v[k] ? x : v[k];
+            for (long long i = threadIdx.x + k * 1024; i < t.parts; i += 16384) v[k] = max(v[k], t.wmax[i]);
+        }
+        thr = block_kth(v, q);
+    }
+    const int lane = threadIdx.x & 31;
+    const int w = 2 + t.ni + 5 * t.nf;
+    const long long n = t.np ? (long long)min(*t.np, (unsigned long long)t.n) : t.n;
+    // 32 parts a warp at a time, one a lane; the warp goes through those that
+    // reach the threshold together, and writes each candidate's row together (a
+    // lane a word: the loads behind it are in flight at once)
+    const long long stride = (long long)gridDim.x * 1024;
+    for (long long p0 = (long long)blockIdx.x * 1024 + (threadIdx.x & ~31); p0 < t.parts; p0 += stride) {
+        unsigned hit = __ballot_sync(0xffffffffu, p0 + lane < t.parts && t.wmax[p0 + lane] >= thr);
+        for (; hit; hit &= hit - 1u) {
+            const long long i0 = (p0 + __ffs(hit) - 1) * 32;
+            // (a threshold of 0 takes every group: occupancy tells a group of rank 0)
+            unsigned take = __ballot_sync(0xffffffffu, i0 + lane < n && t.rank[i0 + lane] >= thr && (thr != 0ull || top_occupied(t, n, i0 + lane)));
+            unsigned long long at = 0ull;
+            if (lane == 0) at = atomicAdd(t.cnt + 1, (unsigned long long)__popc(take));
+            at = __shfl_sync(0xffffffffu, at, 0);
+            for (; take; take &= take - 1u, at++) {
+                if ((long long)at >= t.cap) break;
+                const long long i = i0 + __ffs(take) - 1, p = (long long)at;
+                long long* o = p < t.R ? t.host + 4 + p * w : t.rest + (p - t.R) * w;
+                for (int j = lane; j < w; j += 32) {
+                    long long x;
+                    if (j == 0) x = (long long)(!t.hash ? (unsigned long long)i : !t.np && i == t.n - 1 ? VQ_EMPTY_KEY : t.keys[i]);
+                    else if (j == 1) x = t.first[i];
+                    else if (j < 2 + t.ni) x = t.ival[(long long)(j - 2) * t.stride + i];
+                    else {
+                        const int f = (j - 2 - t.ni) / 5, d = (j - 2 - t.ni) % 5;
+                        const long long a = (long long)f * t.stride + i;
+                        if (t.np) x = d == 0 ? __double_as_longlong(t.fval[a]) : d == 4 ? kTopDouble : 0;
+                        else x = d < 4 ? t.fx[a * 4 + d] : (long long)t.special[a];
+                    }
+                    o[j] = x;
+                }
             }
         }
-        const unsigned long long kth = block_kth16(v, q);
-        if (threadIdx.x == 0) threshold = kth;
-        __syncthreads();
     }
-    const unsigned long long thr = threshold;
-    const long long w = 2 + t.ni + t.nf;
-    const long long n = t.np ? (long long)min(*t.np, (unsigned long long)t.n) : t.n;
-    for (long long i = (long long)blockIdx.x * 1024 + threadIdx.x; i < n; i += (long long)gridDim.x * 1024) {
-        if (t.rank[i] < thr || (thr == 0ull && !t.np && t.ival[i] == 0)) continue;
-        const long long p = (long long)atomicAdd(t.cnt + 1, 1ull);
-        if (p >= t.cap) continue;
-        long long* o = p < t.R ? t.host + 4 + p * w : t.rest + (p - t.R) * w;
-        o[0] = (long long)(!t.hash ? (unsigned long long)i : !t.np && i == t.n - 1 ? VQ_EMPTY_KEY : t.keys[i]);
-        o[1] = t.first[i];
-        for (int s = 0; s < t.ni; s++) o[2 + s] = t.ival[(long long)s * t.stride + i];
-        for (int f = 0; f < t.nf; f++) o[2 + t.ni + f] = __double_as_longlong(top_float(t, f, i));
-    }
-    __threadfence();
+    // the last block hands the counts out; every block's claims have returned
+    // before its arrival (the rows reach the host with the kernel's end)
     __syncthreads();
-    if (threadIdx.x == 0 && atomicAdd(t.cnt + 2, 1ull) == gridDim.x - 1) {  // the last block
-        __threadfence();
+    if (threadIdx.x == 0 && atomicAdd(t.cnt + 2, 1ull) == gridDim.x - 1) {
         t.host[0] = (long long)(t.np ? (unsigned long long)n : t.cnt[0]);
         t.host[1] = t.error ? *t.error : 0;
-        t.host[2] = (long long)*(volatile unsigned long long*)(t.cnt + 1);
+        t.host[2] = (long long)atomicAdd(t.cnt + 1, 0ull);
     }
 }
 
@@ -1346,13 +1375,14 @@ int topk_groups(RunCtx& rc, Compacted& c, Groups& g) {
     int fmin_key = (p.slots[vslot].kind == S_FMIN || p.slots[vslot].kind == S_FMAX) ? 1 : 0;
     if (a.kind == VEXQ_AGG_COUNT) vbank = 0;
     const bool table = c.n < 0;  // a deferred run
-    const long long w = 2 + p.ni + p.nf, nmax = table ? c.cap_out : c.n;
-    const size_t b_rank = (size_t)nmax * 8, b_max = (size_t)(nmax + 31) / 32 * 8;
-    // rank | maxima | counters (compacted groups) | rows past the host block's
+    const long long w = 2 + p.ni + 5 * p.nf, nmax = table ? c.cap_out : c.n;
+    const long long parts = (nmax + 31) / 32;
+    const size_t b_max = (size_t)(nmax + parts + (parts + 7) / 8) * 8;
+    // ranks, maxima | counters (compacted groups) | rows past the host block's
     // R: the last run's candidates and as many again, at least 1,024
     long long R = 1024;
     while (R < 2 * p.topk_seen && R < kCap) R <<= 1;
-    p.scratch_d.ensure(b_rank + b_max + 32 + (size_t)(kCap - R) * w * 8);
+    p.scratch_d.ensure(b_max + 32 + (size_t)(kCap - R) * w * 8);
     p.h_stage.ensure(32 + (size_t)R * w * 8);
     void* mapped = nullptr;
     if (cudaHostGetDevicePointer(&mapped, p.h_stage.p, 0) != cudaSuccess) fail(VEXQ_EDEVICE, "pinned host memory has no device address");
@@ -1360,8 +1390,10 @@ int topk_groups(RunCtx& rc, Compacted& c, Groups& g) {
     std::memset(&t, 0, sizeof t);
     t.rank = p.scratch_d.as<unsigned long long>();
     t.wmax = t.rank + nmax;
-    t.cnt = table ? c.n_dev : t.wmax + (nmax + 31) / 32;
-    t.rest = (long long*)(p.scratch_d.as<char>() + b_rank + b_max + 32);
+    t.parts = parts;
+    t.bmax = t.wmax + parts;
+    t.cnt = table ? c.n_dev : t.bmax + (parts + 7) / 8;
+    t.rest = (long long*)(p.scratch_d.as<char>() + b_max + 32);
     t.host = (long long*)mapped;
     t.R = R;
     t.cap = kCap;
@@ -1394,10 +1426,11 @@ int topk_groups(RunCtx& rc, Compacted& c, Groups& g) {
         t.np = c.n_dev;
         VQ_CUDA(cudaMemsetAsync(t.cnt, 0, 24, rc.s));
     }
-    const int gr = (int)std::max<long long>(1, std::min<long long>((nmax + 255) / 256, (long long)sm_count() * 8));
+    const int gr = (int)std::max<long long>(1, std::min<long long>((parts + 7) / 8, (long long)sm_count() * 8));
     k_rank<<<gr, 256, 0, rc.s>>>(t);
     launch_check(rc.s, "k_rank");
-    k_select<<<(int)std::max<long long>(1, std::min<long long>((nmax + 1023) / 1024, sm_count())), 1024, 0, rc.s>>>(t);
+    // few blocks: every one reads all the maxima
+    k_select<<<(int)std::max<long long>(1, std::min<long long>((parts + 1023) / 1024, 32)), 1024, 0, rc.s>>>(t);
     launch_check(rc.s, "k_select");
     VQ_CUDA(cudaGetLastError());
     rc.launches += 2;
@@ -1441,7 +1474,11 @@ int topk_groups(RunCtx& rc, Compacted& c, Groups& g) {
         g.key[j] = (uint64_t)r[0];
         g.first[j] = r[1];
         for (int s = 0; s < p.ni; s++) g.ival[s][j] = r[2 + s];
-        for (int f = 0; f < p.nf; f++) std::memcpy(&g.fval[f][j], &r[2 + p.ni + f], 8);
+        for (int f = 0; f < p.nf; f++) {
+            const long long* d = r + 2 + p.ni + 5 * f;
+            if (d[4] == kTopDouble) std::memcpy(&g.fval[f][j], d, 8);
+            else g.fval[f][j] = vq_fx_result(d, p.fx_lsb[f], (unsigned)d[4]);
+        }
     }
     return 1;
 }
