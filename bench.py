@@ -203,7 +203,7 @@ def batch_leg(nplans, steps, warmup, peak, cpu=True):
     """One step = every plan of the batching workload. The batched arm (one
     persistent launch per path class, graph replay, autotuned) against the
     same plans one by one through vexq_plan_run; device time is the kernels
-    alone (CUDA events inside the library, before the copy back). The CPU
+    alone (the device clock inside the library, before the copy back). The CPU
     figure is one pass of the C++ restatement of ParallelHashAggregate over
     every plan on all host threads."""
     from vexq_b200 import exec as X

@@ -322,10 +322,12 @@ int32_t vexq_result_free(vexq_result_t r);
 /* Device timing of the last run: kernel milliseconds and launches. */
 int32_t vexq_result_stats(vexq_result_t r, double* kernel_ms, int32_t* launches,
                           int64_t* rows_scanned, int64_t* bytes_scanned);
-/* Duration of the run's scan kernel launches (CUDA events on the plan's
- * stream), in milliseconds. On the register path a scan and the partial merge
- * launched as its programmatic dependent overlap, and the pair is timed as
- * one span; the atomic paths time the scan alone. */
+/* Duration of the run's scan kernel launches, in milliseconds, by the device's
+ * clock: from the first block's start to the last block's end (with CUDA events
+ * on the plan's stream where a launch of its own merges the partials, or a
+ * partitioned join probes). On the register path a scan and the partial merge,
+ * inside it or overlapping its drain, are timed as one span; the atomic paths
+ * time the scan alone. */
 int32_t vexq_result_scan_ms(vexq_result_t r, double* out);
 /* Everything above in one call (rows, columns, kernel and scan milliseconds,
  * launches, rows and bytes scanned); any pointer may be NULL. No reference

@@ -103,6 +103,12 @@ __device__ __forceinline__ void asm_write(const VQAsmDesc& d, const VQAsmCol* co
     }
 }
 
+// The run's stamps and this moment, to the host.
+__device__ void asm_clock(const VQAsmDesc& d, VQAsmHdr* h) {
+    for (int i = 0; i < VQ_CLK_END; i++) h->clk[i] = __ldcg(d.clk + i);
+    h->clk[VQ_CLK_END] = vq_clock();
+}
+
 // Bound by latency, not bytes: 1,000 groups of a 4M-row scan read 500 KB of
 // marks and 68 KB of table. The first-row bitmap is divided over the CTAs for
 // the count, slots and output rows over all of the cluster's threads.
@@ -212,6 +218,7 @@ k_assemble(const VQAsmDesc* descs, char* base, char* const* basep) {
         VQAsmHdr* h = reinterpret_cast<VQAsmHdr*>(out);
         h->n = (unsigned long long)n;
         h->err = *d.error;
+        if (d.clk && d.write) asm_clock(d, h);
         d.pref[d.nwords / 4 + kAsmCtas] = (unsigned)n;
     }
 }
@@ -227,6 +234,9 @@ __global__ void __launch_bounds__(256) k_asm_write(const VQAsmDesc* g, char* bas
     __syncthreads();
     const long long n = d.pref[d.nwords / 4 + kAsmCtas];
     asm_write(d, cols, base + d.out, min(n, d.cap_rows), (blockIdx.x * blockDim.x + threadIdx.x) >> 5, (gridDim.x * blockDim.x) >> 5);
+    if (!d.clk) return;
+    __syncthreads();
+    if (threadIdx.x == 0 && atomicAdd(d.clk + VQ_CLK_DONE, 1ull) % gridDim.x == gridDim.x - 1) asm_clock(d, reinterpret_cast<VQAsmHdr*>(base + d.out));
 }
 
 int out_width(int type) { return (type == VEXQ_TYPE_INT64 || type == VEXQ_TYPE_FLOAT64) ? 8 : type == VEXQ_TYPE_BOOL ? 1 : 4; }

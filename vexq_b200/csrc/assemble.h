@@ -38,6 +38,7 @@ struct VQAsmDesc {
     const unsigned* special;
     const int* fx_lsb;
     const int* error;
+    unsigned long long* clk;  // the run's device clock (null: none)
     const VQAsmCol* cols;
     unsigned* bits;         // [nwords] a bit per row that is some group's first
     unsigned* pref;         // [nwords / 4 + 9] set bits before each four words, then the CTAs' totals and the group count
@@ -49,8 +50,9 @@ struct VQAsmDesc {
 };
 struct VQAsmHdr {           // at the start of a table's output
     unsigned long long n;
-    int err;
-    int pad[13];
+    int err, pad;
+    unsigned long long clk[VQ_CLK_END + 1];  // the run's device clock and the columns' end
+    unsigned long long pad8;
 };
 
 // Byte layout of a plan's output columns for at most cap rows.

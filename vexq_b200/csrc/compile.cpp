@@ -1166,12 +1166,14 @@ static void choose_regs_forms(Plan& p) {
 // first-row keys are order-free as atomics. Float MIN/MAX keep the merge
 // kernel, whose fold in block order keeps the first of two equal extremes
 // (+0 against -0), and so do plans whose blocks would add more than 128
-// atomics. VEXQ_TUNE "rfuse=0" keeps the merge kernel for measurement,
+// atomics. A join's integer accumulators merge in its probe the same way (6.0M
+// probe rows, 2 groups: 81 us with the merge kernel's 10, 73 us without); its
+// float sums keep the kernel. VEXQ_TUNE "rfuse=0" keeps the merge kernel for measurement,
 // "rfuse=2" folds any eligible plan into the scan, "rcopies=K" sets the
 // accumulator copies.
 static void choose_regs_fused(Plan& p) {
     p.rfused = false;
-    if (p.path != AggPath::Regs || p.is_join || !p.t || p.nf > 16) return;
+    if (p.path != AggPath::Regs || !p.t || p.nf > 16) return;
     if (p.t->nrows > (int64_t(1) << 31)) return;  // the window holds sums of 2^31 rows
     int force = 1;
     if (const char* e = std::getenv("VEXQ_TUNE")) {
@@ -1195,6 +1197,7 @@ static void choose_regs_fused(Plan& p) {
         const Slot& sl = p.slots[s];
         if (sl.kind == S_FMIN || sl.kind == S_FMAX) return;
         if (sl.kind != S_FSUM) continue;
+        if (p.is_join) return;  // a join can emit more than 2^31 rows
         if (!p.rfma[s] && !p.rdx[s]) return;  // a sum that may meet NaN or inf
         const INode& x = p.ir[sl.input];
         if (!x.bounded || !std::isfinite(x.lo) || !std::isfinite(x.hi)) return;
@@ -1451,9 +1454,11 @@ void emit_regs_flush(std::ostringstream& os, const Plan& p, int block, const Flu
            << " + t), (unsigned long long)vq_racc_identity(kd)));\n";
         os << "                P.rout_i[t] = (long long)v;\n";
         os << "            }\n";
+        os << "            __syncthreads();\n";
         os << "            if (threadIdx.x == 0) {\n";
         os << "                *P.rerr_out = atomicExch(P.error, 0);\n";
         os << "                atomicExch(P.racc_done, 0u);\n";
+        os << "                vq_clock_out(P.clk, P.clk_out);\n";
         os << "            }\n";
         os << "        }\n";
         os << "    } else {\n";
@@ -1490,6 +1495,7 @@ void emit_regs_flush(std::ostringstream& os, const Plan& p, int block, const Flu
         os << "            if (threadIdx.x == 0) {\n";
         os << "                *P.merr_out = atomicExch(P.error, 0);\n";
         os << "                atomicExch(P.mdone, 0u);\n";
+        os << "                vq_clock_out(P.clk, P.clk_out);\n";
         os << "            }\n";
         os << "        }\n";
         os << "    }\n";
@@ -1779,6 +1785,15 @@ void emit_cache_flush(std::ostringstream& os, const Plan& p) {
         }
     }
     os << "    }\n";
+}
+
+// The scan's clock stamps: its first block's start, and (group tables; the
+// register path's last block hands its end out) its last block's end.
+void emit_clock_start(std::ostringstream& os) {
+    os << "    if (P.clk && blockIdx.x == 0 && threadIdx.x == 0) P.clk[VQ_CLK_SCAN] = vq_clock();\n";
+}
+void emit_clock_end(std::ostringstream& os, const Plan& p) {
+    if (p.path != AggPath::Regs) os << "    if (P.clk && threadIdx.x == 0) atomicMax(P.clk + VQ_CLK_SCAN_END, vq_clock());\n";
 }
 
 std::string kernel_head(const std::string& name, int block, int min_blocks = 0) {
@@ -2144,6 +2159,7 @@ static std::string gen_agg_kernel(Plan& p, const std::vector<int>& key_nodes, in
     p.smem = p.smem_groups > 0 ? cache_bytes(p) : loop.smem();
     loop.prologue(os);
     os << kernel_head("vq_agg", block, p.min_blocks);
+    emit_clock_start(os);
     if (p.path == AggPath::Regs) emit_regs_decl(os, p);
     if (p.smem_groups > 0) emit_cache_init(os, p);
     loop.block_steps = p.smem_groups > 0;
@@ -2156,6 +2172,7 @@ static std::string gen_agg_kernel(Plan& p, const std::vector<int>& key_nodes, in
     }
     if (p.path == AggPath::Regs) emit_regs_flush(os, p, block);
     if (p.smem_groups > 0) emit_cache_flush(os, p);
+    emit_clock_end(os, p);
     os << "}\n";
     return os.str();
 }
@@ -2719,6 +2736,7 @@ static std::string gen_probe_kernel(Plan& p, const std::vector<int>& key_nodes, 
     p.smem = loop.smem();
     loop.prologue(os);
     os << kernel_head("vq_agg", block, p.min_blocks);
+    emit_clock_start(os);
     // a build the host did not wait for: its failure or emptiness is raised
     // in this kernel's error word, which comes back with the results
     os << "    if (P.berr && blockIdx.x == 0 && threadIdx.x == 0) {\n";
@@ -2739,6 +2757,7 @@ static std::string gen_probe_kernel(Plan& p, const std::vector<int>& key_nodes, 
         os << "    }\n";
     }
     if (p.path == AggPath::Regs) emit_regs_flush(os, p, block);
+    emit_clock_end(os, p);
     os << "}\n";
     return os.str();
 }

@@ -548,6 +548,24 @@ __device__ __forceinline__ ulonglong2 vq_ld_slot(const ulonglong2* p) {
 #endif
 }
 
+// The device's clock, nanoseconds. Kernels stamp their run's start and end with
+// it: a timing event between two launches keeps the second from starting while
+// the first drains, about 3 us each (a six-group scan of 10,000 rows took 31 us
+// a run with two events around it, 22 us with the stamps).
+__device__ __forceinline__ unsigned long long vq_clock() {
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+    return t;
+}
+
+// The register path's last block: the run's stamps, to the host.
+__device__ __forceinline__ void vq_clock_out(const unsigned long long* clk, unsigned long long* out) {
+    if (!clk) return;
+    out[0] = __ldcg(clk + VQ_CLK_BUILD);
+    out[1] = __ldcg(clk + VQ_CLK_SCAN);
+    out[2] = vq_clock();
+}
+
 // The same for one word of the direct-mapped build table.
 __device__ __forceinline__ unsigned long long vq_ld_dword(const unsigned long long* p) {
 #ifdef VQ_KEEP_TABLES

@@ -94,6 +94,10 @@ struct VQParams {
     long long* mout_i;             // [G][NI + 1] merged integer entries
     int* merr_out;                 // the error word handed out with the merged row
     unsigned* mdone;               // blocks that have written their partials
+    // ---- the run's device clock, nanoseconds (VQ_CLK_* words; null: the host
+    //      times the run with events) ----
+    unsigned long long* clk;
+    unsigned long long* clk_out;   // register path: build start, scan start and end handed out with the merged row
     // ---- COUNT(DISTINCT) sets, one per distinct aggregate: [cap][2] (group
     //      key, value image) and a state word per slot (0 empty, 1 being
     //      written, 2 published); cap = dmask + 1 ----
@@ -120,6 +124,17 @@ struct VQParams {
     int pbits;                 // radix join: partition = top pbits bits of the key hash
     int fx_lsb[16];            // per float-sum slot: exponent of the window's LSB
 };
+
+// Words of a plan's device clock: the build's and the run's start, the scan's
+// first block's start and last block's end, the end of a compaction, and the
+// blocks of the last launch that have finished.
+#define VQ_CLK_BUILD 0
+#define VQ_CLK_BEGIN 1
+#define VQ_CLK_SCAN 2
+#define VQ_CLK_SCAN_END 3
+#define VQ_CLK_END 4
+#define VQ_CLK_DONE 5
+#define VQ_CLK_WORDS 8
 
 // One unit of a batched launch: chunks [cbeg, cend) of one plan, run by one
 // block; pslot is the unit's partial row within its plan (register path).

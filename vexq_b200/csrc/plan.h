@@ -249,6 +249,7 @@ struct Plan {
     // group tables assembled on the device (assemble.cu)
     OutPool out_pool;
     DevBuf d_asm, asm_bits, asm_scr;       // descriptor and columns; first-row bitmap; positions
+    DevBuf d_clk;                          // the run's device clock (VQ_CLK_* words)
     std::vector<char> asm_img;             //   as last uploaded
     long long asm_rows_seen = 0;           // groups of the last run (sizes the next block)
     // GROUP BY exactly the (non-NULL int64) join key on a group-table path:

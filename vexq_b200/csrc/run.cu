@@ -82,8 +82,12 @@ __device__ __forceinline__ void fill64(void* p, long long n, unsigned long long 
 // thread's 32 bytes of digits at a time, 720K slots took 12.5 us).
 __global__ void k_init_table(unsigned long long* keys, long long* first, long long* acc_i, int ni, const long long* init_i,
                              long long* acc_fx, unsigned* special, int nf, long long nslots, int hash,
-                             unsigned long long* ngroups, int* error, unsigned long long* n_out) {
+                             unsigned long long* ngroups, int* error, unsigned long long* n_out, unsigned long long* clk) {
     if (blockIdx.x == 0 && threadIdx.x == 0) {
+        if (clk) {
+            clk[VQ_CLK_BEGIN] = vq_clock();
+            clk[VQ_CLK_SCAN_END] = clk[VQ_CLK_END] = clk[VQ_CLK_DONE] = 0ull;
+        }
         *ngroups = 0ull;
         *error = 0;
         n_out[0] = n_out[1] = n_out[2] = 0ull;  // groups, and the top-k's counters
@@ -156,7 +160,7 @@ __device__ __forceinline__ unsigned long long vq_claim_block(bool occ, unsigned 
 __global__ void k_finalize(const unsigned long long* keys, const long long* first, const long long* acc_i,
                            const long long* acc_fx, const unsigned* special, long long nslots, int ni, int nf,
                            const int* fx_lsb, int hash, unsigned long long* n_out, unsigned long long* o_key,
-                           long long* o_first, long long* o_i, double* o_f, long long cap_out) {
+                           long long* o_first, long long* o_i, double* o_f, long long cap_out, unsigned long long* clk) {
     const long long stride = (long long)gridDim.x * blockDim.x;
     for (long long b0 = (long long)blockIdx.x * blockDim.x; b0 < nslots; b0 += stride) {  // block-uniform trip count
         const long long i = b0 + threadIdx.x;
@@ -165,6 +169,7 @@ __global__ void k_finalize(const unsigned long long* keys, const long long* firs
         if (occ) finalize_write(i, pos, keys, first, acc_i, acc_fx, special, nslots, ni, nf, fx_lsb, hash, o_key, o_first,
                                 o_i, o_f, cap_out);
     }
+    if (clk && threadIdx.x == 0) atomicMax(clk + VQ_CLK_END, vq_clock());
 }
 
 // Batched group tables: global slot g belongs to the table whose slot0 is the
@@ -217,6 +222,15 @@ __global__ void k_finalize_batch(const VQTableDesc* d, int n, long long total) {
                            t.fx_lsb, t.hash, t.o_key, t.o_first, t.o_i, t.o_f, t.cap_out);
         }
     }
+}
+
+// Direct-mapped join build: its table and scalars cleared, its start stamped.
+__global__ void k_clear_dmap(unsigned long long* dmap, long long n, unsigned long long* scalar, int ns, unsigned long long* clk) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        clk[VQ_CLK_BUILD] = vq_clock();
+        for (int i = 0; i < ns; i++) scalar[i] = 0ull;
+    }
+    fill64(dmap, n, 0ull);
 }
 
 // ---- exclusive scan (join build: slot counts → chain starts) ------------------------
@@ -408,6 +422,7 @@ __device__ __forceinline__ unsigned long long vq_rank(long long bits, bool isnul
 // The groups a top-k selects from: a group table as the scan left it (np null:
 // every slot with a row count), or compacted groups (*np of them).
 constexpr long long kTopDouble = -1;
+constexpr int kTopHead = 8;  // words before the rows in the host block
 struct VQTop {
     const unsigned long long* keys;
     const long long* first;
@@ -426,8 +441,9 @@ struct VQTop {
     long long parts;
     unsigned long long* cnt;       // groups, selected groups, blocks done: 0 before k_rank
     const int* error;
+    const unsigned long long* clk; // the run's device clock (null: none)
     long long R, cap;              // rows that fit the host block, and at all
-    long long* host;               // header (groups, error word, selected), rows [0, R)
+    long long* host;               // header (groups, error word, selected, clock), rows [0, R)
     long long* rest;               // rows [R, cap)
 };
 
@@ -602,7 +618,7 @@ __global__ void __launch_bounds__(1024) k_select(const __grid_constant__ VQTop t
             for (; take; take &= take - 1u, at++) {
                 if ((long long)at >= t.cap) break;
                 const long long i = i0 + __ffs(take) - 1, p = (long long)at;
-                long long* o = p < t.R ? t.host + 4 + p * w : t.rest + (p - t.R) * w;
+                long long* o = p < t.R ? t.host + kTopHead + p * w : t.rest + (p - t.R) * w;
                 for (int j = lane; j < w; j += 32) {
                     long long x;
                     if (j == 0) x = (long long)(!t.hash ? (unsigned long long)i : !t.np && i == t.n - 1 ? VQ_EMPTY_KEY : t.keys[i]);
@@ -626,6 +642,10 @@ __global__ void __launch_bounds__(1024) k_select(const __grid_constant__ VQTop t
         t.host[0] = (long long)(t.np ? (unsigned long long)n : t.cnt[0]);
         t.host[1] = t.error ? *t.error : 0;
         t.host[2] = (long long)atomicAdd(t.cnt + 1, 0ull);
+        if (t.clk) {
+            for (int i = 0; i < VQ_CLK_END; i++) t.host[3 + i] = (long long)__ldcg(t.clk + i);
+            t.host[3 + VQ_CLK_END] = (long long)vq_clock();
+        }
     }
 }
 
@@ -757,7 +777,25 @@ struct RunCtx {
     const JitKernel* k = nullptr;  // main kernel other than p.k_main (partition join)
     int grid = 0;                  // and its grid
     long long row0 = 0, row1 = 0;  // rows the main scan's ranges span
+    bool from_build = false;       // the device clock's build start begins the run (a build the host did not wait for)
+
+    // Whether the main kernel stamps the device clock: the scan and global
+    // probe kernels do, where the last launch can hand the stamps out (the
+    // register path's separate merge cannot).
+    bool stamped() const { return !k && (p.path != AggPath::Regs || p.rfused || p.merge_last); }
+    // Adds a stamped run's times (w: VQ_CLK_* words up to VQ_CLK_END; begin: its first launch's word).
+    void add_clock(const unsigned long long* w, int begin) {
+        auto ms = [](unsigned long long a, unsigned long long b) { return (float)((double)(std::max(b, a + 1) - a) * 1e-6); };
+        scan_ms += ms(w[VQ_CLK_SCAN], w[VQ_CLK_SCAN_END]);
+        kernel_ms += ms(w[from_build ? VQ_CLK_BUILD : begin], w[VQ_CLK_END]);
+        from_build = false;
+    }
 };
+
+static unsigned long long* run_clock(Plan& p) {
+    p.d_clk.ensure(VQ_CLK_WORDS * 8);
+    return p.d_clk.as<unsigned long long>();
+}
 
 std::shared_ptr<OutBlock> OutPool::acquire(size_t bytes, bool& lend) {
     auto fit = [&](OutBlock& b) {
@@ -809,6 +847,7 @@ struct RegsPending {
     size_t nout_f = 0, nout_i = 0;
     bool mapped = false;
     int launches = 0;
+    bool stamped = false;  // times from the device clock, behind the error word
     bool lazy = false;  // an event after the copy back marks the run's end (other runs may follow on the stream)
 };
 
@@ -842,15 +881,15 @@ static RegsPending regs_launch(RunCtx& rc, VQParams& P, long long nchunks, bool 
     const int* d_kinds = p.d_kinds.as<int>();
     size_t nout_f = (size_t)G * nfb * 8, nout_i = (size_t)G * (ni + 1) * 8;
     // layout: merged floats, merged ints, the error word handed out (copied
-    // back with the results), then the error word the kernels raise
+    // back with the results), the error word the kernels raise, the clock's stamps
     const size_t before = p.scratch_c.n;
-    p.scratch_c.ensure(nout_f + nout_i + 16);
+    p.scratch_c.ensure(nout_f + nout_i + 48);
     if (p.scratch_c.n != before) p.regs_err_clean = false;
     double* out_f = p.scratch_c.as<double>();
     long long* out_i = (long long*)((char*)p.scratch_c.p + nout_f);
     int* err_out = (int*)((char*)p.scratch_c.p + nout_f + nout_i);
     P.error = err_out + 2;
-    p.h_stage.ensure(nout_f + nout_i + 16);
+    p.h_stage.ensure(nout_f + nout_i + 48);
     // the merge writes the merged row and the handed-out error word straight
     // into the pinned staging buffer when the device can address it, so no
     // copy follows the merge (the kernels' own error word stays on the device)
@@ -868,6 +907,9 @@ static RegsPending regs_launch(RunCtx& rc, VQParams& P, long long nchunks, bool 
         out_i = (long long*)((char*)mapped + nout_f);
         err_out = (int*)((char*)mapped + nout_f + nout_i);
     }
+    const bool stamped = rc.stamped();
+    P.clk = stamped ? run_clock(p) : nullptr;
+    P.clk_out = (unsigned long long*)err_out + 2;
     ensure_events(p);
     if (!p.regs_err_clean) VQ_CUDA(cudaMemsetAsync(P.error, 0, 4, rc.s));
     p.regs_err_clean = false;  // until the merge below has run
@@ -916,12 +958,17 @@ static RegsPending regs_launch(RunCtx& rc, VQParams& P, long long nchunks, bool 
         P.mdone = p.mdone.as<unsigned>();
     }
     bind_distinct(p, P, nchunks * 128, rc.s);
-    // the run's launches: start event, scan, merge, end event (events recorded
-    // as external nodes when captured, so a replayed graph still times them;
-    // plain records when launched directly, where the external flag is refused)
+    // the run's launches: the scan, which stamps the device clock; or a start
+    // event, the scan, its merge and an end event (recorded as external nodes
+    // when captured, so a replayed graph still times them; plain records when
+    // launched directly, where the external flag is refused)
     auto launch_all = [&](bool checks) {
-        if (checks) VQ_CUDA(cudaEventRecord(p.ev[0], rc.s));
-        else VQ_CUDA(cudaEventRecordWithFlags(p.ev[0], rc.s, cudaEventRecordExternal));
+        auto mark = [&](cudaEvent_t e) {
+            if (stamped) return;
+            if (checks) VQ_CUDA(cudaEventRecord(e, rc.s));
+            else VQ_CUDA(cudaEventRecordWithFlags(e, rc.s, cudaEventRecordExternal));
+        };
+        mark(p.ev[0]);
         jit_launch(K, grid, &P, sizeof P, rc.s);
         if (checks) launch_check(rc.s, "p.k_main");
         // no event between the scan and its merge: an event record there stops the
@@ -941,8 +988,7 @@ static RegsPending regs_launch(RunCtx& rc, VQParams& P, long long nchunks, bool 
                                        ni, d_kinds, d_kinds + nfb, out_f, out_i, P.error, err_out));
             if (checks) launch_check(rc.s, "k_merge_regs_dep");
         }
-        if (checks) VQ_CUDA(cudaEventRecord(p.ev[2], rc.s));
-        else VQ_CUDA(cudaEventRecordWithFlags(p.ev[2], rc.s, cudaEventRecordExternal));
+        mark(p.ev[2]);
     };
     // replayed as one CUDA graph while the parameter block and launch shape
     // are those it was captured with: one host call a run instead of four
@@ -991,13 +1037,14 @@ static RegsPending regs_launch(RunCtx& rc, VQParams& P, long long nchunks, bool 
             launch_all(true);
         }
     }
-    if (!mapped) VQ_CUDA(cudaMemcpyAsync(p.h_stage.p, p.scratch_c.p, nout_f + nout_i + 4, cudaMemcpyDeviceToHost, rc.s));
+    if (!mapped) VQ_CUDA(cudaMemcpyAsync(p.h_stage.p, p.scratch_c.p, nout_f + nout_i + 40, cudaMemcpyDeviceToHost, rc.s));
     if (lazy) VQ_CUDA(cudaEventRecord(p.ev[3], rc.s));
     RegsPending q;
     q.nout_f = nout_f;
     q.nout_i = nout_i;
     q.mapped = mapped != nullptr;
     q.launches = fused || last ? 1 : 2;
+    q.stamped = stamped;
     q.lazy = lazy;
     return q;
 }
@@ -1012,9 +1059,18 @@ static Groups regs_collect(RunCtx& rc, const RegsPending& q) {
     else VQ_CUDA(cudaStreamSynchronize(rc.s));
     p.regs_err_clean = true;
     check_regs_flags(*(const int*)((const char*)p.h_stage.p + nout_f + nout_i));
-    const float span = elapsed(p.ev[0], p.ev[2]);  // the scan and the merge (overlapping its drain, or inside it)
-    rc.scan_ms += span;
-    rc.kernel_ms += span;
+    if (q.stamped) {
+        const unsigned long long* c = (const unsigned long long*)((const char*)p.h_stage.p + nout_f + nout_i) + 2;
+        unsigned long long w[VQ_CLK_WORDS] = {};
+        w[VQ_CLK_BUILD] = c[0];
+        w[VQ_CLK_SCAN] = c[1];
+        w[VQ_CLK_SCAN_END] = w[VQ_CLK_END] = c[2];
+        rc.add_clock(w, VQ_CLK_SCAN);
+    } else {
+        const float span = elapsed(p.ev[0], p.ev[2]);  // the scan and the merge overlapping its drain
+        rc.scan_ms += span;
+        rc.kernel_ms += span;
+    }
     rc.launches += q.launches;
     const double* hf = (const double*)p.h_stage.p;
     const long long* hi = (const long long*)((const char*)p.h_stage.p + nout_f);
@@ -1060,7 +1116,8 @@ struct Compacted {
 // Writes the run's result columns from the group table in P (assemble.cu) and
 // waits for them. Returns null, with the error word, when the kernels raised
 // one or no pinned block is addressable (*ok false).
-static vexq_result_s* run_assemble(RunCtx& rc, const VQParams& P, long long nslots, const int* d_lsb, int* herr, bool* ok) {
+static vexq_result_s* run_assemble(RunCtx& rc, const VQParams& P, long long nslots, const int* d_lsb, int* herr, bool* ok,
+                                   unsigned long long* clk) {
     Plan& p = rc.p;
     *ok = true;
     // rows the block holds: every slot of a small table, else a quarter more
@@ -1095,6 +1152,7 @@ static vexq_result_s* run_assemble(RunCtx& rc, const VQParams& P, long long nslo
         d.special = P.special;
         d.fx_lsb = d_lsb;
         d.error = P.error;
+        d.clk = P.clk;
         d.cols = (const VQAsmCol*)(p.d_asm.as<char>() + at);
         d.nslots = nslots;
         d.ncols = (int)L.cols.size();
@@ -1114,9 +1172,10 @@ static vexq_result_s* run_assemble(RunCtx& rc, const VQParams& P, long long nslo
             launch_check(rc.s, "k_asm_write");
             rc.launches++;
         }
-        VQ_CUDA(cudaEventRecord(p.ev[3], rc.s));
+        if (!P.clk) VQ_CUDA(cudaEventRecord(p.ev[3], rc.s));
         VQ_CUDA(cudaStreamSynchronize(rc.s));
         const VQAsmHdr* h = (const VQAsmHdr*)blk->pin.p;
+        std::memcpy(clk, h->clk, sizeof h->clk);
         *herr = h->err;
         if (h->err) return nullptr;
         p.asm_rows_seen = (long long)h->n;
@@ -1142,10 +1201,10 @@ static void compact_table(RunCtx& rc, Compacted& c) {
     c.fval = (double*)(ob + 16 + cap_out * 16 + (size_t)ni * cap_out * 8);
     const int fg = (int)std::min<long long>((nslots + 255) / 256, (long long)sm_count() * 16);
     k_finalize<<<fg, 256, 0, rc.s>>>(c.t_keys, P.first, P.acc_i, P.acc_fx, P.special, nslots, ni, nf, c.d_lsb, c.keyed, c.n_dev, c.key,
-                                     c.first, c.ival, c.fval, cap_out);
+                                     c.first, c.ival, c.fval, cap_out, P.clk);
     launch_check(rc.s, "k_finalize");
     VQ_CUDA(cudaGetLastError());
-    VQ_CUDA(cudaEventRecord(p.ev[3], rc.s));
+    if (!P.clk) VQ_CUDA(cudaEventRecord(p.ev[3], rc.s));
 }
 
 // A deferred run (defer set) launches the scan and returns without waiting or
@@ -1214,26 +1273,35 @@ Compacted run_atomic(RunCtx& rc, VQParams& P, long long nchunks, long long estim
         }
         const long long* d_iv = p.d_tinit.as<long long>();
         const int* d_lsb = (const int*)(p.d_tinit.as<char>() + iv.size() * 8);
-        VQ_CUDA(cudaEventRecord(p.ev[0], rc.s));
+        P.clk = rc.stamped() ? run_clock(p) : nullptr;
+        auto mark = [&](cudaEvent_t e) {
+            if (!P.clk) VQ_CUDA(cudaEventRecord(e, rc.s));
+        };
+        mark(p.ev[0]);
         int ig = (int)std::min<long long>((nslots + 255) / 256, (long long)sm_count() * 16);
         k_init_table<<<ig, 256, 0, rc.s>>>(P.keys, P.first, P.acc_i, ni, d_iv, P.acc_fx, P.special, nf, nslots, hash, P.ngroups,
-                                          P.error, n_out);
+                                          P.error, n_out, P.clk);
         launch_check(rc.s, "k_init_table");
         bind_distinct(p, P, nchunks * 128, rc.s);
         VQ_CUDA(cudaGetLastError());
         const JitKernel& K = rc.k ? *rc.k : p.k_main;
         int grid = rc.k ? rc.grid : grid_for(p.k_main, nchunks, p.staged);
-        VQ_CUDA(cudaEventRecord(p.ev[1], rc.s));
+        mark(p.ev[1]);
         jit_launch(K, grid, &P, sizeof P, rc.s);
         launch_check(rc.s, "p.k_main");
-        VQ_CUDA(cudaEventRecord(p.ev[2], rc.s));
+        mark(p.ev[2]);
+        auto add_times = [&](const unsigned long long* w) {
+            if (P.clk) return rc.add_clock(w, VQ_CLK_BEGIN);
+            rc.scan_ms += elapsed(p.ev[1], p.ev[2]);
+            rc.kernel_ms += elapsed(p.ev[0], p.ev[3]);
+        };
+        unsigned long long clk[VQ_CLK_WORDS] = {};
         if (assemble && asm_run_ok(p, nslots, rc.row0, rc.row1)) {
             int herr = 0;
             bool ok = true;
-            c.done = run_assemble(rc, P, nslots, d_lsb, &herr, &ok);
+            c.done = run_assemble(rc, P, nslots, d_lsb, &herr, &ok, clk);
             if (ok) {
-                rc.scan_ms += elapsed(p.ev[1], p.ev[2]);
-                rc.kernel_ms += elapsed(p.ev[0], p.ev[3]);
+                add_times(clk);
                 rc.launches += 2;
                 if (c.done) {
                     if (hash) {
@@ -1262,12 +1330,12 @@ Compacted run_atomic(RunCtx& rc, VQParams& P, long long nchunks, long long estim
             return c;
         }
         compact_table(rc, c);
-        p.h_stage.ensure(32);
+        p.h_stage.ensure(16 + sizeof clk);
         VQ_CUDA(cudaMemcpyAsync(p.h_stage.p, n_out, 8, cudaMemcpyDeviceToHost, rc.s));
         VQ_CUDA(cudaMemcpyAsync((char*)p.h_stage.p + 8, P.error, 4, cudaMemcpyDeviceToHost, rc.s));
+        if (P.clk) VQ_CUDA(cudaMemcpyAsync((char*)p.h_stage.p + 16, P.clk, sizeof clk, cudaMemcpyDeviceToHost, rc.s));
         VQ_CUDA(cudaStreamSynchronize(rc.s));
-        rc.scan_ms += elapsed(p.ev[1], p.ev[2]);
-        rc.kernel_ms += elapsed(p.ev[0], p.ev[3]);
+        add_times((const unsigned long long*)((const char*)p.h_stage.p + 16));
         rc.launches += 3;
         unsigned long long nn = *(unsigned long long*)p.h_stage.p;
         int herr = *(int*)((char*)p.h_stage.p + 8);
@@ -1383,7 +1451,7 @@ int topk_groups(RunCtx& rc, Compacted& c, Groups& g) {
     long long R = 1024;
     while (R < 2 * p.topk_seen && R < kCap) R <<= 1;
     p.scratch_d.ensure(b_max + 32 + (size_t)(kCap - R) * w * 8);
-    p.h_stage.ensure(32 + (size_t)R * w * 8);
+    p.h_stage.ensure(kTopHead * 8 + (size_t)R * w * 8);
     void* mapped = nullptr;
     if (cudaHostGetDevicePointer(&mapped, p.h_stage.p, 0) != cudaSuccess) fail(VEXQ_EDEVICE, "pinned host memory has no device address");
     VQTop t;
@@ -1417,6 +1485,7 @@ int topk_groups(RunCtx& rc, Compacted& c, Groups& g) {
         t.fx_lsb = c.d_lsb;
         t.hash = c.keyed;
         t.error = c.P->error;
+        t.clk = c.P->clk;
     } else {
         t.keys = c.key;
         t.first = c.first;
@@ -1434,12 +1503,16 @@ int topk_groups(RunCtx& rc, Compacted& c, Groups& g) {
     launch_check(rc.s, "k_select");
     VQ_CUDA(cudaGetLastError());
     rc.launches += 2;
-    if (table) VQ_CUDA(cudaEventRecord(p.ev[3], rc.s));
+    if (table && !t.clk) VQ_CUDA(cudaEventRecord(p.ev[3], rc.s));
     VQ_CUDA(cudaStreamSynchronize(rc.s));
     const long long* hs = (const long long*)p.h_stage.p;
     if (table) {  // its time, count and error word
-        rc.scan_ms += elapsed(p.ev[1], p.ev[2]);
-        rc.kernel_ms += elapsed(p.ev[0], p.ev[3]);
+        if (t.clk) {
+            rc.add_clock((const unsigned long long*)hs + 3, VQ_CLK_BEGIN);
+        } else {
+            rc.scan_ms += elapsed(p.ev[1], p.ev[2]);
+            rc.kernel_ms += elapsed(p.ev[0], p.ev[3]);
+        }
         c.n = std::min<long long>(hs[0], c.cap_out);
         if (check_table_flags((int)hs[1], c.hash)) return -1;
         if (c.hash) {
@@ -1468,7 +1541,7 @@ int topk_groups(RunCtx& rc, Compacted& c, Groups& g) {
     g.first.resize(ns);
     g.ival.assign(p.ni, std::vector<int64_t>(ns));
     g.fval.assign(p.nf, std::vector<double>(ns));
-    const long long* head = hs + 4;
+    const long long* head = hs + kTopHead;
     for (long long j = 0; j < ns; j++) {
         const long long* r = j < R ? head + j * w : rest.data() + (j - R) * w;
         g.key[j] = (uint64_t)r[0];
@@ -2224,9 +2297,12 @@ vexq_result_s* run_plan(Plan& p, int rg_start, int rg_end) {
             B.error = (int*)(p.jt_scalar.as<char>() + 8);
             B.jtotal = (unsigned long long*)(p.jt_scalar.as<char>() + 24);
             ensure_events(p);
-            VQ_CUDA(cudaEventRecord(p.ev[4], rc.s));
-            VQ_CUDA(cudaMemsetAsync(p.jt_scalar.p, 0, 40, rc.s));
-            VQ_CUDA(cudaMemsetAsync(p.jt_dmap.p, 0, (size_t)drange * 8, rc.s));
+            const bool timed = !spec || !rc.stamped();  // by events: the host waits for the build, or nothing stamps the run's end
+            if (timed) VQ_CUDA(cudaEventRecord(p.ev[4], rc.s));
+            k_clear_dmap<<<(int)std::max<unsigned long long>(1, std::min<unsigned long long>((drange + 2047) / 2048, (unsigned long long)sm_count() * 8)),
+                           256, 0, rc.s>>>(p.jt_dmap.as<unsigned long long>(), (long long)drange, p.jt_scalar.as<unsigned long long>(), 5,
+                                           run_clock(p));
+            VQ_CUDA(cudaGetLastError());
             VQParams F = B;
             F.mode = 3;
             F.dmap = p.jt_dmap.as<unsigned long long>();
@@ -2241,7 +2317,8 @@ vexq_result_s* run_plan(Plan& p, int rg_start, int rg_end) {
             }
             rc.launches += 1;
             if (spec) {
-                VQ_CUDA(cudaEventRecord(p.ev[5], rc.s));
+                if (timed) VQ_CUDA(cudaEventRecord(p.ev[5], rc.s));
+                rc.from_build = !timed;
                 p.dmap_used = true;
                 join_keys = p.join_keys_seen;
                 break;
@@ -2542,7 +2619,7 @@ vexq_result_s* run_plan(Plan& p, int rg_start, int rg_end) {
             p.dmap_used = false;
             return run_plan(p, rg_start, rg_end);
         }
-        if (spec) r->kernel_ms += elapsed(p.ev[4], p.ev[5]);
+        if (spec && !rc.stamped()) r->kernel_ms += elapsed(p.ev[4], p.ev[5]);
     }
     r->rows_scanned = rows_scanned;
     r->bytes_scanned = bytes;
