@@ -52,7 +52,7 @@ __device__ __forceinline__ bool asm_value(const VQAsmDesc& d, const VQAsmCol& c,
         return true;
     }
     if (c.src == ASM_PACKED_KEY) {
-        const unsigned long long key = slot == d.nslots - 1 ? VQ_EMPTY_KEY : d.keys[slot];
+        const unsigned long long key = slot == d.nslots - 1 ? VQ_EMPTY_KEY : d.keys[slot * d.kst];
         const unsigned long long raw = (key >> c.shift) & (c.bits >= 64 ? ~0ull : ((1ull << c.bits) - 1));
         if (c.domain) {
             if (c.nullable && raw == c.domain - 1) return false;
@@ -136,7 +136,7 @@ k_assemble(const VQAsmDesc* descs, char* base, char* const* basep) {
     // the bitmap is clear: the last run left it so
     long long mine = -1;  // the first-row bit of the thread's first slot
     for (long long i = gtid; i < d.nslots; i += kAll) {
-        const long long cnt = d.acc_i[i], f = d.first[i];
+        const long long cnt = d.acc_i[i], f = d.first[i * d.kst];
         if (cnt == 0) continue;  // slot 0 of the integer bank is the row count
         const long long b = order_bit(d, f);
         atomicOr(d.bits + (b >> 5), 1u << (b & 31));
@@ -200,7 +200,7 @@ k_assemble(const VQAsmDesc* descs, char* base, char* const* basep) {
     const long long n = cta_base[kAsmCtas];
     for (long long i = gtid; i < d.nslots; i += kAll) {
         long long b = mine;
-        if (i != gtid) b = d.acc_i[i] != 0 ? order_bit(d, d.first[i]) : -1;
+        if (i != gtid) b = d.acc_i[i] != 0 ? order_bit(d, d.first[i * d.kst]) : -1;
         if (b < 0) continue;
         const int w = (int)(b >> 5);
         const uint4 q = __ldcg(reinterpret_cast<const uint4*>(d.bits + (w & ~3)));

@@ -46,6 +46,7 @@ struct VQAsmDesc {
     long long nslots, nwords, row0, phase_bits, cap_rows;
     long long out;          // offset of the header and columns from the output base
     int ncols;
+    int kst;                // words from a slot's key and first row to the next slot's
     int write;              // the cluster writes the columns too
 };
 struct VQAsmHdr {           // at the start of a table's output

@@ -212,8 +212,8 @@ struct Batch {
             } else {
                 const long long ns = it.nslots;
                 it.cache_n = it.hash || it.join ? 0 : dense_cache_groups(*it.p, cache_kb);
-                it.a_keys = it.hash ? take(ns * 8) : 0;
-                it.a_first = take(ns * 8);
+                it.a_keys = it.hash ? take(ns * 16) : 0;  // {key, first row} pairs
+                it.a_first = it.hash ? it.a_keys + 8 : take(ns * 8);
                 it.a_acc_i = take((size_t)it.ni * ns * 8);
                 it.a_acc_fx = take((size_t)it.nf * ns * 32);
                 it.a_special = take((size_t)it.nf * ns * 4);
@@ -346,6 +346,7 @@ struct Batch {
                 std::memset(&t, 0, sizeof t);
                 t.keys = P.keys;
                 t.first = P.first;
+                t.kst = it.hash ? 2 : 1;
                 t.acc_i = P.acc_i;
                 t.acc_fx = P.acc_fx;
                 t.special = P.special;
@@ -358,7 +359,6 @@ struct Batch {
                 if (it.gid) {  // keys come from the build's number → key array
                     t.keys = (unsigned long long*)(D + it.a_jgkey);
                     t.hash = 1;
-                    t.gid = 1;
                 }
                 t.n_out = (unsigned long long*)(O + it.o_nout);
                 t.ngroups = P.ngroups;
@@ -383,6 +383,7 @@ struct Batch {
                     asm_scratch(d, it.nslots, D + it.a_asm);
                     d.keys = P.keys;
                     d.first = P.first;
+                    d.kst = it.hash ? 2 : 1;
                     d.acc_i = P.acc_i;
                     d.acc_fx = P.acc_fx;
                     d.special = P.special;

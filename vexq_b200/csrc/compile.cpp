@@ -938,9 +938,12 @@ void choose_path(Plan& p) {
             if (!x.bounded) fail(VEXQ_ENOTSUP, "float sum over an unbounded expression (division by a range containing 0)");
             int e = 0;
             if (m > 0) std::frexp(m, &e);  // |x| <= m < 2^e
-            // values of magnitude ≥ 2^(e-45) keep every mantissa bit; the top 31
-            // bits of the 128-bit window hold sums of 2^31 rows
-            p.fx_lsb[p.slot_pos[s]] = e - 97;
+            // the window ends where the largest values do: those of the top 11
+            // binades lie in the two top digits (two atomics; three when the
+            // window ended one bit into a digit), the counters' upper halves
+            // hold the sums of 2^31 rows, and values of magnitude ≥ 2^(e-76)
+            // keep every mantissa bit (2^(e-45) in the block's group cache)
+            p.fx_lsb[p.slot_pos[s]] = e - VQ_FX_WINDOW;
         }
     }
 }
@@ -1513,11 +1516,11 @@ void emit_atomic_update(std::ostringstream& os, const Plan& p, const std::string
     } else if (p.path == AggPath::Dense) {
         os << ind << "const unsigned long long slot = key;\n";
     } else {
-        os << ind << "const unsigned long long slot = vq_insert(P.keys, P.cap_mask, P.cap, key, nullptr, P.error);\n";
+        os << ind << "const unsigned long long slot = vq_insert_first(P.keys, P.cap_mask, P.cap, key, " << order << ", P.error);\n";
         os << ind << "if (slot == VQ_NOSLOT) continue;\n";
     }
     os << ind << "const long long stride = (long long)P.cap + 1;\n";
-    os << ind << "atomicMin(&P.first[slot], " << order << ");\n";
+    if (gid_slot || p.path == AggPath::Dense) os << ind << "atomicMin(&P.first[slot], " << order << ");\n";
     for (size_t s = 0; s < p.slots.size(); s++) {
         std::string S = std::to_string(s);
         const Slot& sl = p.slots[s];
@@ -1664,10 +1667,11 @@ void emit_cache_norm(std::ostringstream& os, const Plan& p, int block, const std
 // One row's update of the global table's slot. Unguarded (fire-and-forget)
 // MIN/MAX and first-row atomics: a read of the current value to skip them
 // measured slower there (4M rows, 65,536 Zipf groups mostly uncached: 118.9
-// against 74.8 us; 200K hash keys: 201.6 against 197.7 us).
+// against 74.8 us). A hashed table's first row came with its key
+// (vq_insert_first).
 void emit_table_update(std::ostringstream& os, const Plan& p, const std::string& in, const std::string& order) {
     os << in << "const long long stride = (long long)P.cap + 1;\n";
-    os << in << "atomicMin(&P.first[slot], " << order << ");\n";
+    if (p.path == AggPath::Dense) os << in << "atomicMin(&P.first[slot], " << order << ");\n";
     for (size_t s = 0; s < p.slots.size(); s++) {
         const std::string S = std::to_string(s), SV = "sv" + S, pos = std::to_string(p.slot_pos[s]), iff = "if (sok" + S + ") ";
         const std::string ai = "P.acc_i[" + pos + " * stride + slot]", aiu = "(unsigned long long*)&" + ai;
@@ -1697,7 +1701,7 @@ void emit_group_update(std::ostringstream& os, const Plan& p, const std::string&
         // lanes leave the probe loop at different steps: the warp meets again
         // before the atomics
         os << ind << "unsigned long long slot = VQ_NOSLOT;\n";
-        os << ind << "if (live) slot = vq_insert(P.keys, P.cap_mask, P.cap, key, nullptr, P.error);\n";
+        os << ind << "if (live) slot = vq_insert_first(P.keys, P.cap_mask, P.cap, key, " << order << ", P.error);\n";
         os << ind << "__syncwarp();\n";
         os << ind << "if (slot != VQ_NOSLOT) {\n";
     }
@@ -2964,13 +2968,12 @@ static std::string gen_rjoin_kernel(Plan& p, const std::vector<int>& key_nodes, 
         os << "            const bool ok" << kn << " = true;\n";
         os << "            const " << ctype(kx.type) << " x" << kn << " = (" << ctype(kx.type) << ")(long long)sk[i];\n";
         emit_key(os, p, key_nodes, "            ");
-        if (p.path == AggPath::Dense) os << "            const unsigned long long slot = key;\n";
+        if (p.path == AggPath::Dense) os << "            const unsigned long long slot = key;\n            P.first[slot] = LF[i];\n";
         else {
-            os << "            const unsigned long long slot = vq_insert(P.keys, P.cap_mask, P.cap, key, nullptr, P.error);\n";
+            os << "            const unsigned long long slot = vq_insert_first(P.keys, P.cap_mask, P.cap, key, LF[i], P.error);\n";
             os << "            if (slot == VQ_NOSLOT) continue;\n";
         }
         os << "            const long long stride = (long long)P.cap + 1;\n";
-        os << "            P.first[slot] = LF[i];\n";
         for (int s = 0; s < p.ni; s++)
             os << "            P.acc_i[" << s << " * stride + slot] = LI[" << s << " * " << CAP << " + i];\n";
         for (int f = 0; f < p.nf; f++) {

@@ -97,7 +97,8 @@ __device__ __forceinline__ void vq_add64_as32(vq_i64* c, vq_i64 d) {
 // four signed 64-bit counters holding 32-bit digits (c[k] weighs 2^(32k+lsb)).
 // Integer addition is associative, so the sum is the same whatever order the
 // atomics land in. Bits of x below 2^lsb are truncated (the window is chosen
-// so that only values below 2^-45 of the largest possible |x| lose bits).
+// so that only values below 2^-45 (register path) or 2^-76 (group tables) of the
+// largest possible |x| lose bits).
 // Non-finite values set flags instead. stride is the distance between digits.
 template <bool kAtomic, bool kPair32 = false>
 __device__ __forceinline__ void vq_fx_add(vq_i64* c, double x, int lsb, unsigned* special, int* err) {
@@ -167,10 +168,10 @@ __device__ __forceinline__ void vq_s_add64(unsigned lo, unsigned hi, vq_u64 v) {
 
 // x as an integer multiple of 2^lsb: its 53-bit magnitude (mh, lo) and the
 // position sh of bit 0 above the window's LSB (the window's bound keeps |x|
-// below 2^(lsb + 97), so sh <= 44). Bits below 2^lsb are truncated. Returns
+// below 2^(lsb + kBits), so sh <= kBits - 53). Bits below 2^lsb are truncated. Returns
 // false where nothing is added: NaN and infinities, which set flags instead,
 // and values below the window. kFinite: x is never NaN or infinite.
-template <bool kFinite>
+template <bool kFinite, int kBits>
 __device__ __forceinline__ bool vq_fx_image(double x, int lsb, unsigned& mh, unsigned& lo, int& sh, unsigned& special, int* err) {
     const unsigned hi = (unsigned)__double2hiint(x);
     lo = (unsigned)__double2loint(x);
@@ -183,8 +184,8 @@ __device__ __forceinline__ bool vq_fx_image(double x, int lsb, unsigned& mh, uns
     }
     if (e) mh |= 0x100000u;
     sh = (e ? e : 1) - 1075 - lsb;
-    if ((unsigned)sh <= 44u) return true;
-    if (sh > 44) {  // outside the window's bound
+    if ((unsigned)sh <= (unsigned)(kBits - 53)) return true;
+    if (sh > kBits - 53) {  // outside the window's bound
         atomicOr(reinterpret_cast<unsigned*>(err), 2u);
         return false;
     }
@@ -206,16 +207,17 @@ __device__ __forceinline__ bool vq_fx_image(double x, int lsb, unsigned& mh, uns
 // until vq_s_limbs_norm. Unsigned limbs of 19 bits, or signed ones of 18 where
 // x may be negative, hold VQ_LIMB_ROWS rows between two normalisations.
 #define VQ_LIMBS 7
+#define VQ_LIMB_WINDOW 97  // bits of the limbs' window, which ends where the digits' does
 #define VQ_LIMB_ROWS 8191u
 template <bool kSigned> __device__ __forceinline__ constexpr int vq_limb_bits() { return kSigned ? 18 : 19; }
-template <bool kSigned> __device__ __forceinline__ constexpr int vq_limb_shift() { return 6 * vq_limb_bits<kSigned>() - 97; }
+template <bool kSigned> __device__ __forceinline__ constexpr int vq_limb_shift() { return 6 * vq_limb_bits<kSigned>() - VQ_LIMB_WINDOW; }
 template <bool kFinite, bool kSigned>
 __device__ __forceinline__ void vq_s_fx_add(unsigned a, unsigned s, double x, int lsb, int* err) {
     constexpr int W = vq_limb_bits<kSigned>(), kShift = vq_limb_shift<kSigned>();
     constexpr unsigned M = (1u << W) - 1u;
     unsigned mh, lo, special;
     int sh;
-    if (!vq_fx_image<kFinite>(x, lsb, mh, lo, sh, special, err)) {
+    if (!vq_fx_image<kFinite, VQ_LIMB_WINDOW>(x, lsb + (VQ_FX_WINDOW - VQ_LIMB_WINDOW), mh, lo, sh, special, err)) {
         if (!kFinite && special) vq_s_or(a + VQ_LIMBS * s, special);
         return;
     }
@@ -263,13 +265,10 @@ __device__ __forceinline__ void vq_s_limbs_flush(unsigned a, unsigned s, vq_i64*
             carry = v >> W;
             v &= (1 << W) - 1;
         }
-        // bits [W j - kShift, …) of the sum: values hold no bit below the LSB
-        const int at = W * j - kShift;
-        if (at < 0) {
-            d[0] += v >> -at;
-        } else {
-            d[at >> 5] += (vq_i64)((vq_u64)v << (at & 31));
-        }
+        // bits [W j - kShift, …) of the limbs' window; what is above the digits'
+        // window (the last limb, below 2^31) stays in the top digit
+        const int at = W * j - kShift + (VQ_FX_WINDOW - VQ_LIMB_WINDOW), k = at >> 5 < VQ_FX_DIGITS ? at >> 5 : VQ_FX_DIGITS - 1;
+        d[k] += (vq_i64)((vq_u64)v << (at - 32 * k));
     }
 #pragma unroll
     for (int k = 0; k < VQ_FX_DIGITS; k++)
@@ -282,7 +281,7 @@ template <bool kFinite, bool kSigned>
 __device__ __forceinline__ void vq_g_fx_add(vq_i64* c, unsigned* sp, double x, int lsb, int* err) {
     unsigned mh, lo, special;
     int sh;
-    if (!vq_fx_image<kFinite>(x, lsb, mh, lo, sh, special, err)) {
+    if (!vq_fx_image<kFinite, VQ_FX_WINDOW>(x, lsb, mh, lo, sh, special, err)) {
         if (!kFinite && special) atomicOr(sp, special);
         return;
     }
@@ -393,36 +392,48 @@ static __device__ __host__ __noinline__ double vq_fx_value_wide(const vq_i64* c,
     return neg ? -r : r;
 }
 
-// The same where the top counter leaves the sum below 2^127 units, as sums of up
-// to 2^30 rows do: two 64-bit words instead of four (a quarter of the
-// instructions; ranking 720K groups is bound by them).
+// The same for sums below 2^157 units, as sums of up to 2^28 rows are: the low
+// digit's 32 bits apart and two 64-bit words above them, instead of four words
+// (a quarter of the instructions; ranking 720K groups is bound by them).
 __device__ __host__ inline double vq_fx_value(const vq_i64* c, int lsb) {
-    if (c[3] < -0x20000000LL || c[3] > 0x20000000LL || c[2] < -0x2000000000000000LL || c[2] > 0x2000000000000000LL)
-        return vq_fx_value_wide(c, lsb);
-    // c0 + c1·2^32 + c2·2^64 + c3·2^96, each sign-extended to 128 bits
-    vq_u64 lo = (vq_u64)c[0], hi = c[0] < 0 ? ~0ull : 0ull;
-    const vq_u64 l1 = (vq_u64)c[1] << 32;
-    lo += l1;
-    hi += (vq_u64)(c[1] >> 32) + (lo < l1);
-    hi += (vq_u64)c[2] + ((vq_u64)c[3] << 32);
+    const vq_i64 big = 0x1000000000000000LL;
+    if (c[1] < -big || c[1] > big || c[2] < -big || c[2] > big || c[3] < -big || c[3] > big) return vq_fx_value_wide(c, lsb);
+    // low + 2^32·(c1 + carry + c2·2^32 + c3·2^64), the bracket in 128 bits
+    vq_u64 low = (vq_u64)c[0] << 32;  // c0's 32 bits, at the top of a word
+    const vq_i64 c1 = c[1] + (c[0] >> 32);
+    vq_u64 lo = (vq_u64)c1, hi = c1 < 0 ? ~0ull : 0ull;
+    const vq_u64 l2 = (vq_u64)c[2] << 32;
+    lo += l2;
+    hi += (vq_u64)(c[2] >> 32) + (lo < l2) + (vq_u64)c[3];
     const bool neg = hi >> 63;
     if (neg) {
-        lo = ~lo + 1ull;
-        hi = ~hi + (lo == 0ull);
+        low = 0ull - low;
+        lo = ~lo + (low == 0ull);
+        hi = ~hi + (lo == 0ull && low == 0ull);
     }
-    if (!(hi | lo)) return 0.0;
-    const int z = hi ? vq_clz64(hi) : 64 + vq_clz64(lo);  // leading zeros of 128
-    if (z >= 64) {
-        hi = lo << (z - 64);
-        lo = 0ull;
-    } else if (z) {
-        hi = (hi << z) | (lo >> (64 - z));
-        lo <<= z;
+    int z = 0;  // leading zeros of the three words
+    if (!hi) {
+        hi = lo;
+        lo = low;
+        low = 0ull;
+        z = 64;
+        if (!hi) {
+            hi = lo;
+            lo = 0ull;
+            z = 128;
+            if (!hi) return 0.0;
+        }
+    }
+    const int n = vq_clz64(hi);
+    if (n) {
+        hi = (hi << n) | (lo >> (64 - n));
+        lo = (lo << n) | (low >> (64 - n));
+        low <<= n;
     }
     // bit 63 of hi is the leading one: 53 bits, the guard bit, the rest
     vq_u64 mant = hi >> 11;
-    int exp2 = 64 - z + 11 + lsb;
-    const bool sticky = (hi & 0x3FFull) != 0 || lo != 0ull;
+    int exp2 = 96 - z - n + 11 + lsb;
+    const bool sticky = (hi & 0x3FFull) != 0 || lo != 0ull || low != 0ull;
     if (((hi >> 10) & 1ull) && (sticky || (mant & 1ull))) {
         mant++;
         if (mant >> 53) {
@@ -486,35 +497,43 @@ __device__ __forceinline__ bool vq_dset_insert(unsigned long long* keys, unsigne
 
 #define VQ_NOSLOT 0xFFFFFFFFFFFFFFFFull
 
-// Open-addressing insert (linear probing, atomicCAS on the key). The key equal
-// to the empty sentinel lives in the extra slot `cap`, whose key word is a
-// used-flag. Returns VQ_NOSLOT and raises err bit 0 when the probe limit is
-// reached, so a full table ends the kernel's work instead of spinning. New
-// keys are counted in *nkeys when it is not null (a block-local counter: one
-// global word taking an atomic per key serialises the whole insert).
-__device__ __forceinline__ vq_u64 vq_insert(vq_u64* keys, vq_u64 mask, vq_u64 cap, vq_u64 key,
-                                            vq_u64* nkeys, int* err) {
+// Open-addressing insert (linear probing) into a group table, whose entries are
+// {key, first-row key} pairs, of a row with order key `order`. The key equal to
+// the empty sentinel lives in the extra slot `cap`, whose key word is a used
+// flag. Returns VQ_NOSLOT and raises err bit 0 when the probe limit is reached,
+// so a full table ends the kernel's work instead of spinning.
+//
+// Group tables are bound by L2 atomics. One 16-byte read finds a key that is
+// there already together with its first row, so a row costs an atomic on neither
+// unless it is the key's first to arrive or comes before it: 4.0M rows, SUM and
+// COUNT, over 200,000 keys 148 -> 105 us, over 20,000 143 -> 92, over 500,000 (eight
+// rows a key) 145 -> 140; with separate arrays the extra read cost what it saved.
+__device__ __forceinline__ vq_u64 vq_insert_first(vq_u64* keys, vq_u64 mask, vq_u64 cap, vq_u64 key, vq_i64 order, int* err) {
     if (key == VQ_EMPTY_KEY) {
-        if (atomicCAS(keys + cap, 0ull, 1ull) == 0ull && nkeys) atomicAdd(nkeys, 1ull);
+        atomicCAS(keys + 2 * cap, 0ull, 1ull);
+        atomicMin(reinterpret_cast<long long*>(keys + 2 * cap + 1), (long long)order);
         return cap;
     }
     vq_u64 i = vq_hash(key) & mask;
     const vq_u64 limit = mask < (vq_u64)VQ_MAX_PROBES ? mask + 1 : (vq_u64)VQ_MAX_PROBES;
     for (vq_u64 n = 0; n < limit; n++) {
-        // one round trip: claim the slot or learn its key
-        vq_u64 old = atomicCAS(keys + i, VQ_EMPTY_KEY, key);
-        if (old == VQ_EMPTY_KEY) {
-            if (nkeys) atomicAdd(nkeys, 1ull);  // callers count in shared memory, not one global word
+        ulonglong2 e = __ldcg(reinterpret_cast<const ulonglong2*>(keys + 2 * i));
+        if (e.x == VQ_EMPTY_KEY) {
+            const vq_u64 old = atomicCAS(keys + 2 * i, VQ_EMPTY_KEY, key);
+            e.x = old == VQ_EMPTY_KEY ? key : old;
+        }
+        if (e.x == key) {
+            // (a first row read before another's minimum is only larger)
+            if ((long long)order < (long long)e.y) atomicMin(reinterpret_cast<long long*>(keys + 2 * i + 1), (long long)order);
             return i;
         }
-        if (old == key) return i;
         i = (i + 1) & mask;
     }
     atomicOr(err, 1);
     return VQ_NOSLOT;
 }
 
-// Insert that also reports whether this call claimed the key's slot.
+// Insert of a bare key that also reports whether this call claimed its slot.
 __device__ __forceinline__ vq_u64 vq_insert_fresh(vq_u64* keys, vq_u64 mask, vq_u64 cap, vq_u64 key, bool& fresh, int* err) {
     fresh = false;
     if (key == VQ_EMPTY_KEY) {

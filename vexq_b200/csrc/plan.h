@@ -409,7 +409,7 @@ struct VQTableDesc {           // one group table
     const int* fx_lsb;
     long long nslots;
     int ni, nf, hash;
-    int gid;                   // a join's build-key-numbered table: keys[] is the number → key array, not initialised
+    int kst;                   // words from a slot's key and first row to the next slot's (2: {key, first row} pairs)
     unsigned long long* n_out;
     unsigned long long* ngroups;
     int* error;

@@ -75,6 +75,14 @@ __device__ __forceinline__ void fill64(void* p, long long n, unsigned long long 
     if (tid == 0 && ((n - head) & 1)) q[n - 1] = v;
 }
 
+// The {key, first-row key} pairs of a hashed table; the last slot's key is the
+// used flag of the key equal to the empty sentinel.
+__device__ __forceinline__ void fill_pairs(unsigned long long* keys, long long nslots) {
+    ulonglong2* w = (ulonglong2*)keys;
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < nslots; i += (long long)gridDim.x * blockDim.x)
+        w[i] = make_ulonglong2(i == nslots - 1 ? 0ull : VQ_EMPTY_KEY, 0x7FFFFFFFFFFFFFFFull);
+}
+
 // Atomic path: every slot at its identities (keys empty, first-row keys max,
 // integer accumulators at their kind's identity, fixed-point digits and
 // special flags 0), and the run's counters and error word cleared. Bound by L2
@@ -91,10 +99,9 @@ __global__ void k_init_table(unsigned long long* keys, long long* first, long lo
         *ngroups = 0ull;
         *error = 0;
         n_out[0] = n_out[1] = n_out[2] = 0ull;  // groups, and the top-k's counters
-        if (hash) keys[nslots - 1] = 0ull;      // used flag of the key equal to the empty sentinel
     }
-    if (hash) fill64(keys, nslots - 1, VQ_EMPTY_KEY);
-    fill64(first, nslots, 0x7FFFFFFFFFFFFFFFull);
+    if (hash) fill_pairs(keys, nslots);
+    else fill64(first, nslots, 0x7FFFFFFFFFFFFFFFull);
     for (int s = 0; s < ni; s++) fill64(acc_i + (long long)s * nslots, nslots, (unsigned long long)init_i[s]);
     fill64(acc_fx, (long long)nf * nslots * 4, 0ull);
     const long long nsp = (long long)nf * nslots;  // 4-byte flags, from an 8-byte boundary
@@ -109,10 +116,10 @@ __device__ __forceinline__ void finalize_write(long long i, unsigned long long p
                                                const long long* first, const long long* acc_i, const long long* acc_fx,
                                                const unsigned* special, long long nslots, int ni, int nf,
                                                const int* fx_lsb, int hash, unsigned long long* o_key,
-                                               long long* o_first, long long* o_i, double* o_f, long long cap_out) {
+                                               long long* o_first, long long* o_i, double* o_f, long long cap_out, int kst) {
     if ((long long)pos >= cap_out) return;
-    o_key[pos] = hash ? (i == nslots - 1 ? VQ_EMPTY_KEY : keys[i]) : (unsigned long long)i;
-    o_first[pos] = first[i];
+    o_key[pos] = hash ? (i == nslots - 1 ? VQ_EMPTY_KEY : keys[i * kst]) : (unsigned long long)i;
+    o_first[pos] = first[i * kst];
     for (int s = 0; s < ni; s++) o_i[(long long)s * cap_out + pos] = acc_i[(long long)s * nslots + i];
     for (int f = 0; f < nf; f++) {
         o_f[(long long)f * cap_out + pos] =
@@ -160,14 +167,14 @@ __device__ __forceinline__ unsigned long long vq_claim_block(bool occ, unsigned 
 __global__ void k_finalize(const unsigned long long* keys, const long long* first, const long long* acc_i,
                            const long long* acc_fx, const unsigned* special, long long nslots, int ni, int nf,
                            const int* fx_lsb, int hash, unsigned long long* n_out, unsigned long long* o_key,
-                           long long* o_first, long long* o_i, double* o_f, long long cap_out, unsigned long long* clk) {
+                           long long* o_first, long long* o_i, double* o_f, long long cap_out, int kst, unsigned long long* clk) {
     const long long stride = (long long)gridDim.x * blockDim.x;
     for (long long b0 = (long long)blockIdx.x * blockDim.x; b0 < nslots; b0 += stride) {  // block-uniform trip count
         const long long i = b0 + threadIdx.x;
         const bool occ = i < nslots && acc_i[i] != 0;  // slot 0 of the int bank is the row count
         const unsigned long long pos = vq_claim_block(occ, n_out);
         if (occ) finalize_write(i, pos, keys, first, acc_i, acc_fx, special, nslots, ni, nf, fx_lsb, hash, o_key, o_first,
-                                o_i, o_f, cap_out);
+                                o_i, o_f, cap_out, kst);
     }
     if (clk && threadIdx.x == 0) atomicMax(clk + VQ_CLK_END, vq_clock());
 }
@@ -187,8 +194,8 @@ __global__ void k_init_batch(const VQTableDesc* d, int n, long long total) {
     for (long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x; g < total; g += (long long)gridDim.x * blockDim.x) {
         const VQTableDesc& t = d[table_of(d, n, g)];
         const long long i = g - t.slot0;
-        if (t.hash && !t.gid) t.keys[i] = (i == t.nslots - 1) ? 0ull : VQ_EMPTY_KEY;
-        t.first[i] = 0x7FFFFFFFFFFFFFFFLL;
+        if (t.kst == 2) t.keys[2 * i] = (i == t.nslots - 1) ? 0ull : VQ_EMPTY_KEY;
+        t.first[i * t.kst] = 0x7FFFFFFFFFFFFFFFLL;
         for (int s = 0; s < t.ni; s++) t.acc_i[(long long)s * t.nslots + i] = t.init_i[s];
         for (int f = 0; f < t.nf; f++) {
             for (int k = 0; k < 4; k++) t.acc_fx[((long long)f * t.nslots + i) * 4 + k] = 0;
@@ -219,7 +226,7 @@ __global__ void k_finalize_batch(const VQTableDesc* d, int n, long long total) {
         if (occ) {
             const VQTableDesc& t = d[ti];
             finalize_write(g - t.slot0, pos, t.keys, t.first, t.acc_i, t.acc_fx, t.special, t.nslots, t.ni, t.nf,
-                           t.fx_lsb, t.hash, t.o_key, t.o_first, t.o_i, t.o_f, t.cap_out);
+                           t.fx_lsb, t.hash, t.o_key, t.o_first, t.o_i, t.o_f, t.cap_out, t.kst);
         }
     }
 }
@@ -434,6 +441,7 @@ struct VQTop {
     const unsigned long long* np;
     long long n, stride;           // slots (or the most groups); distance between banks
     int ni, nf, hash;              // hash: keys[] holds the keys (else the slot is the key)
+    int kst;                       // words from a slot's key and first row to the next slot's
     int kind, vbank, vpos, nnpos, fmin_key, desc, limit;
     unsigned long long* rank;      // [n] sort rank of every slot, 0 without a group
     unsigned long long* wmax;      // [parts] largest sort rank of every 32 slots, 0 without a group
@@ -621,8 +629,8 @@ __global__ void __launch_bounds__(1024) k_select(const __grid_constant__ VQTop t
                 long long* o = p < t.R ? t.host + kTopHead + p * w : t.rest + (p - t.R) * w;
                 for (int j = lane; j < w; j += 32) {
                     long long x;
-                    if (j == 0) x = (long long)(!t.hash ? (unsigned long long)i : !t.np && i == t.n - 1 ? VQ_EMPTY_KEY : t.keys[i]);
-                    else if (j == 1) x = t.first[i];
+                    if (j == 0) x = (long long)(!t.hash ? (unsigned long long)i : !t.np && i == t.n - 1 ? VQ_EMPTY_KEY : t.keys[i * t.kst]);
+                    else if (j == 1) x = t.first[i * t.kst];
                     else if (j < 2 + t.ni) x = t.ival[(long long)(j - 2) * t.stride + i];
                     else {
                         const int f = (j - 2 - t.ni) / 5, d = (j - 2 - t.ni) % 5;
@@ -1104,6 +1112,7 @@ struct Compacted {
     unsigned long long* n_dev = nullptr;  // the group count on the device (and two counters of the top-k)
     // deferred run: the table as the scan left it, not compacted yet
     const unsigned long long* t_keys = nullptr;
+    int kst = 1;               // words from a slot's key and first row to the next slot's
     const VQParams* P = nullptr;
     const int* d_lsb = nullptr;
     bool keyed = false;            // t_keys holds the groups' keys
@@ -1147,6 +1156,7 @@ static vexq_result_s* run_assemble(RunCtx& rc, const VQParams& P, long long nslo
         p.d_asm.ensure(bytes);
         d.keys = P.keys;
         d.first = P.first;
+        d.kst = P.keys ? 2 : 1;
         d.acc_i = P.acc_i;
         d.acc_fx = P.acc_fx;
         d.special = P.special;
@@ -1201,7 +1211,7 @@ static void compact_table(RunCtx& rc, Compacted& c) {
     c.fval = (double*)(ob + 16 + cap_out * 16 + (size_t)ni * cap_out * 8);
     const int fg = (int)std::min<long long>((nslots + 255) / 256, (long long)sm_count() * 16);
     k_finalize<<<fg, 256, 0, rc.s>>>(c.t_keys, P.first, P.acc_i, P.acc_fx, P.special, nslots, ni, nf, c.d_lsb, c.keyed, c.n_dev, c.key,
-                                     c.first, c.ival, c.fval, cap_out, P.clk);
+                                     c.first, c.ival, c.fval, cap_out, c.kst, P.clk);
     launch_check(rc.s, "k_finalize");
     VQ_CUDA(cudaGetLastError());
     if (!P.clk) VQ_CUDA(cudaEventRecord(p.ev[3], rc.s));
@@ -1249,7 +1259,7 @@ Compacted run_atomic(RunCtx& rc, VQParams& P, long long nchunks, long long estim
         p.scratch_a.ensure(tot);
         char* base = (char*)p.scratch_a.p;
         P.keys = hash ? (unsigned long long*)base : nullptr;
-        P.first = (long long*)(base + b_keys);
+        P.first = (long long*)(hash ? base + 8 : base);  // hashed tables: {key, first row} pairs
         P.acc_i = (long long*)(base + b_keys + b_first);
         P.acc_fx = (long long*)(base + b_keys + b_first + b_i);
         P.special = (unsigned*)(base + b_keys + b_first + b_i + b_fx);
@@ -1322,6 +1332,7 @@ Compacted run_atomic(RunCtx& rc, VQParams& P, long long nchunks, long long estim
         c.P = &P;
         c.d_lsb = d_lsb;
         c.keyed = hash || gid;
+        c.kst = hash ? 2 : 1;
         c.hash = hash;
         c.rows = rows;
         if (defer) {
@@ -1479,6 +1490,7 @@ int topk_groups(RunCtx& rc, Compacted& c, Groups& g) {
     if (table) {
         t.keys = c.t_keys;
         t.first = c.P->first;
+        t.kst = c.kst;
         t.ival = c.P->acc_i;
         t.fx = c.P->acc_fx;
         t.special = c.P->special;
@@ -1489,6 +1501,7 @@ int topk_groups(RunCtx& rc, Compacted& c, Groups& g) {
     } else {
         t.keys = c.key;
         t.first = c.first;
+        t.kst = 1;
         t.ival = c.ival;
         t.fval = c.fval;
         t.hash = 1;
