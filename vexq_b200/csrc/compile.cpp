@@ -1506,11 +1506,20 @@ void emit_regs_flush(std::ostringstream& os, const Plan& p, int block, const Flu
     if (fused) os << "    }\n";
 }
 
+// A converged warp's rows added to their slots' float sum s (vq_w_fx_add).
+void emit_warp_sum(std::ostringstream& os, const Plan& p, size_t s, const std::string& in, const std::string& flags, const std::string& on,
+                   const std::string& slot, const std::string& value) {
+    const std::string at = std::to_string(p.slot_pos[s]) + " * ((long long)P.cap + 1)";
+    os << in << "vq_w_fx_add" << flags << "(" << on << ", " << slot << ", P.cap, P.acc_fx + " << at << " * 4, P.special + " << at << ", "
+       << value << ", P.fx_lsb[" << p.slot_pos[s] << "], P.error);\n";
+}
+
 // Atomic path: group table in global memory.
 // gid_slot: the global join probe's group number (vq_gid) is the slot; the
 // partitioned join, which has no build slots, inserts the packed key instead.
+// hoist: the float sums are left to the warp (vq_t, vq_v<slot>, vq_o<slot>, declared by the caller).
 void emit_atomic_update(std::ostringstream& os, const Plan& p, const std::string& ind, const std::string& order,
-                        bool gid_slot = false) {
+                        bool gid_slot = false, bool hoist = false) {
     if (gid_slot) {
         os << ind << "const unsigned long long slot = vq_gid;\n";
     } else if (p.path == AggPath::Dense) {
@@ -1536,6 +1545,10 @@ void emit_atomic_update(std::ostringstream& os, const Plan& p, const std::string
             case S_FMIN: os << ind << "if (sok" << S << " && !isnan(sv" << S << ")) atomicMin(" << aiu << ", vq_fkey(sv" << S << "));\n"; break;
             case S_FMAX: os << ind << "if (sok" << S << " && !isnan(sv" << S << ")) atomicMax(" << aiu << ", vq_fkey(sv" << S << "));\n"; break;
             case S_FSUM:
+                if (hoist) {
+                    os << ind << "vq_t = slot; vq_v" << S << " = sv" << S << "; vq_o" << S << " = sok" << S << ";\n";
+                    break;
+                }
                 os << ind << "if (sok" << S << ") vq_fx_add<true>(P.acc_fx + ((long long)" << pos << " * stride + (long long)slot) * 4, sv" << S
                    << ", P.fx_lsb[" << pos << "], P.special + (long long)" << pos << " * stride + slot, P.error);\n";
                 break;
@@ -1669,7 +1682,7 @@ void emit_cache_norm(std::ostringstream& os, const Plan& p, int block, const std
 // measured slower there (4M rows, 65,536 Zipf groups mostly uncached: 118.9
 // against 74.8 us). A hashed table's first row came with its key
 // (vq_insert_first).
-void emit_table_update(std::ostringstream& os, const Plan& p, const std::string& in, const std::string& order) {
+void emit_table_update(std::ostringstream& os, const Plan& p, const std::string& in, const std::string& order, bool sums = true) {
     os << in << "const long long stride = (long long)P.cap + 1;\n";
     if (p.path == AggPath::Dense) os << in << "atomicMin(&P.first[slot], " << order << ");\n";
     for (size_t s = 0; s < p.slots.size(); s++) {
@@ -1684,6 +1697,7 @@ void emit_table_update(std::ostringstream& os, const Plan& p, const std::string&
             case S_FMIN: os << in << "if (sok" << S << " && !isnan(" << SV << ")) atomicMin(" << aiu << ", vq_fkey(" << SV << "));\n"; break;
             case S_FMAX: os << in << "if (sok" << S << " && !isnan(" << SV << ")) atomicMax(" << aiu << ", vq_fkey(" << SV << "));\n"; break;
             case S_FSUM:
+                if (!sums) break;
                 os << in << iff << "vq_g_fx_add" << fx_flags(p, s) << "(P.acc_fx + ((long long)" << pos << " * stride + (long long)slot) * 4, P.special + (long long)"
                    << pos << " * stride + slot, " << SV << ", P.fx_lsb[" << pos << "], P.error);\n";
                 break;
@@ -2150,6 +2164,110 @@ static void emit_agg_rows(std::ostringstream& os, Plan& p, const std::vector<int
     os << "        }\n";
 }
 
+// The warp's queue of rows whose key was not in its home slot (up to 31 left
+// over and a chunk's 128) and whether a plan's scan kernel has it: it fits the
+// static shared memory for every warp of the block.
+constexpr int kHashQueue = 160;
+static bool hash_queue(const Plan& p, int block) { return p.path == AggPath::Hash && !p.is_join && (block / 32) * kHashQueue * 24 <= 46 * 1024; }
+static void emit_hash_queue_decl(std::ostringstream& os, int block) {
+    const std::string dim = "[" + std::to_string(block / 32) + "][" + std::to_string(kHashQueue) + "];\n";
+    os << "    __shared__ unsigned long long vq_qk" << dim << "    __shared__ unsigned long long vq_qi" << dim << "    __shared__ long long vq_qr" << dim;
+    os << "    const int vq_qw = threadIdx.x >> 5;\n    int vq_qn = 0;\n";
+    os << "    const unsigned long long vq_lim = min(P.cap_mask + 1ull, (unsigned long long)VQ_MAX_PROBES);\n";
+}
+
+// A converged warp's rows r in the slots found for them (hit, slot, the first
+// row vq_f0 read there).
+static void emit_hash_update(std::ostringstream& os, Plan& p, Gen& g, const std::string& ind) {
+    for (auto& s : p.slots) if (s.input >= 0) g.emit(s.input);
+    emit_slot_values(os, p, ind, "hit");
+    os << ind << "if (hit) {\n";
+    os << ind << "    const long long vq_o = " << order_expr(p, "r") << ";\n";
+    // (a first row read before another's minimum is only larger)
+    os << ind << "    if (vq_o < vq_f0) atomicMin(&P.first[2 * slot], vq_o);\n";
+    emit_table_update(os, p, ind + "    ", "vq_o", false);
+    os << ind << "}\n";
+    for (size_t s = 0; s < p.slots.size(); s++)
+        if (p.slots[s].kind == S_FSUM)
+            emit_warp_sum(os, p, s, ind, fx_flags(p, s), "hit && sok" + std::to_string(s), "slot", "sv" + std::to_string(s));
+}
+
+// Takes one queued row a lane: a step of its probe (claiming an empty slot), its
+// update if that found the slot, else back into the queue.
+static void emit_hash_take(std::ostringstream& os, Plan& p) {
+    os << "        __syncwarp();\n";
+    os << "        const int vq_m = min(vq_qn, 32);\n        vq_qn -= vq_m;\n";
+    os << "        const bool vq_in = lane < vq_m;\n";
+    os << "        const int vq_at = vq_qn + (vq_in ? lane : 0);\n";
+    os << "        const unsigned long long key = vq_in ? vq_qk[vq_qw][vq_at] : 0ull, vq_w = vq_in ? vq_qi[vq_qw][vq_at] : 0ull;\n";
+    os << "        const long long r = vq_in ? vq_qr[vq_qw][vq_at] : 0ll;\n";
+    os << "        unsigned long long slot = key == VQ_EMPTY_KEY ? P.cap : vq_w & 0xFFFFFFFFFFull, vq_n = vq_w >> 40;\n";
+    os << "        bool hit = false;\n        long long vq_f0 = 0ll;\n";
+    os << "        if (vq_in) {\n";
+    os << "            ulonglong2 e = __ldcg(reinterpret_cast<const ulonglong2*>(P.keys + 2 * slot));\n";
+    os << "            if (key == VQ_EMPTY_KEY) {  // its own slot, whose key word is a used flag\n";
+    os << "                if (e.x == 0ull) atomicCAS(P.keys + 2 * slot, 0ull, 1ull);\n";
+    os << "                e.x = key;\n";
+    os << "            } else if (e.x == VQ_EMPTY_KEY) {\n";
+    os << "                const unsigned long long old = atomicCAS(P.keys + 2 * slot, VQ_EMPTY_KEY, key);\n";
+    os << "                e.x = old == VQ_EMPTY_KEY ? key : old;\n            }\n";
+    os << "            hit = e.x == key;\n            vq_f0 = (long long)e.y;\n";
+    os << "            if (!hit && ++vq_n >= vq_lim) atomicOr(P.error, 1);\n        }\n";
+    os << "        __syncwarp();\n";
+    os << "        const bool vq_again = vq_in && !hit && vq_n < vq_lim;\n";
+    os << "        const unsigned vq_b = __ballot_sync(0xffffffffu, vq_again);\n";
+    os << "        if (vq_again) {\n";
+    os << "            const int at = vq_qn + __popc(vq_b & ((1u << lane) - 1u));\n";
+    os << "            vq_qk[vq_qw][at] = key;\n            vq_qi[vq_qw][at] = ((slot + 1) & P.cap_mask) | vq_n << 40;\n            vq_qr[vq_qw][at] = r;\n";
+    os << "        }\n        vq_qn += __popc(vq_b);\n";
+    Gen g(p, os);
+    g.gather = true;
+    g.ind = "        ";
+    emit_hash_update(os, p, g, "        ");
+}
+
+// One chunk of a hashed GROUP BY (a lane's four rows, loaded). A first pass runs
+// the filter and the key and issues the four loads of the home slots; rows whose
+// key is there are folded where they lie, the others go into the warp's queue and
+// probe on 32 at a time. Probed in place, a warp waited for the longest of 32
+// chains in every row (15 of 32 lanes at work). With the sums added together
+// (vq_w_fx_add), 4.0M rows, SUM and COUNT, over 200,000 keys 105 -> 86 us, over
+// 20,000 92 -> 74, over 500,000 140 -> 112; either alone gained nothing (106 with
+// the four loads ahead, 118 with the sums added together).
+static void emit_hash_rows(std::ostringstream& os, Plan& p, const std::vector<int>& key_nodes) {
+    os << "        const int vq_lo = (int)max(min(s0 - r0, 128LL), -128LL), vq_hi = (int)max(min(s1 - r0, 128LL), -128LL);\n";
+    os << "        unsigned long long vq_k[4], vq_i[4]; ulonglong2 vq_e[4]; bool vq_on[4];\n";
+    os << "#pragma unroll\n        for (int k = 0; k < 4; k++) {\n";
+    os << "            bool live = k >= vq_lo && k < vq_hi;\n";
+    {
+        Gen g0(p, os);
+        if (p.pred >= 0) {
+            g0.emit(p.pred);
+            os << "            live = live && x" << p.pred << " && ok" << p.pred << ";\n";
+        }
+        for (int k : key_nodes) g0.emit(k);
+        emit_key(os, p, key_nodes, "            ");
+    }
+    os << "            vq_on[k] = live;\n            vq_k[k] = key;\n            vq_i[k] = vq_hash(key) & P.cap_mask;\n";
+    os << "            vq_e[k] = live ? __ldcg(reinterpret_cast<const ulonglong2*>(P.keys + 2 * vq_i[k])) : make_ulonglong2(0ull, 0ull);\n";
+    os << "        }\n";
+    os << "#pragma unroll\n        for (int k = 0; k < 4; k++) {\n";
+    os << "            const long long r = r0 + k;\n";
+    os << "            const bool hit = vq_on[k] && vq_e[k].x == vq_k[k] && vq_k[k] != VQ_EMPTY_KEY;\n";
+    os << "            const unsigned long long key = vq_k[k], slot = vq_i[k];\n            const long long vq_f0 = (long long)vq_e[k].y;\n";
+    os << "            const unsigned vq_b = __ballot_sync(0xffffffffu, vq_on[k] && !hit);\n";
+    os << "            if (vq_on[k] && !hit) {\n";
+    os << "                const int at = vq_qn + __popc(vq_b & ((1u << lane) - 1u));\n";
+    os << "                vq_qk[vq_qw][at] = vq_k[k];\n                vq_qi[vq_qw][at] = slot;\n                vq_qr[vq_qw][at] = r;\n";
+    os << "            }\n            vq_qn += __popc(vq_b);\n";
+    Gen g(p, os);
+    emit_hash_update(os, p, g, "            ");
+    os << "        }\n";
+    os << "        while (vq_qn >= 32) {\n";
+    emit_hash_take(os, p);
+    os << "        }\n";
+}
+
 // Generates the aggregate scan kernel (table → filter → project → aggregate).
 static std::string gen_agg_kernel(Plan& p, const std::vector<int>& key_nodes, int block) {
     std::ostringstream os;
@@ -2166,10 +2284,18 @@ static std::string gen_agg_kernel(Plan& p, const std::vector<int>& key_nodes, in
     emit_clock_start(os);
     if (p.path == AggPath::Regs) emit_regs_decl(os, p);
     if (p.smem_groups > 0) emit_cache_init(os, p);
+    if (hash_queue(p, block)) emit_hash_queue_decl(os, block);
     loop.block_steps = p.smem_groups > 0;
     loop.open(os);
-    emit_agg_rows(os, p, key_nodes, p.smem_groups > 0, loop.strided());
+    const bool queue = hash_queue(p, block);
+    if (queue) emit_hash_rows(os, p, key_nodes);
+    else emit_agg_rows(os, p, key_nodes, p.smem_groups > 0, loop.strided());
     loop.close(os);
+    if (queue) {
+        os << "    while (vq_qn > 0) {\n";
+        emit_hash_take(os, p);
+        os << "    }\n";
+    }
     if (loop.block_steps) {
         emit_cache_norm(os, p, block, "vq_step");
         os << "    }\n";
@@ -2577,30 +2703,50 @@ static std::string gen_build_kernel(Plan& p, int key_node, int block) {
 // keeps: 2% 63 -> 44 us, 20% 84 -> 59, 50% 90 -> 75, 60% 90 -> 88, 100% 92 -> 98
 // (the per-chunk count); the line is drawn at 5/8, where queueing costs as much
 // as it saves. Without a filter on the probe side most keys of a foreign key
-// match, and the kernel has no queue. Group tables have none either: their
-// atomics, not the lanes, bound the probe (26% kept, 76 us with or without).
+// match, and the kernel has no queue.
+//
+// A group table's probe is bound by its L2 atomics. With float sums, every match
+// goes through the queue, so that a full warp adds them together (vq_w_fx_add):
+// 6.0M rows without a filter, grouped by the join key 176 -> 155 us, by a date
+// 230 -> 194; 26% kept 69 -> 66 (four blocks an SM, 70 with the three that the
+// compiler's 74 registers leave; folding together in place 92, at 92 registers).
 constexpr int kProbeQueue = 160;  // up to 31 left over and a chunk's 128
 constexpr int kQueueDense = 80;
 
 static bool probe_queue(const Plan& p, int block) {
-    const size_t queue = (size_t)(block / 32) * kProbeQueue * 16;
-    return p.path == AggPath::Regs && p.pred >= 0 && queue + regs_flush_smem(p, block) <= 46 * 1024;
+    const size_t queue = (size_t)(block / 32) * kProbeQueue * (p.join_gid ? 20 : 16);
+    if (p.path != AggPath::Regs) return p.nf > 0 && queue <= 46 * 1024;
+    return p.pred >= 0 && queue + regs_flush_smem(p, block) <= 46 * 1024;
 }
 
-void emit_probe_queue_decl(std::ostringstream& os, int block) {
+void emit_probe_queue_decl(std::ostringstream& os, const Plan& p, int block) {
     const int W = block / 32;
     os << "    __shared__ long long vq_qr[" << W << "][" << kProbeQueue << "];\n";
     os << "    __shared__ unsigned long long vq_qc[" << W << "][" << kProbeQueue << "];\n";
-    os << "    const int vq_qw = threadIdx.x >> 5;\n    int vq_qn = 0, vq_last = 0;\n";
+    if (p.join_gid) os << "    __shared__ unsigned vq_qg[" << W << "][" << kProbeQueue << "];\n";
+    os << "    const int vq_qw = threadIdx.x >> 5;\n    int vq_qn = 0" << (p.path == AggPath::Regs ? ", vq_last = 0" : "") << ";\n";
 }
 
 // What every match of a probe row r runs: the residual filter and the fold into
 // the aggregate, ordered by (probe row, chain position), from the row's chain word
-// jc (and, grouping by the join key, its group number vq_gid).
-static void emit_probe_matches(std::ostringstream& os, Plan& p, const std::vector<int>& key_nodes, const Gen& scope) {
+// jc (and, grouping by the join key, its group number vq_gid). on: the lane has a
+// row; on the group-table paths the warp goes through its rows' matches together
+// and adds the float sums together (vq_w_fx_add).
+static void emit_probe_matches(std::ostringstream& os, Plan& p, const std::vector<int>& key_nodes, const Gen& scope, const std::string& on) {
+    const bool table = p.path != AggPath::Regs && !on.empty();
     os << "            const int ja = (int)(unsigned)jc, jn = (int)(jc >> 32);\n";
     os << "            const int jb = jn < 0 ? 0 : ja, je = jn < 0 ? 1 : ja + jn;\n";
-    os << "            for (int ji = jb; ji < je; ji++) {\n";
+    if (table) {
+        os << "            const int vq_n = __reduce_max_sync(0xffffffffu, " << on << " ? je - jb : 0);\n";
+        os << "            for (int vq_j = 0; vq_j < vq_n; vq_j++) {\n";
+        os << "                const int ji = jb + vq_j;\n";
+        os << "                unsigned long long vq_t = 0ull;\n";
+        for (size_t s = 0; s < p.slots.size(); s++)
+            if (p.slots[s].kind == S_FSUM) os << "                double vq_v" << s << " = 0.0; bool vq_o" << s << " = false;\n";
+        os << "                if (" << on << " && ji < je) do {\n";
+    } else {
+        os << "            for (int ji = jb; ji < je; ji++) {\n";
+    }
     os << "                const long long brow = jn < 0 ? (long long)ja : (long long)P.jrows[ji];\n";
     // above-join expressions: a fresh memo scope per match for build-side reads
     Gen g2(p, os);
@@ -2617,23 +2763,36 @@ static void emit_probe_matches(std::ostringstream& os, Plan& p, const std::vecto
     emit_key(os, p, key_nodes, "                ");
     emit_slot_values(os, p, "                ");
     std::string order = order_expr(p, "((r << 16) | (long long)min(ji - jb, 65535))");
-    if (p.path == AggPath::Regs) emit_regs_update(os, p, "                ", order);
-    else emit_atomic_update(os, p, "                ", order, p.join_gid);
+    if (!table) {
+        if (p.path == AggPath::Regs) emit_regs_update(os, p, "                ", order);
+        else emit_atomic_update(os, p, "                ", order, p.join_gid);
+        os << "            }\n";
+        return;
+    }
+    emit_atomic_update(os, p, "                ", order, p.join_gid, true);
+    os << "                } while (false);\n";
+    for (size_t s = 0; s < p.slots.size(); s++)
+        if (p.slots[s].kind == S_FSUM)
+            emit_warp_sum(os, p, s, "                ", "<false, true>", "vq_o" + std::to_string(s), "vq_t", "vq_v" + std::to_string(s));
     os << "            }\n";
 }
 
 // Takes one queued row a lane (the last 32, or the vq_qn < 32 that are left) and
 // runs its matches; the probe columns above the join are read again at the row.
 static void emit_probe_take(std::ostringstream& os, Plan& p, const std::vector<int>& key_nodes, bool rest) {
+    const bool table = p.path != AggPath::Regs;
     os << "        __syncwarp();\n";
     if (!rest) os << "        vq_qn -= 32;\n";
     os << "        const int vq_at = " << (rest ? "lane" : "vq_qn + lane") << ";\n";
-    os << "        " << (rest ? "if (lane < vq_qn) {\n" : "{\n");
-    os << "            const long long r = vq_qr[vq_qw][vq_at];\n";
-    os << "            const unsigned long long jc = vq_qc[vq_qw][vq_at];\n";
+    if (rest && table) os << "        const bool vq_in = lane < vq_qn;\n";
+    os << "        " << (rest && !table ? "if (lane < vq_qn) {\n" : "{\n");
+    const std::string in = rest && table ? "vq_in ? " : "", z = rest && table ? " : 0" : "";
+    os << "            const long long r = " << in << "vq_qr[vq_qw][vq_at]" << z << ";\n";
+    os << "            const unsigned long long jc = " << in << "vq_qc[vq_qw][vq_at]" << z << ";\n";
+    if (p.join_gid) os << "            const unsigned long long vq_gid = " << in << "vq_qg[vq_qw][vq_at]" << z << ";\n";
     Gen g(p, os);
     g.gather = true;
-    emit_probe_matches(os, p, key_nodes, g);
+    emit_probe_matches(os, p, key_nodes, g, !table ? "" : rest ? "vq_in" : "true");
     os << "        }\n        __syncwarp();\n";
 }
 
@@ -2673,7 +2832,7 @@ static void emit_probe_rows(std::ostringstream& os, Plan& p, const std::vector<i
         os << "            vq_on[k] = true;\n";
     }
     os << "        }\n";
-    if (queue) os << "        if (vq_last >= " << kQueueDense << ") {\n";
+    if (queue && p.path == AggPath::Regs) os << "        if (vq_last >= " << kQueueDense << ") {\n";
     os << "#pragma unroll\n        for (int k = 0; k < 4; k++) {\n";
     os << "            const long long r = " << rk << ";\n";
     Gen g(p, os);
@@ -2696,19 +2855,22 @@ static void emit_probe_rows(std::ostringstream& os, Plan& p, const std::vector<i
     if (!queue) {
         os << "            if (!vq_on[k]) continue;\n" << decl;
         resolve("continue;");
-        emit_probe_matches(os, p, key_nodes, g);
+        emit_probe_matches(os, p, key_nodes, g, "");
         os << "        }\n";
         return;
     }
-    os << "            if (!vq_on[k]) continue;\n" << decl;
-    resolve("{ vq_on[k] = false; continue; }");
-    emit_probe_matches(os, p, key_nodes, g);
-    os << "        }\n";
-    os << "        vq_last = 0;\n";
-    os << "#pragma unroll\n        for (int k = 0; k < 4; k++) vq_last += __popc(__ballot_sync(0xffffffffu, vq_on[k]));\n";
-    os << "        } else {\n        vq_last = 0;\n";
-    os << "#pragma unroll\n        for (int k = 0; k < 4; k++) {\n";
-    os << "            const long long r = " << rk << ";\n" << decl;
+    if (p.path == AggPath::Regs) {
+        os << "            if (!vq_on[k]) continue;\n" << decl;
+        resolve("{ vq_on[k] = false; continue; }");
+        emit_probe_matches(os, p, key_nodes, g, "");
+        os << "        }\n";
+        os << "        vq_last = 0;\n";
+        os << "#pragma unroll\n        for (int k = 0; k < 4; k++) vq_last += __popc(__ballot_sync(0xffffffffu, vq_on[k]));\n";
+        os << "        } else {\n        vq_last = 0;\n";
+        os << "#pragma unroll\n        for (int k = 0; k < 4; k++) {\n";
+        os << "            const long long r = " << rk << ";\n";
+    }
+    os << decl;
     std::fill(g.done.begin(), g.done.end(), 0);
     os << "            if (vq_on[k]) do {\n";
     resolve("{ vq_on[k] = false; break; }");
@@ -2717,10 +2879,11 @@ static void emit_probe_rows(std::ostringstream& os, Plan& p, const std::vector<i
     os << "            if (vq_on[k]) {\n";
     os << "                const int at = vq_qn + __popc(vq_b & ((1u << lane) - 1u));\n";
     os << "                vq_qr[vq_qw][at] = r;\n                vq_qc[vq_qw][at] = jc;\n";
-    os << "            }\n            vq_qn += __popc(vq_b);\n            vq_last += __popc(vq_b);\n        }\n";
+    if (p.join_gid) os << "                vq_qg[vq_qw][at] = (unsigned)vq_gid;\n";
+    os << "            }\n            vq_qn += __popc(vq_b);\n" << (p.path == AggPath::Regs ? "            vq_last += __popc(vq_b);\n" : "") << "        }\n";
     os << "        while (vq_qn >= 32) {\n";
     emit_probe_take(os, p, key_nodes, false);
-    os << "        }\n        }\n";
+    os << "        }\n" << (p.path == AggPath::Regs ? "        }\n" : "");
 }
 
 // Join probe kernel: probe rows pass the probe filter, look their key up, and
@@ -2739,7 +2902,8 @@ static std::string gen_probe_kernel(Plan& p, const std::vector<int>& key_nodes, 
     p.tile = loop.tile_rows();
     p.smem = loop.smem();
     loop.prologue(os);
-    os << kernel_head("vq_agg", block, p.min_blocks);
+    const bool queue = probe_queue(p, block);
+    os << kernel_head("vq_agg", block, p.min_blocks > 0 || !queue || p.path == AggPath::Regs ? p.min_blocks : 1024 / block);
     emit_clock_start(os);
     // a build the host did not wait for: its failure or emptiness is raised
     // in this kernel's error word, which comes back with the results
@@ -2750,8 +2914,7 @@ static std::string gen_probe_kernel(Plan& p, const std::vector<int>& key_nodes, 
     os << "        else if (*P.bnk == 0ull) atomicOr(P.error, 128);\n";
     os << "    }\n";
     if (p.path == AggPath::Regs) emit_regs_decl(os, p);
-    const bool queue = probe_queue(p, block);
-    if (queue) emit_probe_queue_decl(os, block);
+    if (queue) emit_probe_queue_decl(os, p, block);
     loop.open(os);
     emit_probe_rows(os, p, key_nodes, loop.strided(), queue);
     loop.close(os);
