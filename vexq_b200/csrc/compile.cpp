@@ -2712,19 +2712,27 @@ static std::string gen_build_kernel(Plan& p, int key_node, int block) {
 // compiler's 74 registers leave; folding together in place 92, at 92 registers).
 constexpr int kProbeQueue = 160;  // up to 31 left over and a chunk's 128
 constexpr int kQueueDense = 80;
+constexpr int kQueueSparse = 24;
+
+// Whether rows that pass the filter are queued before the lookup too
+// (emit_probe_rows).
+static bool probe_ahead(const Plan& p) { return p.path == AggPath::Regs && !p.staged && p.async_stages > 1; }
+
+static std::string queue_row(const Plan& p) { return probe_ahead(p) && p.t->nrows < (1ll << 32) ? "unsigned" : "long long"; }
 
 static bool probe_queue(const Plan& p, int block) {
-    const size_t queue = (size_t)(block / 32) * kProbeQueue * (p.join_gid ? 20 : 16);
-    if (p.path != AggPath::Regs) return p.nf > 0 && queue <= 46 * 1024;
-    return p.pred >= 0 && queue + regs_flush_smem(p, block) <= 46 * 1024;
+    const size_t row = p.t->nrows < (1ll << 32) ? 4 : 8, entries = (size_t)(block / 32) * kProbeQueue;
+    if (p.path != AggPath::Regs) return p.nf > 0 && entries * (row + 8 + (p.join_gid ? 4 : 0)) <= 46 * 1024;
+    return p.pred >= 0 && entries * (probe_ahead(p) ? 2 : 1) * (row + 8) + regs_flush_smem(p, block) <= 46 * 1024;
 }
 
 void emit_probe_queue_decl(std::ostringstream& os, const Plan& p, int block) {
-    const int W = block / 32;
-    os << "    __shared__ long long vq_qr[" << W << "][" << kProbeQueue << "];\n";
-    os << "    __shared__ unsigned long long vq_qc[" << W << "][" << kProbeQueue << "];\n";
-    if (p.join_gid) os << "    __shared__ unsigned vq_qg[" << W << "][" << kProbeQueue << "];\n";
-    os << "    const int vq_qw = threadIdx.x >> 5;\n    int vq_qn = 0" << (p.path == AggPath::Regs ? ", vq_last = 0" : "") << ";\n";
+    const std::string dim = "[" + std::to_string(block / 32) + "][" + std::to_string(kProbeQueue) + "];\n", row = "    __shared__ " + queue_row(p);
+    os << row << " vq_qr" << dim << "    __shared__ unsigned long long vq_qc" << dim;
+    if (p.join_gid) os << "    __shared__ unsigned vq_qg" << dim;
+    os << "    const int vq_qw = threadIdx.x >> 5;\n    int vq_qn = 0;\n";
+    if (p.path == AggPath::Regs) os << "    int vq_last = 0;\n";
+    if (probe_ahead(p)) os << row << " vq_fr" << dim << "    __shared__ unsigned long long vq_fk" << dim << "    int vq_fn = 0;\n";
 }
 
 // What every match of a probe row r runs: the residual filter and the fold into
@@ -2777,15 +2785,15 @@ static void emit_probe_matches(std::ostringstream& os, Plan& p, const std::vecto
     os << "            }\n";
 }
 
-// Takes one queued row a lane (the last 32, or the vq_qn < 32 that are left) and
-// runs its matches; the probe columns above the join are read again at the row.
+// Takes one queued match a lane (the last 32, or rest: those that are left) and
+// folds it; the probe columns above the join are read again at the row.
 static void emit_probe_take(std::ostringstream& os, Plan& p, const std::vector<int>& key_nodes, bool rest) {
     const bool table = p.path != AggPath::Regs;
     os << "        __syncwarp();\n";
-    if (!rest) os << "        vq_qn -= 32;\n";
-    os << "        const int vq_at = " << (rest ? "lane" : "vq_qn + lane") << ";\n";
-    if (rest && table) os << "        const bool vq_in = lane < vq_qn;\n";
-    os << "        " << (rest && !table ? "if (lane < vq_qn) {\n" : "{\n");
+    os << "        const int vq_m = " << (rest ? "min(vq_qn, 32)" : "32") << ";\n        vq_qn -= vq_m;\n";
+    if (rest) os << "        const bool vq_in = lane < vq_m;\n";
+    os << "        const int vq_at = vq_qn + " << (rest ? "(vq_in ? lane : 0)" : "lane") << ";\n";
+    os << "        " << (rest && !table ? "if (vq_in) {\n" : "{\n");
     const std::string in = rest && table ? "vq_in ? " : "", z = rest && table ? " : 0" : "";
     os << "            const long long r = " << in << "vq_qr[vq_qw][vq_at]" << z << ";\n";
     os << "            const unsigned long long jc = " << in << "vq_qc[vq_qw][vq_at]" << z << ";\n";
@@ -2796,45 +2804,93 @@ static void emit_probe_take(std::ostringstream& os, Plan& p, const std::vector<i
     os << "        }\n        __syncwarp();\n";
 }
 
-// One chunk of the join probe (a lane's four rows, loaded): a first pass runs
-// the filter and the key and issues the four table loads, a second resolves
-// them and folds the matches. With the queue, a chunk that follows a sparse one
-// queues its matches instead, and 32 at a time run the residual and the
-// aggregate with every lane at work.
-static void emit_probe_rows(std::ostringstream& os, Plan& p, const std::vector<int>& key_nodes, bool strided, bool queue) {
-    const std::string rk = std::string("r0 + ") + (strided ? "(k << 5)" : "k");
-    std::string K = std::to_string(p.probe_key);
-    // first pass over the lane's four rows: the filter, the key and the load
-    // of the key's home slot, so four table loads are in flight at once
-    os << "        unsigned long long vq_h[4]; ulonglong2 vq_s[4]; bool vq_on[4];\n";
+// Register path: takes up to 32 rows that passed a selective filter, looks their
+// keys up with every lane at work and queues the matches.
+static void emit_probe_lookup(std::ostringstream& os) {
+    os << "        __syncwarp();\n";
+    os << "        const int vq_m = min(vq_fn, 32);\n        vq_fn -= vq_m;\n";
+    os << "        const bool vq_in = lane < vq_m;\n        const int vq_at = vq_fn + (vq_in ? lane : 0);\n";
+    os << "        const unsigned long long jk = vq_fk[vq_qw][vq_at];\n        const auto vq_row = vq_fr[vq_qw][vq_at];\n";
+    os << "        unsigned long long jc = 0ull, jat = 0ull;\n        bool hit = false;\n";
+    os << "        if (vq_in) {\n            if (P.dmap) {\n";
+    os << "                const unsigned long long di = jk - (unsigned long long)P.dmin;\n";
+    os << "                jc = di < P.drange ? vq_ld_dword(P.dmap + di) : 0ull;\n                hit = jc != 0ull;\n";
+    os << "            } else {\n";
+    os << "                const unsigned long long h = jk == VQ_EMPTY_KEY ? P.jmask + 1 : (vq_hash(jk) & P.jmask);\n";
+    os << "                hit = vq_find_slot_from(P.jslot, P.jmask, jk, h, vq_ld_slot(P.jslot + h), jc, jat);\n";
+    os << "            }\n        }\n";
+    os << "        const unsigned vq_b = __ballot_sync(0xffffffffu, hit);\n";
+    os << "        if (hit) {\n            const int at = vq_qn + __popc(vq_b & ((1u << lane) - 1u));\n";
+    os << "            vq_qr[vq_qw][at] = vq_row;\n            vq_qc[vq_qw][at] = jc;\n        }\n        vq_qn += __popc(vq_b);\n";
+}
+
+// The lane's four rows of a probe chunk: the filter and the key, and per row
+// what `then` emits for a row that passes (with its key jk).
+template <class F>
+static void emit_probe_filter(std::ostringstream& os, Plan& p, bool strided, const std::string& rk, F then) {
+    const std::string K = std::to_string(p.probe_key);
     os << "#pragma unroll\n        for (int k = 0; k < 4; k++) {\n";
     os << "            const long long r = " << rk << ";\n";
     os << "            vq_on[k] = false;\n";
     os << "            if (r < s0 || r >= s1) continue;\n";
-    {
-        Gen g0(p, os);
-        if (strided) g0.kidx = "(k << 5)";
-        if (p.pred >= 0) {
-            g0.emit(p.pred);
-            os << "            if (!(x" << p.pred << " && ok" << p.pred << ")) continue;\n";
-        }
-        g0.emit(p.probe_key);
-        os << "            if (!ok" << K << ") continue;\n";
-        os << "            const unsigned long long jk = (unsigned long long)(long long)x" << K << ";\n";
-        // direct-mapped table: the key's own word (0: no build row)
-        os << "            if (P.dmap) {\n";
-        os << "                const unsigned long long di = jk - (unsigned long long)P.dmin;\n";
-        os << "                vq_s[k].y = di < P.drange ? vq_ld_dword(P.dmap + di) : 0ull;\n";
-        os << "            } else {\n";
-        os << "                vq_h[k] = jk == VQ_EMPTY_KEY ? P.jmask + 1 : (vq_hash(jk) & P.jmask);\n";
-        os << "                vq_s[k] = vq_ld_slot(P.jslot + vq_h[k]);\n";
-        os << "            }\n";
-        os << "            vq_on[k] = true;\n";
+    Gen g0(p, os);
+    if (strided) g0.kidx = "(k << 5)";
+    if (p.pred >= 0) {
+        g0.emit(p.pred);
+        os << "            if (!(x" << p.pred << " && ok" << p.pred << ")) continue;\n";
     }
-    os << "        }\n";
-    if (queue && p.path == AggPath::Regs) os << "        if (vq_last >= " << kQueueDense << ") {\n";
-    os << "#pragma unroll\n        for (int k = 0; k < 4; k++) {\n";
-    os << "            const long long r = " << rk << ";\n";
+    g0.emit(p.probe_key);
+    os << "            if (!ok" << K << ") continue;\n";
+    os << "            const unsigned long long jk = (unsigned long long)(long long)x" << K << ";\n";
+    then();
+    os << "            vq_on[k] = true;\n        }\n";
+}
+
+// The load of key jk's home slot (a direct-mapped table: the key's own word, 0: no build row).
+static void emit_probe_load(std::ostringstream& os) {
+    os << "            if (P.dmap) {\n";
+    os << "                const unsigned long long di = jk - (unsigned long long)P.dmin;\n";
+    os << "                vq_s[k].y = di < P.drange ? vq_ld_dword(P.dmap + di) : 0ull;\n";
+    os << "            } else {\n";
+    os << "                vq_h[k] = jk == VQ_EMPTY_KEY ? P.jmask + 1 : (vq_hash(jk) & P.jmask);\n";
+    os << "                vq_s[k] = vq_ld_slot(P.jslot + vq_h[k]);\n";
+    os << "            }\n";
+}
+
+// One chunk of the join probe (a lane's four rows, loaded): a first pass runs
+// the filter and the key and issues the four table loads, a second resolves
+// them and folds the matches, or queues them where the kernel has the queue.
+//
+// Looked up where the rows lie, nearly every warp waits for a load of one or two
+// lanes in every chunk. With the cp.async loop (plans of many accumulators) a
+// chunk that follows one of fewer than kQueueSparse rows queues the rows that
+// pass the filter instead, and the lookups run 32 at a time too: 6.0M rows, 4%
+// kept, 7 groups of 3 integer accumulators, 48 -> 31 us. The loop that prefetches
+// into registers has none to spare for it (5 groups of COUNT and SUM: 30% kept 63
+// us without, 73 with; 90% kept 100 and 110).
+static void emit_probe_rows(std::ostringstream& os, Plan& p, const std::vector<int>& key_nodes, bool strided, bool queue) {
+    const std::string rk = std::string("r0 + ") + (strided ? "(k << 5)" : "k");
+    const std::string K = std::to_string(p.probe_key);
+    const bool ahead = queue && probe_ahead(p), regs = p.path == AggPath::Regs;
+    os << "        unsigned long long vq_h[4]; ulonglong2 vq_s[4]; bool vq_on[4];\n";
+    auto push = [&](const std::string& row, const std::string& key, const std::string& rows, const std::string& keys, const std::string& n) {
+        os << "            const unsigned vq_b = __ballot_sync(0xffffffffu, vq_on[k]);\n";
+        os << "            if (vq_on[k]) {\n";
+        os << "                const int at = " << n << " + __popc(vq_b & ((1u << lane) - 1u));\n";
+        os << "                " << rows << "[vq_qw][at] = " << row << ";\n                " << keys << "[vq_qw][at] = " << key << ";\n";
+        if (p.join_gid) os << "                vq_qg[vq_qw][at] = (unsigned)vq_gid;\n";
+        os << "            }\n            " << n << " += __popc(vq_b);\n";
+    };
+    if (ahead) {
+        os << "        if (vq_last < " << kQueueSparse << ") {\n        vq_last = 0;\n";
+        emit_probe_filter(os, p, strided, rk, [&] { os << "            vq_h[k] = jk;\n"; });
+        os << "#pragma unroll\n        for (int k = 0; k < 4; k++) {\n";
+        push(rk, "vq_h[k]", "vq_fr", "vq_fk", "vq_fn");
+        os << "            vq_last += __popc(vq_b);\n        }\n        while (vq_fn >= 32) {\n";
+        emit_probe_lookup(os);
+        os << "        }\n        } else {\n";
+    }
+    emit_probe_filter(os, p, strided, rk, [&] { emit_probe_load(os); });
     Gen g(p, os);
     if (strided) g.kidx = "(k << 5)";
     // a single-row chain carries its build row in the slot (count word ~group
@@ -2852,38 +2908,40 @@ static void emit_probe_rows(std::ostringstream& os, Plan& p, const std::vector<i
         }
     };
     const std::string decl = std::string("            unsigned long long jc = 0ull, jat = 0ull") + (p.join_gid ? ", vq_gid = 0ull" : "") + ";\n";
-    if (!queue) {
-        os << "            if (!vq_on[k]) continue;\n" << decl;
-        resolve("continue;");
-        emit_probe_matches(os, p, key_nodes, g, "");
-        os << "        }\n";
-        return;
-    }
-    if (p.path == AggPath::Regs) {
+    auto fold = [&] {  // every row's matches, where they lie
+        os << "#pragma unroll\n        for (int k = 0; k < 4; k++) {\n";
+        os << "            const long long r = " << rk << ";\n";
         os << "            if (!vq_on[k]) continue;\n" << decl;
         resolve("{ vq_on[k] = false; continue; }");
         emit_probe_matches(os, p, key_nodes, g, "");
         os << "        }\n";
+        std::fill(g.done.begin(), g.done.end(), 0);
+    };
+    auto enqueue = [&] {
+        os << "#pragma unroll\n        for (int k = 0; k < 4; k++) {\n";
+        os << decl << "            if (vq_on[k]) do {\n";
+        resolve("{ vq_on[k] = false; break; }");
+        os << "            } while (false);\n";
+        push(rk, "jc", "vq_qr", "vq_qc", "vq_qn");
+        if (regs) os << "            vq_last += __popc(vq_b);\n";
+        os << "        }\n";
+    };
+    if (!queue) return fold();
+    if (regs) {
+        os << "        if (vq_last >= " << kQueueDense << ") {\n";
+        fold();
         os << "        vq_last = 0;\n";
         os << "#pragma unroll\n        for (int k = 0; k < 4; k++) vq_last += __popc(__ballot_sync(0xffffffffu, vq_on[k]));\n";
         os << "        } else {\n        vq_last = 0;\n";
-        os << "#pragma unroll\n        for (int k = 0; k < 4; k++) {\n";
-        os << "            const long long r = " << rk << ";\n";
+        enqueue();
+        if (ahead) os << "        }\n        }\n";
+    } else {
+        enqueue();
     }
-    os << decl;
-    std::fill(g.done.begin(), g.done.end(), 0);
-    os << "            if (vq_on[k]) do {\n";
-    resolve("{ vq_on[k] = false; break; }");
-    os << "            } while (false);\n";
-    os << "            const unsigned vq_b = __ballot_sync(0xffffffffu, vq_on[k]);\n";
-    os << "            if (vq_on[k]) {\n";
-    os << "                const int at = vq_qn + __popc(vq_b & ((1u << lane) - 1u));\n";
-    os << "                vq_qr[vq_qw][at] = r;\n                vq_qc[vq_qw][at] = jc;\n";
-    if (p.join_gid) os << "                vq_qg[vq_qw][at] = (unsigned)vq_gid;\n";
-    os << "            }\n            vq_qn += __popc(vq_b);\n" << (p.path == AggPath::Regs ? "            vq_last += __popc(vq_b);\n" : "") << "        }\n";
     os << "        while (vq_qn >= 32) {\n";
     emit_probe_take(os, p, key_nodes, false);
-    os << "        }\n" << (p.path == AggPath::Regs ? "        }\n" : "");
+    // (inside the branch that queued, where that is the only one)
+    os << "        }\n" << (regs && !ahead ? "        }\n" : "");
 }
 
 // Join probe kernel: probe rows pass the probe filter, look their key up, and
@@ -2919,7 +2977,12 @@ static std::string gen_probe_kernel(Plan& p, const std::vector<int>& key_nodes, 
     emit_probe_rows(os, p, key_nodes, loop.strided(), queue);
     loop.close(os);
     if (queue) {
-        os << "    {\n";
+        if (probe_ahead(p)) {
+            os << "    if (vq_fn > 0) {\n";
+            emit_probe_lookup(os);
+            os << "    }\n";
+        }
+        os << (probe_ahead(p) ? "    while" : "    if") << " (vq_qn > 0) {\n";  // (31 at most, and the last lookups' matches)
         emit_probe_take(os, p, key_nodes, true);
         os << "    }\n";
     }
