@@ -729,7 +729,7 @@ def main():
             "frac": round(achieved / peak, 4), "traffic": tr, "peak_source": f"{src} hbm_gbs",
             "kernel": ("vq_agg (Q1 scan-filter-project-aggregate, one launch: every block adds its partials as exact "
                        "fixed-point atomics into one of 8 accumulator copies and the last block to finish writes the "
-                       "merged row into pinned host memory; one event span)"),
+                       "merged row into pinned host memory; first block's start to that write, device clock)"),
             "q6_kernel_gbs": round(stats[0][1] / (q6_scan / 1e3) / 1e9, 1)}
     if rank == 0:
         line = {
