@@ -1,0 +1,78 @@
+// Compiles plans against tables that have a schema and no rows in memory, for
+// tests on hosts without a GPU: the library generates and compiles a plan's
+// kernels there and leaves them unloaded. Built and called by plan_probe.py.
+#include <cstring>
+#include <sstream>
+#include <string>
+
+#include "plan.h"
+
+using namespace vq;
+
+namespace {
+
+int put(const std::string& s, char* out, int cap) {
+    std::strncpy(out, s.c_str(), cap - 1);
+    out[cap - 1] = 0;
+    return s.rfind("error ", 0) == 0 ? -1 : 0;
+}
+
+std::string show(const Plan& p) {
+    std::ostringstream o;
+    o << "lsb=";
+    for (size_t i = 0; i < p.fx_lsb.size(); i++) o << (i ? "," : "") << p.fx_lsb[i];
+    o << " " << p.explain;
+    return o.str();
+}
+
+}  // namespace
+
+extern "C" {
+
+struct ProbeColumn {
+    int32_t type, nullable, has_range, finite;
+    int64_t dict, imin, imax;  // dict: entries of a STRING column's dictionary
+    double fmin, fmax;
+};
+
+void* probe_table(int n, const ProbeColumn* c, int64_t nrows) {
+    Table* t = new Table;
+    t->nrows = nrows;
+    t->n_rg = (int32_t)((nrows + t->rg_rows - 1) / t->rg_rows);
+    t->cols.resize(n);
+    for (int i = 0; i < n; i++) {
+        Column& k = t->cols[i];
+        k.name = "c" + std::to_string(i);
+        k.type = c[i].type;
+        k.nullable = c[i].nullable;
+        k.has_range = c[i].has_range;
+        k.finite = c[i].finite;
+        k.imin = c[i].imin;
+        k.imax = c[i].imax;
+        k.fmin = c[i].fmin;
+        k.fmax = c[i].fmax;
+        for (int64_t d = 0; d < c[i].dict; d++) k.dict.add("s" + std::to_string(d));
+    }
+    return t;
+}
+
+void probe_table_free(void* t) { delete (Table*)t; }
+
+int probe_agg(void* t, const vexq_agg_plan_desc* d, char* out, int cap) {
+    try {
+        std::unique_ptr<Plan> p(compile_agg((Table*)t, d));
+        return put(show(*p), out, cap);
+    } catch (const std::exception& e) {
+        return put(std::string("error ") + e.what(), out, cap);
+    }
+}
+
+int probe_join(void* build, void* probe, const vexq_join_plan_desc* d, char* out, int cap) {
+    try {
+        std::unique_ptr<Plan> p(compile_join((Table*)build, (Table*)probe, d));
+        return put(show(*p), out, cap);
+    } catch (const std::exception& e) {
+        return put(std::string("error ") + e.what(), out, cap);
+    }
+}
+}

@@ -2182,6 +2182,15 @@ static void emit_hash_update(std::ostringstream& os, Plan& p, Gen& g, const std:
     for (auto& s : p.slots) if (s.input >= 0) g.emit(s.input);
     emit_slot_values(os, p, ind, "hit");
     os << ind << "if (hit) {\n";
+    if (p.intkey_order) {
+        // the phase of the row's order key, from its packed key: a queued row
+        // carries the key and not its columns' NULLs
+        os << ind << "    bool anynull = false;\n";
+        for (const KeyCol& k : p.keys)
+            if (k.nullable)
+                os << ind << "    anynull = anynull || ((key >> " << k.shift << ") & " << (k.bits >= 64 ? ~0ull : (1ull << k.bits) - 1)
+                   << "ull) == " << k.domain - 1 << "ull;\n";
+    }
     os << ind << "    const long long vq_o = " << order_expr(p, "r") << ";\n";
     // (a first row read before another's minimum is only larger)
     os << ind << "    if (vq_o < vq_f0) atomicMin(&P.first[2 * slot], vq_o);\n";
