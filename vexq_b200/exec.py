@@ -409,9 +409,13 @@ class GpuFilter:
             pass
 
     def bitmap(self, row_start: int = 0, row_end: int = -1):
-        n = (self.table.host.nrows if row_end < 0 else row_end) - row_start
+        host = self.table.host
+        n = (host.nrows if row_end < 0 else row_end) - row_start
+        nb = max(0, (n + 7) // 8)
         # the library fills the bytes object itself: no cleared array, no copy
-        out = _new_bytes(None, max(0, (n + 7) // 8))
+        out = _new_bytes(None, nb)
+        if row_end >= 0 and (host is None or row_end > host.nrows):
+            C.memset(C.c_char_p(out), 0, nb)  # the rows past the table, which it does not write
         cnt = C.c_int64()
         abi.check(abi.load().vexq_filter_run(self.table.h, self.nodes, self.nn, self.ch, self.nc, self.root,
                                              row_start, row_end, C.cast(C.c_char_p(out), C.POINTER(C.c_uint8)), C.byref(cnt)))
