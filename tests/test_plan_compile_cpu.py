@@ -4,7 +4,7 @@ from __future__ import annotations
 
 import pytest
 
-from tests.plan_probe import Probe, abi, column
+from tests.plan_probe import Probe, abi, column, lsb
 from vexq_b200 import plan as P
 
 
@@ -24,3 +24,23 @@ def test_hashed_group_by_of_strings_compiles(probe, nullable):
     t = probe.table([column(abi.TYPE_STRING, n, 2100) for n in nullable] + [column(abi.TYPE_FLOAT64, True, lo=-9, hi=9)], 100_000)
     text = probe.agg(t, P.AggPlan(None, [0, 1], [P.count_star("n"), P.sum_(P.col(2), "s")]))
     assert "path=hash" in text, text
+
+
+@pytest.mark.parametrize("join", [False, True])
+def test_float_sum_windows_hold_every_row(probe, join):
+    """A sum's top digit takes up to 2^32 a row into a signed 64-bit counter where
+    the window ends with the values: 2^31 rows of one group."""
+    def window(nrows):
+        t = probe.table([column(abi.TYPE_INT64, lo=0, hi=99), column(abi.TYPE_FLOAT64, lo=0, hi=1.9999)], nrows)
+        if join:
+            b = probe.table([column(abi.TYPE_INT64, lo=0, hi=99), column(abi.TYPE_INT64, lo=0, hi=99)], 100)
+            text = probe.join(b, t, P.JoinPlan(0, 0, None, None, None, [1], [P.sum_(P.col(3), "s")]))
+        else:
+            text = probe.agg(t, P.AggPlan(None, [0], [P.sum_(P.col(1), "s")]))
+        return max(lsb(text)), text  # |x| < 2: the value's top bit weighs 2^0
+
+    for nrows in (1_000, 2 ** 31, 2 ** 31 + 1, 2 ** 32 - 2, 2 ** 33):
+        bottom, text = window(nrows)
+        top_digit = 2.0 ** (1 - bottom - 96)  # the most a row adds to the counter that weighs 2^(bottom + 96)
+        assert top_digit * nrows <= 2.0 ** 63, (nrows, text)
+        assert 1 - bottom <= 128 and bottom <= 1 - 97, (nrows, text)  # the window holds the values, 97 bits of them or more

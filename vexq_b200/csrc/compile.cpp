@@ -929,6 +929,7 @@ void choose_path(Plan& p) {
         p.slot_pos[s] = in_float ? p.nf++ : p.ni++;
     }
     p.fx_lsb.assign(std::max(p.nf, 1), 0);
+    p.fx_head = fx_headroom(p.t->nrows);
     if (p.path != AggPath::Regs) {
         if (p.nf > 16) fail(VEXQ_ENOTSUP, "more than 16 float sums in one aggregate");
         for (size_t s = 0; s < p.slots.size(); s++) {
@@ -942,8 +943,10 @@ void choose_path(Plan& p) {
             // binades lie in the two top digits (two atomics; three when the
             // window ended one bit into a digit), the counters' upper halves
             // hold the sums of 2^31 rows, and values of magnitude ≥ 2^(e-76)
-            // keep every mantissa bit (2^(e-45) in the block's group cache)
-            p.fx_lsb[p.slot_pos[s]] = e - VQ_FX_WINDOW;
+            // keep every mantissa bit (2^(e-45) in the block's group cache).
+            // Where more rows may meet in a sum the window begins VQ_FX_HEAD
+            // bits higher (fx_headroom)
+            p.fx_lsb[p.slot_pos[s]] = e - VQ_FX_WINDOW + p.fx_head;
         }
     }
 }
@@ -1603,6 +1606,8 @@ std::string cache_word(int k) { return "vq_a4 + " + std::to_string(k) + "u * vq_
 std::string fx_flags(const Plan& p, size_t s) {
     return std::string("<") + (slot_finite(p, s) ? "true" : "false") + ", " + (slot_signed(p, s) ? "true" : "false") + ">";
 }
+// The limbs' window lies in the digits' window so that both end where the values do.
+std::string limbs_up(const Plan& p) { return std::to_string(VQ_FX_HEAD - p.fx_head); }
 
 // MIN/MAX inputs as unsigned keys in the value's order
 std::string minmax_key(const Plan& p, size_t s) {
@@ -1649,8 +1654,8 @@ void emit_cache_update(std::ostringstream& os, const Plan& p, const std::string&
             case S_NN: os << in << iff << "vq_s_add(" << w << ", 1u);\n"; break;
             case S_ISUM: os << in << iff << "vq_s_add64(" << w << ", " << cache_word(F.at[s] + 1) << ", (unsigned long long)" << SV << ");\n"; break;
             case S_FSUM:
-                os << in << iff << "vq_s_fx_add" << fx_flags(p, s) << "(" << w << ", vq_s4, " << SV << ", P.fx_lsb[" << p.slot_pos[s]
-                   << "], P.error);\n";
+                os << in << iff << "vq_s_fx_add<" << (slot_finite(p, s) ? "true" : "false") << ", " << (slot_signed(p, s) ? "true" : "false") << ", "
+                   << limbs_up(p) << ">(" << w << ", vq_s4, " << SV << ", P.fx_lsb[" << p.slot_pos[s] << "], P.error);\n";
                 break;
             default: break;
         }
@@ -1794,7 +1799,7 @@ void emit_cache_flush(std::ostringstream& os, const Plan& p) {
             case S_FMIN: os << "        atomicMin(" << gu << ", " << v8 << ");\n"; break;
             case S_FMAX: os << "        atomicMax(" << gu << ", " << v8 << ");\n"; break;
             case S_FSUM:
-                os << "        vq_s_limbs_flush<" << (slot_signed(p, s) ? "true" : "false") << ">(" << w << ", vq_s4, (vq_i64*)P.acc_fx + (" << pos
+                os << "        vq_s_limbs_flush<" << (slot_signed(p, s) ? "true" : "false") << ", " << limbs_up(p) << ">(" << w << ", vq_s4, (vq_i64*)P.acc_fx + (" << pos
                    << " * stride + slot) * 4);\n";
                 if (!slot_finite(p, s))
                     os << "        { const unsigned f = vq_s_ld(" << cache_word(F.at[s] + kCacheLimbs) << "); if (f) atomicOr(&P.special[" << pos

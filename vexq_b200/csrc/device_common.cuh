@@ -207,17 +207,18 @@ __device__ __forceinline__ bool vq_fx_image(double x, int lsb, unsigned& mh, uns
 // until vq_s_limbs_norm. Unsigned limbs of 19 bits, or signed ones of 18 where
 // x may be negative, hold VQ_LIMB_ROWS rows between two normalisations.
 #define VQ_LIMBS 7
-#define VQ_LIMB_WINDOW 97  // bits of the limbs' window, which ends where the digits' does
+#define VQ_LIMB_WINDOW 97  // bits of the limbs' window, which ends where the values do
 #define VQ_LIMB_ROWS 8191u
 template <bool kSigned> __device__ __forceinline__ constexpr int vq_limb_bits() { return kSigned ? 18 : 19; }
 template <bool kSigned> __device__ __forceinline__ constexpr int vq_limb_shift() { return 6 * vq_limb_bits<kSigned>() - VQ_LIMB_WINDOW; }
-template <bool kFinite, bool kSigned>
+// (kUp: bits of the digits' window, whose LSB lsb is, below the limbs')
+template <bool kFinite, bool kSigned, int kUp>
 __device__ __forceinline__ void vq_s_fx_add(unsigned a, unsigned s, double x, int lsb, int* err) {
     constexpr int W = vq_limb_bits<kSigned>(), kShift = vq_limb_shift<kSigned>();
     constexpr unsigned M = (1u << W) - 1u;
     unsigned mh, lo, special;
     int sh;
-    if (!vq_fx_image<kFinite, VQ_LIMB_WINDOW>(x, lsb + (VQ_FX_WINDOW - VQ_LIMB_WINDOW), mh, lo, sh, special, err)) {
+    if (!vq_fx_image<kFinite, VQ_LIMB_WINDOW>(x, lsb + kUp, mh, lo, sh, special, err)) {
         if (!kFinite && special) vq_s_or(a + VQ_LIMBS * s, special);
         return;
     }
@@ -252,7 +253,7 @@ __device__ __forceinline__ void vq_s_limbs_norm(unsigned a, unsigned s) {
 }
 // The entry's sum in units of the window's LSB, added to the global table's
 // four 64-bit counters of 32-bit digits.
-template <bool kSigned>
+template <bool kSigned, int kUp>
 __device__ __forceinline__ void vq_s_limbs_flush(unsigned a, unsigned s, vq_i64* c) {
     constexpr int W = vq_limb_bits<kSigned>(), kShift = vq_limb_shift<kSigned>();
     vq_i64 d[VQ_FX_DIGITS] = {0, 0, 0, 0};
@@ -267,8 +268,10 @@ __device__ __forceinline__ void vq_s_limbs_flush(unsigned a, unsigned s, vq_i64*
         }
         // bits [W j - kShift, …) of the limbs' window; what is above the digits'
         // window (the last limb, below 2^31) stays in the top digit
-        const int at = W * j - kShift + (VQ_FX_WINDOW - VQ_LIMB_WINDOW), k = at >> 5 < VQ_FX_DIGITS ? at >> 5 : VQ_FX_DIGITS - 1;
-        d[k] += (vq_i64)((vq_u64)v << (at - 32 * k));
+        // (the lowest limb may begin below the digits' window, its bits there clear)
+        const int at = W * j - kShift + kUp, k = at < 0 ? 0 : at >> 5 < VQ_FX_DIGITS ? at >> 5 : VQ_FX_DIGITS - 1;
+        const int down = at < 0 ? -at : 0, left = at < 0 ? 0 : at - 32 * k;
+        d[k] += (vq_i64)((vq_u64)(v >> down) << left);
     }
 #pragma unroll
     for (int k = 0; k < VQ_FX_DIGITS; k++)

@@ -164,6 +164,7 @@ struct Plan {
     int nf = 0, ni = 0;            // float / int slots (path-specific layout)
     std::vector<int> slot_pos;     // slot → index within its float/int bank
     std::vector<int> fx_lsb;       // per float-sum slot
+    int fx_head = 0;               // bits its window leaves free above the largest values (fx_headroom)
     std::vector<long long> lits;   // launch-time literal table (VQParams::lit)
     std::vector<int> key_nodes;    // IR roots of the GROUP BY keys
     std::mutex body_mu;            // batch body text per block size, generated once
@@ -366,6 +367,14 @@ vexq_result_s* build_result(Plan& p, Groups& g);
 void own_dictionaries(vexq_result_s* r);
 int64_t scanned_bytes(const Plan& p, const Table& t, long long rows, bool build);
 long long estimate_groups(const Plan& p, long long rows, long long join_keys);
+// Bits a float sum's window leaves free above the largest values when up to
+// `adds` rows meet in one group. A digit takes up to 2^32 a row and its counter
+// is a signed 64-bit word, which holds 2^31 rows. Of a window that ends where
+// the values do the top digit is the one large values fill: 2^31 rows next to
+// the bound, or 2^32 ones, pass it. With VQ_FX_HEAD bits free it takes at most 2
+// a row and the digits below carry the sum (2^32 rows of evenly spread
+// mantissas, any number of small whole numbers), at a third digit a row.
+inline int fx_headroom(double adds) { return adds > 2147483648.0 ? VQ_FX_HEAD : 0; }
 void set_columns(VQParams& P, const Table& t, bool build_side);
 vexq_result_s* run_plan(Plan& p, int rg_start, int rg_end);
 // The same run, returning as soon as its launches are queued when the plan

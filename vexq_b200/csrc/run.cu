@@ -785,6 +785,7 @@ struct RunCtx {
     const JitKernel* k = nullptr;  // main kernel other than p.k_main (partition join)
     int grid = 0;                  // and its grid
     long long row0 = 0, row1 = 0;  // rows the main scan's ranges span
+    int fx_up = 0;                 // this run's float-sum windows begin higher than the plan's by (a join of repeated keys)
     bool from_build = false;       // the device clock's build start begins the run (a build the host did not wait for)
 
     // Whether the main kernel stamps the device clock: the scan and global
@@ -1270,19 +1271,24 @@ Compacted run_atomic(RunCtx& rc, VQParams& P, long long nchunks, long long estim
         unsigned long long* n_out = (unsigned long long*)(tail + 16);
         P.cap = (unsigned long long)cap;
         P.cap_mask = hash ? (unsigned long long)(cap - 1) : 0;
-        for (int f = 0; f < nf && f < 16; f++) P.fx_lsb[f] = p.fx_lsb[f];
+        for (int f = 0; f < nf && f < 16; f++) P.fx_lsb[f] = p.fx_lsb[f] + rc.fx_up;
         Compacted c;
-        // the plan's constant identities and float-sum windows, uploaded once
-        const size_t tinit = iv.size() * 8 + (size_t)std::max(nf, 1) * 4;
+        // the plan's constant identities and float-sum windows (its own and
+        // those VQ_FX_HEAD bits higher), uploaded once
+        const size_t b_lsb = (size_t)std::max(nf, 1) * 4, tinit = iv.size() * 8 + 2 * b_lsb;
         if (p.d_tinit.n < tinit) {
             std::vector<char> img(tinit, 0);
             std::memcpy(img.data(), iv.data(), iv.size() * 8);
-            if (nf) std::memcpy(img.data() + iv.size() * 8, p.fx_lsb.data(), (size_t)nf * 4);
+            int* lsb = (int*)(img.data() + iv.size() * 8);
+            for (int f = 0; f < nf; f++) {
+                lsb[f] = p.fx_lsb[f];
+                lsb[std::max(nf, 1) + f] = p.fx_lsb[f] + VQ_FX_HEAD;
+            }
             p.d_tinit.ensure(tinit);
             h2d(p.d_tinit.p, img.data(), tinit, rc.s);
         }
         const long long* d_iv = p.d_tinit.as<long long>();
-        const int* d_lsb = (const int*)(p.d_tinit.as<char>() + iv.size() * 8);
+        const int* d_lsb = (const int*)(p.d_tinit.as<char>() + iv.size() * 8 + (rc.fx_up ? b_lsb : 0));
         P.clk = rc.stamped() ? run_clock(p) : nullptr;
         auto mark = [&](cudaEvent_t e) {
             if (!P.clk) VQ_CUDA(cudaEventRecord(e, rc.s));
@@ -1563,7 +1569,7 @@ int topk_groups(RunCtx& rc, Compacted& c, Groups& g) {
         for (int f = 0; f < p.nf; f++) {
             const long long* d = r + 2 + p.ni + 5 * f;
             if (d[4] == kTopDouble) std::memcpy(&g.fval[f][j], d, 8);
-            else g.fval[f][j] = vq_fx_result(d, p.fx_lsb[f], (unsigned)d[4]);
+            else g.fval[f][j] = vq_fx_result(d, p.fx_lsb[f] + rc.fx_up, (unsigned)d[4]);
         }
     }
     return 1;
@@ -2159,6 +2165,7 @@ vexq_result_s* run_plan(Plan& p, int rg_start, int rg_end) {
     int64_t bytes = 0, rows_scanned = 0;
     bool use_radix = false;
     bool spec = false;  // the probe follows a direct-mapped build without the host waiting
+    double chain_most = 1;  // build rows a join key has at most
     int pbits = 0;
     if (p.is_join) {
         Table& bt = *p.bt;
@@ -2214,6 +2221,7 @@ vexq_result_s* run_plan(Plan& p, int rg_start, int rg_end) {
                 bytes += scanned_bytes(p, bt, bs.rows, true);
                 rows_scanned += bs.rows;
                 join_keys = total;  // at least the distinct build keys
+                chain_most = (double)std::min<long long>(total, p.rcap);
                 set_columns(P, bt, true);
                 P.bstart = bstart;
                 P.bkeys = p.rp_bkeys.as<unsigned long long>();
@@ -2513,6 +2521,7 @@ vexq_result_s* run_plan(Plan& p, int rg_start, int rg_end) {
             p.gid_groups = join_keys;
             p.join_keys_seen = join_keys;
             p.join_rows_seen = bs.rows;
+            if (!unique) chain_most = (double)(ntot - nk + 1);
         }
         break;
         }
@@ -2574,6 +2583,8 @@ vexq_result_s* run_plan(Plan& p, int rg_start, int rg_end) {
         rc.row0 = ss.seg.front();
         rc.row1 = ss.seg[ss.seg.size() - 2];
     }
+    // a join of repeated keys can emit more rows than the plan's window holds
+    if (p.is_join && !p.fx_head) rc.fx_up = fx_headroom((double)ss.rows * chain_most);
     bytes += sm.bytes;
     rows_scanned += ss.rows;
     if (use_radix && ss.nchunks > 0) {
