@@ -943,7 +943,8 @@ void choose_path(Plan& p) {
             // binades lie in the two top digits (two atomics; three when the
             // window ended one bit into a digit), the counters' upper halves
             // hold the sums of 2^31 rows, and values of magnitude ≥ 2^(e-76)
-            // keep every mantissa bit (2^(e-45) in the block's group cache).
+            // keep every mantissa bit (2^(e-45) in a dense table, in the block's
+            // group cache and beside it).
             // Where more rows may meet in a sum the window begins VQ_FX_HEAD
             // bits higher (fx_headroom)
             p.fx_lsb[p.slot_pos[s]] = e - VQ_FX_WINDOW + p.fx_head;
@@ -1603,8 +1604,9 @@ CacheField cache_fields(const Plan& p) {
 }
 std::string cache_word(int k) { return "vq_a4 + " + std::to_string(k) + "u * vq_s4"; }
 
-std::string fx_flags(const Plan& p, size_t s) {
-    return std::string("<") + (slot_finite(p, s) ? "true" : "false") + ", " + (slot_signed(p, s) ? "true" : "false") + ">";
+// Template arguments of float sum s's adds (up: the last one, "" none).
+std::string fx_flags(const Plan& p, size_t s, const std::string& up = "") {
+    return std::string("<") + (slot_finite(p, s) ? "true" : "false") + ", " + (slot_signed(p, s) ? "true" : "false") + (up.empty() ? "" : ", " + up) + ">";
 }
 // The limbs' window lies in the digits' window so that both end where the values do.
 std::string limbs_up(const Plan& p) { return std::to_string(VQ_FX_HEAD - p.fx_head); }
@@ -1654,8 +1656,7 @@ void emit_cache_update(std::ostringstream& os, const Plan& p, const std::string&
             case S_NN: os << in << iff << "vq_s_add(" << w << ", 1u);\n"; break;
             case S_ISUM: os << in << iff << "vq_s_add64(" << w << ", " << cache_word(F.at[s] + 1) << ", (unsigned long long)" << SV << ");\n"; break;
             case S_FSUM:
-                os << in << iff << "vq_s_fx_add<" << (slot_finite(p, s) ? "true" : "false") << ", " << (slot_signed(p, s) ? "true" : "false") << ", "
-                   << limbs_up(p) << ">(" << w << ", vq_s4, " << SV << ", P.fx_lsb[" << p.slot_pos[s] << "], P.error);\n";
+                os << in << iff << "vq_s_fx_add" << fx_flags(p, s, limbs_up(p)) << "(" << w << ", vq_s4, " << SV << ", P.fx_lsb[" << p.slot_pos[s] << "], P.error);\n";
                 break;
             default: break;
         }
@@ -1703,7 +1704,7 @@ void emit_table_update(std::ostringstream& os, const Plan& p, const std::string&
             case S_FMAX: os << in << "if (sok" << S << " && !isnan(" << SV << ")) atomicMax(" << aiu << ", vq_fkey(" << SV << "));\n"; break;
             case S_FSUM:
                 if (!sums) break;
-                os << in << iff << "vq_g_fx_add" << fx_flags(p, s) << "(P.acc_fx + ((long long)" << pos << " * stride + (long long)slot) * 4, P.special + (long long)"
+                os << in << iff << "vq_g_fx_add" << fx_flags(p, s, p.path == AggPath::Dense ? limbs_up(p) : "0") << "(P.acc_fx + ((long long)" << pos << " * stride + (long long)slot) * 4, P.special + (long long)"
                    << pos << " * stride + slot, " << SV << ", P.fx_lsb[" << pos << "], P.error);\n";
                 break;
         }

@@ -97,8 +97,8 @@ __device__ __forceinline__ void vq_add64_as32(vq_i64* c, vq_i64 d) {
 // four signed 64-bit counters holding 32-bit digits (c[k] weighs 2^(32k+lsb)).
 // Integer addition is associative, so the sum is the same whatever order the
 // atomics land in. Bits of x below 2^lsb are truncated (the window is chosen
-// so that only values below 2^-45 (register path) or 2^-76 (group tables) of the
-// largest possible |x| lose bits).
+// so that only values below 2^-45 (register path, dense tables) or 2^-76 (the
+// other group tables) of the largest possible |x| lose bits).
 // Non-finite values set flags instead. stride is the distance between digits.
 template <bool kAtomic, bool kPair32 = false>
 __device__ __forceinline__ void vq_fx_add(vq_i64* c, double x, int lsb, unsigned* special, int* err) {
@@ -279,15 +279,19 @@ __device__ __forceinline__ void vq_s_limbs_flush(unsigned a, unsigned s, vq_i64*
 }
 
 // The same sum in the global table: four 64-bit counters of signed 32-bit
-// digits (vq_fx_add's), at most three of them touched by a value.
-template <bool kFinite, bool kSigned>
+// digits (vq_fx_add's), at most three of them touched by a value. kUp: bits of
+// the window left out at its low end, so that a table whose groups may have a
+// cache entry keeps the same bits of a value in it and beside it, whatever the
+// cache's size (0: the whole window).
+template <bool kFinite, bool kSigned, int kUp>
 __device__ __forceinline__ void vq_g_fx_add(vq_i64* c, unsigned* sp, double x, int lsb, int* err) {
     unsigned mh, lo, special;
     int sh;
-    if (!vq_fx_image<kFinite, VQ_FX_WINDOW>(x, lsb, mh, lo, sh, special, err)) {
+    if (!vq_fx_image<kFinite, VQ_FX_WINDOW - kUp>(x, lsb + kUp, mh, lo, sh, special, err)) {
         if (!kFinite && special) atomicOr(sp, special);
         return;
     }
+    sh += kUp;
     const int off = sh & 31;
     const unsigned t[3] = {lo << off, __funnelshift_l(lo, mh, off), __funnelshift_l(mh, 0u, off)};
     unsigned long long* p = reinterpret_cast<unsigned long long*>(c + (sh >> 5));
@@ -309,7 +313,7 @@ __device__ __forceinline__ void vq_g_fx_add(vq_i64* c, unsigned* sp, double x, i
 template <bool kFinite, bool kSigned>
 __device__ __forceinline__ void vq_w_fx_add(bool on, vq_u64 slot, vq_u64 cap, vq_i64* c, unsigned* sp, double x, int lsb, int* err) {
     if (cap >= 0x7FFFFFFFull) {  // slot and sign do not fit a word
-        if (on) vq_g_fx_add<kFinite, kSigned>(c + slot * 4, sp + slot, x, lsb, err);
+        if (on) vq_g_fx_add<kFinite, kSigned, 0>(c + slot * 4, sp + slot, x, lsb, err);
         return;
     }
     unsigned mh = 0u, lo = 0u, special = 0u;
