@@ -100,7 +100,11 @@ struct Batch {
     std::vector<vexq_plan_s*> handles;
     std::vector<Item> items;
     ClassKernel ck[3];  // register path, group tables, join builds (run before both)
-    int cache_kb = 190, unit_div = 2;
+    // units a resident block of each class: two of the group tables' (kBlockTable),
+    // four of the others'. A register-path sum runs over its unit's rows before
+    // the merge's compensation, so its rounding goes with the unit's size (32 plans,
+    // 12.6M rows: 1.8e-17 of the exact values off with two, 1.5e-19 with four)
+    int cache_kb = 190, unit_div[3] = {4, 2, 4};
     DevBuf dev, out;
     PinnedBuf h_out;
     size_t out_bytes = 0, a_params = 0, a_bparams = 0, a_tdesc = 0, a_mdesc = 0, a_ticket = 0, o_aerr = 0;
@@ -146,12 +150,12 @@ struct Batch {
     // parameter blocks, unit lists and descriptors.
     void layout() {
         drop_graph();
-        // units: about unit_div units per resident block of each class, at
-        // least 16 chunks (2,048 rows) each
+        // units: about unit_div per resident block of each class, at least 16
+        // chunks (2,048 rows) each
         for (int c = 0; c < 3; c++) {
             long long chunks = 0;
             for (int i : ck[c].items) chunks += c == 2 ? items[i].bnchunks : items[i].nchunks;
-            long long target = std::max<long long>(1, (long long)ck[c].grid * unit_div);
+            long long target = std::max<long long>(1, (long long)ck[c].grid * unit_div[c]);
             long long U = std::max<long long>(16, (chunks + target - 1) / target);
             ck[c].nunits = 0;
             for (int i : ck[c].items) {
@@ -435,7 +439,7 @@ struct Batch {
         ex << "batch plans=" << items.size() << " regs_plans=" << ck[0].items.size() << " regs_bodies=" << ck[0].nbodies
            << " regs_units=" << ck[0].nunits << " table_plans=" << ck[1].items.size() << " table_bodies=" << ck[1].nbodies
            << " table_units=" << ck[1].nunits << " joins=" << njoins << " build_units=" << ck[2].nunits << " cache_kb=" << cache_kb
-           << " unit_div=" << unit_div;
+           << " unit_div=" << unit_div[0] << "/" << unit_div[1] << "/" << unit_div[2];
         explain = ex.str();
     }
 
@@ -631,10 +635,10 @@ struct Batch {
     struct Tuning {
         int cache_kb, unit_div, block_regs, block_table;
     };
-    Tuning tuning() const { return {cache_kb, unit_div, ck[0].block, ck[1].block}; }
+    Tuning tuning() const { return {cache_kb, unit_div[1], ck[0].block, ck[1].block}; }
     void apply(const Tuning& t) {
         cache_kb = t.cache_kb;
-        unit_div = t.unit_div;
+        for (int& u : unit_div) u = t.unit_div;  // a tuned batch: one for all classes
         for (int c = 0; c < 2; c++) {
             const int b = c ? t.block_table : t.block_regs;
             if (b != ck[c].block) {
