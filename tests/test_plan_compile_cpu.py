@@ -44,3 +44,15 @@ def test_float_sum_windows_hold_every_row(probe, join):
         top_digit = 2.0 ** (1 - bottom - 96)  # the most a row adds to the counter that weighs 2^(bottom + 96)
         assert top_digit * nrows <= 2.0 ** 63, (nrows, text)
         assert 1 - bottom <= 128 and bottom <= 1 - 97, (nrows, text)  # the window holds the values, 97 bits of them or more
+
+
+@pytest.mark.parametrize("block", [64, 128, 256, 384, 512])
+@pytest.mark.parametrize("shape", ["by_key", "by_date", "registers"])
+def test_join_probes_compile_at_every_block_size(probe, monkeypatch, block, shape):
+    # the probe's queues are in static shared memory, 48 KB a block at most
+    monkeypatch.setenv("VEXQ_TUNE", f"block={block} async=2")
+    b = probe.table([column(abi.TYPE_INT64, lo=0, hi=99_999), column(abi.TYPE_DATE, lo=8000, hi=9000), column(abi.TYPE_INT64, lo=0, hi=4)], 100_000)
+    t = probe.table([column(abi.TYPE_INT64, lo=0, hi=99_999), column(abi.TYPE_FLOAT64, True, lo=-9, hi=9), column(abi.TYPE_INT64, lo=0, hi=9)], 400_000)
+    by = {"by_key": 0, "by_date": 1, "registers": 2}[shape]
+    text = probe.join(b, t, P.JoinPlan(0, 0, None, P.col(2) < 3, None, [by], [P.sum_(P.col(4), "s"), P.count_star("n")]))
+    assert text.startswith("lsb="), text

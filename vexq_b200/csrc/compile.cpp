@@ -2736,7 +2736,7 @@ static bool probe_ahead(const Plan& p) { return p.path == AggPath::Regs && !p.st
 static std::string queue_row(const Plan& p) { return probe_ahead(p) && p.t->nrows < (1ll << 32) ? "unsigned" : "long long"; }
 
 static bool probe_queue(const Plan& p, int block) {
-    const size_t row = p.t->nrows < (1ll << 32) ? 4 : 8, entries = (size_t)(block / 32) * kProbeQueue;
+    const size_t row = queue_row(p) == "unsigned" ? 4 : 8, entries = (size_t)(block / 32) * kProbeQueue;
     if (p.path != AggPath::Regs) return p.nf > 0 && entries * (row + 8 + (p.join_gid ? 4 : 0)) <= 46 * 1024;
     return p.pred >= 0 && entries * (probe_ahead(p) ? 2 : 1) * (row + 8) + regs_flush_smem(p, block) <= 46 * 1024;
 }
