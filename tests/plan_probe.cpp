@@ -67,6 +67,17 @@ int probe_agg(void* t, const vexq_agg_plan_desc* d, char* out, int cap) {
     }
 }
 
+// The key a Filter call's plan is kept under: its length, and the key's bytes in out.
+int probe_filter_key(void* t, const vexq_expr* nodes, int nnodes, const int32_t* children, int nchildren, int pred, char* out, int cap) {
+    try {
+        SelectLease l(*(Table*)t, 'f', nodes, nnodes, children, nchildren, pred, nullptr, 0);
+        std::memcpy(out, l.key.data(), std::min<size_t>(l.key.size(), cap));
+        return (int)l.key.size();
+    } catch (const std::exception& e) {
+        return put(std::string("error ") + e.what(), out, cap);
+    }
+}
+
 int probe_join(void* build, void* probe, const vexq_join_plan_desc* d, char* out, int cap) {
     try {
         std::unique_ptr<Plan> p(compile_join((Table*)build, (Table*)probe, d));

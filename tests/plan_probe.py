@@ -7,6 +7,7 @@ import os
 import subprocess
 
 from vexq_b200 import abi, build
+from vexq_b200 import plan as P
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 PACKAGE = os.path.dirname(os.path.abspath(build.__file__))
@@ -35,6 +36,7 @@ class Probe:
         L.probe_table.argtypes = [C.c_int, C.c_void_p, C.c_int64]
         L.probe_table_free.argtypes = [C.c_void_p]
         L.probe_agg.argtypes = [C.c_void_p, C.c_void_p, C.c_char_p, C.c_int]
+        L.probe_filter_key.argtypes = [C.c_void_p, C.c_void_p, C.c_int, C.c_void_p, C.c_int, C.c_int, C.c_char_p, C.c_int]
         L.probe_join.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p, C.c_char_p, C.c_int]
         self.tables = []
 
@@ -53,6 +55,17 @@ class Probe:
         out = C.create_string_buffer(8192)
         self.lib.probe_join(build_table, probe_table, C.byref(plan.desc), out, len(out))
         return out.value.decode(errors="replace")
+
+    def filter_key(self, table, pred, lit_strs=None) -> bytes:
+        """The key a Filter call's plan is kept under; lit_strs: {node: text}
+        put into lit_str whatever the node's kind."""
+        arena, nodes, nn, ch, nc, root = P.predicate_arrays(pred)
+        for i, s in (lit_strs or {}).items():
+            nodes[i].lit_str = s
+        out = C.create_string_buffer(8192)
+        n = self.lib.probe_filter_key(table, nodes, nn, ch, nc, root, out, len(out))
+        assert n > 0, out.value
+        return out.raw[:n]
 
     def close(self):
         for t in self.tables:

@@ -56,3 +56,15 @@ def test_join_probes_compile_at_every_block_size(probe, monkeypatch, block, shap
     by = {"by_key": 0, "by_date": 1, "registers": 2}[shape]
     text = probe.join(b, t, P.JoinPlan(0, 0, None, P.col(2) < 3, None, [by], [P.sum_(P.col(4), "s"), P.count_star("n")]))
     assert text.startswith("lsb="), text
+
+
+def test_a_kept_filter_plan_is_keyed_by_its_expression(probe):
+    t = probe.table([column(abi.TYPE_INT64, lo=0, hi=99), column(abi.TYPE_DATE, lo=8000, hi=9000)], 100_000)
+    number, date = P.col(0) < 7, P.col(1) < P.lit("1994-01-01")
+    assert [n.kind for n in P.predicate_arrays(number)[0].nodes] == [abi.E_COLUMN, abi.E_LITERAL, abi.E_BINARY]
+    # lit_str is read of STRING literals only: a caller leaves it unset elsewhere
+    key = probe.filter_key(t, number)
+    assert all(probe.filter_key(t, number, {i: b"stray"}) == key for i in range(3))
+    assert probe.filter_key(t, date, {0: b"stray"}) == probe.filter_key(t, date)
+    keys = [probe.filter_key(t, p) for p in (number, P.col(0) < 8, P.col(0) <= 7, date, P.col(1) < P.lit("1994-01-02"))]
+    assert len(set(keys)) == len(keys)

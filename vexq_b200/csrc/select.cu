@@ -231,9 +231,11 @@ SelectLease::SelectLease(Table& tb, char kind, const vexq_expr* nodes, int nnode
         raw(head, sizeof head);
         raw(&e.lit_int, 8);
         raw(&e.lit_float, 8);
-        const int64_t len = e.lit_str ? (int64_t)std::strlen(e.lit_str) : -1;
+        // (lit_str of any other node is the caller's to leave unset)
+        const char* s = e.kind == VEXQ_E_LITERAL && e.lit_kind == VEXQ_LIT_STRING ? e.lit_str : nullptr;
+        const int64_t len = s ? (int64_t)std::strlen(s) : -1;
         raw(&len, 8);
-        if (len > 0) raw(e.lit_str, (size_t)len);
+        if (len > 0) raw(s, (size_t)len);
     }
     {
         const std::shared_ptr<SelectPlans> sp = selects_of(t);
