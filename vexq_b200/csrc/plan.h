@@ -133,6 +133,7 @@ struct OutPool {
     // address; lend tells whether the result may keep it.
     std::shared_ptr<OutBlock> acquire(size_t bytes, bool& lend);
     void trim(size_t most);  // drops blocks of more than `most` bytes (a result that holds one keeps it)
+    size_t bytes() const;    // of its blocks, lent or not
 };
 
 struct Plan {

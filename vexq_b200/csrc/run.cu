@@ -840,6 +840,12 @@ void OutPool::trim(size_t most) {
     if (stage && stage->pin.n > most) stage.reset();
 }
 
+size_t OutPool::bytes() const {
+    size_t n = stage ? stage->pin.n : 0;
+    for (const auto& b : lent) n += b->pin.n;
+    return n;
+}
+
 void ensure_events(Plan& p) {
     for (auto& e : p.ev)
         if (!e) VQ_CUDA(cudaEventCreate(&e));

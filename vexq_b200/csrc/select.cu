@@ -195,23 +195,65 @@ std::map<const Table*, std::unique_ptr<HostMirror>> g_mirrors;
 
 // Plans kept per table: the most recent kKept, each holding at most kKeptBytes
 // of device and of pinned memory between calls (larger buffers are freed with
-// the call that grew them). A call used to compile its plan, create a stream
-// and allocate every buffer: about 450 us of a 6M-row selection bitmap's 655.
-struct SelectPlans {
-    std::mutex mu;
-    struct Kept {
-        std::string key;
-        std::unique_ptr<Plan> p;
-    };
-    std::vector<Kept> kept;  // oldest first
+// the call that grew them, and allocated again by the next). A call used to
+// compile its plan, create a stream and allocate every buffer: about 450 us of a
+// 6M-row selection bitmap's 655. Over all tables at most kAllKept plans and
+// kAllBytes of each memory are kept; the least recently used go first, and a
+// table's go with it.
+struct KeptPlan {
+    std::string key;
+    std::unique_ptr<Plan> p;
+    size_t dev = 0, pinned = 0;  // bytes it holds
+    uint64_t used = 0;
 };
-static std::mutex g_selects_mu;
-constexpr size_t kKept = 8, kKeptBytes = 32u << 20;
+struct SelectPlans {
+    std::vector<KeptPlan> kept;
+    SelectPlans();
+    ~SelectPlans();
+};
+namespace {
+constexpr size_t kKept = 8, kKeptBytes = 32u << 20, kAllKept = 64, kAllBytes = 128u << 20;
+// every table's plans, and what they hold together (guarded by mu)
+struct AllKept {
+    std::mutex mu;
+    std::vector<SelectPlans*> tables;
+    size_t n = 0, dev = 0, pinned = 0;
+    uint64_t clock = 0;
+    KeptPlan take(SelectPlans& s, size_t i) {
+        KeptPlan k = std::move(s.kept[i]);
+        s.kept.erase(s.kept.begin() + i);
+        n--;
+        dev -= k.dev;
+        pinned -= k.pinned;
+        return k;
+    }
+    // the least recently used plan of one table, or of all (null)
+    KeptPlan oldest(SelectPlans* of) {
+        SelectPlans* at = nullptr;
+        size_t ix = 0;
+        for (SelectPlans* s : tables)
+            if (!of || s == of)
+                for (size_t i = 0; i < s->kept.size(); i++)
+                    if (!at || s->kept[i].used < at->kept[ix].used) {
+                        at = s;
+                        ix = i;
+                    }
+        return take(*at, ix);
+    }
+};
+AllKept& all_kept() {
+    static auto* a = new AllKept;  // (tables may outlive the statics)
+    return *a;
+}
+}  // namespace
 
-static std::shared_ptr<SelectPlans> selects_of(Table& t) {
-    std::lock_guard<std::mutex> lk(g_selects_mu);
-    if (!t.selects) t.selects = std::make_shared<SelectPlans>();
-    return t.selects;
+SelectPlans::SelectPlans() { all_kept().tables.push_back(this); }
+SelectPlans::~SelectPlans() {
+    AllKept& a = all_kept();
+    std::vector<KeptPlan> gone;  // plans are destroyed without the lock
+    std::lock_guard<std::mutex> lk(a.mu);
+    while (!kept.empty()) gone.push_back(a.take(*this, kept.size() - 1));
+    a.tables.erase(std::find(a.tables.begin(), a.tables.end(), this));
 }
 
 SelectLease::SelectLease(Table& tb, char kind, const vexq_expr* nodes, int nnodes, const int32_t* children, int nchildren, int pred,
@@ -238,16 +280,15 @@ SelectLease::SelectLease(Table& tb, char kind, const vexq_expr* nodes, int nnode
         if (len > 0) raw(s, (size_t)len);
     }
     {
-        const std::shared_ptr<SelectPlans> sp = selects_of(t);
-        std::lock_guard<std::mutex> lk(sp->mu);
-        for (size_t i = sp->kept.size(); i-- > 0;) {
+        AllKept& a = all_kept();
+        std::vector<KeptPlan> gone;
+        std::lock_guard<std::mutex> lk(a.mu);
+        if (!t.selects) t.selects = std::make_shared<SelectPlans>();
+        std::vector<KeptPlan>& kept = t.selects->kept;
+        for (size_t i = kept.size(); i-- > 0;) {
             // a refill that widened a column's range changes what is generated
-            if (sp->kept[i].p->range_epoch != t.range_epoch) {
-                sp->kept.erase(sp->kept.begin() + i);
-            } else if (!p && sp->kept[i].key == key) {
-                p = std::move(sp->kept[i].p);
-                sp->kept.erase(sp->kept.begin() + i);
-            }
+            if (kept[i].p->range_epoch != t.range_epoch) gone.push_back(a.take(*t.selects, i));
+            else if (!p && kept[i].key == key) p = a.take(*t.selects, i).p;
         }
     }
     if (!p) p.reset(kind == 'f' ? compile_filter(&t, nodes, nnodes, children, nchildren, pred)
@@ -256,20 +297,29 @@ SelectLease::SelectLease(Table& tb, char kind, const vexq_expr* nodes, int nnode
 
 void SelectLease::done() {
     DevBuf* bufs[] = {&p->scratch_a, &p->scratch_b, &p->scratch_c, &p->scratch_d};
-    size_t held = 0;
-    for (DevBuf* b : bufs) held += b->n;
-    if (held > kKeptBytes)
+    KeptPlan k;
+    for (DevBuf* b : bufs) k.dev += b->n;
+    if (k.dev > kKeptBytes) {
         for (DevBuf* b : bufs) b->release();
+        k.dev = 0;
+    }
     if (p->h_stage.n > kKeptBytes) p->h_stage.release();
     p->out_pool.trim(kKeptBytes / 2);
-    const std::shared_ptr<SelectPlans> sp = selects_of(t);
-    std::unique_ptr<Plan> old;
-    std::lock_guard<std::mutex> lk(sp->mu);
-    if (sp->kept.size() >= kKept) {
-        old = std::move(sp->kept.front().p);
-        sp->kept.erase(sp->kept.begin());
-    }
-    sp->kept.push_back({std::move(key), std::move(p)});
+    k.dev += p->d_seg.n + p->d_sets.n + p->d_present.n;
+    k.pinned = p->h_stage.n + p->out_pool.bytes();
+    k.key = std::move(key);
+    k.p = std::move(p);
+    AllKept& a = all_kept();
+    std::vector<KeptPlan> gone;
+    std::lock_guard<std::mutex> lk(a.mu);
+    SelectPlans& s = *t.selects;
+    if (s.kept.size() >= kKept) gone.push_back(a.oldest(&s));
+    k.used = ++a.clock;
+    a.n++;
+    a.dev += k.dev;
+    a.pinned += k.pinned;
+    s.kept.push_back(std::move(k));
+    while (a.n > kAllKept || a.dev > kAllBytes || a.pinned > kAllBytes) gone.push_back(a.oldest(nullptr));
 }
 
 void drop_host_mirror(const Table* t) {
