@@ -78,6 +78,28 @@ int probe_filter_key(void* t, const vexq_expr* nodes, int nnodes, const int32_t*
     }
 }
 
+// Pinned bytes a pool holds after n blocks of `bytes` were taken and kept, and
+// (in lent) how many of them results may keep. Needs a GPU.
+int64_t probe_out_pool(int n, int64_t bytes, int64_t lend_most, int32_t* lent) {
+    try {
+        OutPool pool;
+        pool.lend_most = (size_t)lend_most;
+        std::vector<std::shared_ptr<OutBlock>> held;
+        *lent = 0;
+        for (int i = 0; i < n; i++) {
+            bool lend = false;
+            std::shared_ptr<OutBlock> b = pool.acquire((size_t)bytes, lend);
+            if (lend) {
+                held.push_back(b);
+                ++*lent;
+            }
+        }
+        return (int64_t)pool.bytes();
+    } catch (const std::exception&) {
+        return -1;
+    }
+}
+
 int probe_join(void* build, void* probe, const vexq_join_plan_desc* d, char* out, int cap) {
     try {
         std::unique_ptr<Plan> p(compile_join((Table*)build, (Table*)probe, d));

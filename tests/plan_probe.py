@@ -37,6 +37,8 @@ class Probe:
         L.probe_table_free.argtypes = [C.c_void_p]
         L.probe_agg.argtypes = [C.c_void_p, C.c_void_p, C.c_char_p, C.c_int]
         L.probe_filter_key.argtypes = [C.c_void_p, C.c_void_p, C.c_int, C.c_void_p, C.c_int, C.c_int, C.c_char_p, C.c_int]
+        L.probe_out_pool.restype = C.c_int64
+        L.probe_out_pool.argtypes = [C.c_int, C.c_int64, C.c_int64, C.c_void_p]
         L.probe_join.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p, C.c_char_p, C.c_int]
         self.tables = []
 
@@ -66,6 +68,11 @@ class Probe:
         n = self.lib.probe_filter_key(table, nodes, nn, ch, nc, root, out, len(out))
         assert n > 0, out.value
         return out.raw[:n]
+
+    def out_pool(self, n: int, bytes_: int, lend_most: int):
+        """(pinned bytes, blocks lent) of a result pool that gave n blocks out; needs a GPU."""
+        lent = C.c_int32()
+        return self.lib.probe_out_pool(n, bytes_, lend_most, C.byref(lent)), lent.value
 
     def close(self):
         for t in self.tables:

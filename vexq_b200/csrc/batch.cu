@@ -115,6 +115,10 @@ struct Batch {
     int n_fdesc = 0, n_adesc = 0;
     long long fin_slots = 0;
     size_t a_adesc = 0, a_outp = 0, asm_bytes = 0;
+    // a block holds every slot of every assembled table (one result keeps all
+    // of it): above kLendMost one block serves every execution, as the copied
+    // outputs' does
+    static constexpr size_t kLendMost = 64u << 20;
     OutPool pool;
     std::shared_ptr<OutBlock> blk;  // the current execution's block of assembled columns
     bool blk_lend = true;
@@ -563,6 +567,7 @@ struct Batch {
     void take_block() {
         if (n_adesc == 0) return;
         blk.reset();
+        pool.lend_most = kLendMost;
         blk = pool.acquire(asm_bytes, blk_lend);
         if (!blk) fail(VEXQ_EDEVICE, "pinned host memory has no device address");
         if (blk->dev == blk_sent) return;

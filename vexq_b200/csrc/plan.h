@@ -125,8 +125,10 @@ struct OutBlock {
 // The pinned blocks of one plan or batch. A block goes to one result at a
 // time and comes back when that result (its last holder) is freed; at most two
 // are lent, and a run that finds both with results still alive writes the
-// third, whose rows its result copies.
+// third, whose rows its result copies. Blocks of more than lend_most bytes are
+// not lent: the pool then has one, and every result copies its rows.
 struct OutPool {
+    size_t lend_most = ~(size_t)0;
     std::vector<std::shared_ptr<OutBlock>> lent;
     std::shared_ptr<OutBlock> stage;
     // A block of at least `bytes`, null where pinned memory has no device

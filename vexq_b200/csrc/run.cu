@@ -815,11 +815,11 @@ std::shared_ptr<OutBlock> OutPool::acquire(size_t bytes, bool& lend) {
         if (cudaHostGetDevicePointer(&d, b.pin.p, 0) == cudaSuccess) b.dev = (char*)d;
         else (void)cudaGetLastError();
     };
-    lend = true;
+    lend = bytes <= lend_most;
     std::shared_ptr<OutBlock> b;
     for (auto& x : lent)
-        if (x.use_count() == 1 && (!b || x->pin.n > b->pin.n)) b = x;  // the pool is its only holder
-    if (!b && lent.size() < 2) {
+        if (lend && x.use_count() == 1 && (!b || x->pin.n > b->pin.n)) b = x;  // the pool is its only holder
+    if (lend && !b && lent.size() < 2) {
         b = std::make_shared<OutBlock>();
         lent.push_back(b);
     }
