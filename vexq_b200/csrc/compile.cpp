@@ -1812,12 +1812,14 @@ void emit_cache_flush(std::ostringstream& os, const Plan& p) {
 }
 
 // The scan's clock stamps: its first block's start, and (group tables; the
-// register path's last block hands its end out) its last block's end.
+// register path's last block hands its end out) its last block's end, when all
+// of the block's warps are through.
 void emit_clock_start(std::ostringstream& os) {
     os << "    if (P.clk && blockIdx.x == 0 && threadIdx.x == 0) P.clk[VQ_CLK_SCAN] = vq_clock();\n";
 }
 void emit_clock_end(std::ostringstream& os, const Plan& p) {
-    if (p.path != AggPath::Regs) os << "    if (P.clk && threadIdx.x == 0) atomicMax(P.clk + VQ_CLK_SCAN_END, vq_clock());\n";
+    if (p.path == AggPath::Regs) return;
+    os << "    if (P.clk) {\n        __syncthreads();\n        if (threadIdx.x == 0) atomicMax(P.clk + VQ_CLK_SCAN_END, vq_clock());\n    }\n";
 }
 
 std::string kernel_head(const std::string& name, int block, int min_blocks = 0) {
