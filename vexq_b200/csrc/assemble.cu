@@ -218,8 +218,12 @@ k_assemble(const VQAsmDesc* descs, char* base, char* const* basep) {
         VQAsmHdr* h = reinterpret_cast<VQAsmHdr*>(out);
         h->n = (unsigned long long)n;
         h->err = *d.error;
-        if (d.clk && d.write) asm_clock(d, h);
         d.pref[d.nwords / 4 + kAsmCtas] = (unsigned)n;
+    }
+    // the columns' end: the last CTA's, when all of its warps are through
+    if (d.clk && d.write) {
+        __syncthreads();
+        if (tid == 0 && atomicAdd(d.clk + VQ_CLK_DONE, 1ull) % kAsmCtas == kAsmCtas - 1) asm_clock(d, reinterpret_cast<VQAsmHdr*>(out));
     }
 }
 
