@@ -21,7 +21,9 @@ std::string show(const Plan& p) {
     std::ostringstream o;
     o << "lsb=";
     for (size_t i = 0; i < p.fx_lsb.size(); i++) o << (i ? "," : "") << p.fx_lsb[i];
-    o << " " << p.explain;
+    int sums = 0;  // places the main kernel's text adds a warp's float sum
+    for (size_t at = 0; (at = p.src_main.find("vq_w_fx_add<", at)) != std::string::npos; at++) sums++;
+    o << " warp_sums=" << sums << " " << p.explain;
     return o.str();
 }
 
@@ -95,6 +97,27 @@ int64_t probe_out_pool(int n, int64_t bytes, int64_t lend_most, int32_t* lent) {
             }
         }
         return (int64_t)pool.bytes();
+    } catch (const std::exception&) {
+        return -1;
+    }
+}
+
+// The kernel for group tables too large for a slot and a sign in a word, for a
+// plan compiled here or (probe_widen) a prepared one.
+int probe_agg_wide(void* t, const vexq_agg_plan_desc* d, char* out, int cap) {
+    try {
+        std::unique_ptr<Plan> p(compile_agg((Table*)t, d));
+        widen_slots(*p);
+        return put(show(*p), out, cap);
+    } catch (const std::exception& e) {
+        return put(std::string("error ") + e.what(), out, cap);
+    }
+}
+
+int probe_widen(vexq_plan_s* h) {
+    try {
+        widen_slots(*h->p);
+        return 0;
     } catch (const std::exception&) {
         return -1;
     }

@@ -39,6 +39,8 @@ class Probe:
         L.probe_filter_key.argtypes = [C.c_void_p, C.c_void_p, C.c_int, C.c_void_p, C.c_int, C.c_int, C.c_char_p, C.c_int]
         L.probe_out_pool.restype = C.c_int64
         L.probe_out_pool.argtypes = [C.c_int, C.c_int64, C.c_int64, C.c_void_p]
+        L.probe_agg_wide.argtypes = [C.c_void_p, C.c_void_p, C.c_char_p, C.c_int]
+        L.probe_widen.argtypes = [C.c_void_p]
         L.probe_join.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p, C.c_char_p, C.c_int]
         self.tables = []
 
@@ -52,6 +54,16 @@ class Probe:
         out = C.create_string_buffer(8192)
         self.lib.probe_agg(table, C.byref(plan.desc), out, len(out))
         return out.value.decode(errors="replace")
+
+    def agg_wide(self, table, plan) -> str:
+        """agg, with the kernel for tables of 2^31 - 1 slots or more."""
+        out = C.create_string_buffer(8192)
+        self.lib.probe_agg_wide(table, C.byref(plan.desc), out, len(out))
+        return out.value.decode(errors="replace")
+
+    def widen(self, op) -> None:
+        """Gives a prepared plan that kernel."""
+        assert self.lib.probe_widen(op.h) == 0
 
     def join(self, build_table, probe_table, plan) -> str:
         out = C.create_string_buffer(8192)

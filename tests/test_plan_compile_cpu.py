@@ -68,3 +68,14 @@ def test_a_kept_filter_plan_is_keyed_by_its_expression(probe):
     assert probe.filter_key(t, date, {0: b"stray"}) == probe.filter_key(t, date)
     keys = [probe.filter_key(t, p) for p in (number, P.col(0) < 8, P.col(0) <= 7, date, P.col(1) < P.lit("1994-01-02"))]
     assert len(set(keys)) == len(keys)
+
+
+@pytest.mark.parametrize("tune,places", [("", 2), ("staged=1", 3)])
+def test_a_hashed_kernel_holds_its_update_twice(probe, monkeypatch, tune, places):
+    # where rows lie and out of the queue; a third copy for the queue's rest was
+    # a quarter of the plan's compile time (the staged loop has no step for it)
+    monkeypatch.setenv("VEXQ_TUNE", tune)
+    t = probe.table([column(abi.TYPE_INT64, lo=-2 ** 62, hi=2 ** 62), column(abi.TYPE_FLOAT64, True, lo=-9, hi=9)], 100_000)
+    plan = P.AggPlan(P.col(1) < 5.0, [0], [P.sum_(P.col(1), "s"), P.count_star("n")])
+    assert f"warp_sums={places} " in probe.agg(t, plan)
+    assert f"warp_sums={places} " in probe.agg_wide(t, plan)

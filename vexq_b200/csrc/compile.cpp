@@ -1510,11 +1510,12 @@ void emit_regs_flush(std::ostringstream& os, const Plan& p, int block, const Flu
     if (fused) os << "    }\n";
 }
 
-// A converged warp's rows added to their slots' float sum s (vq_w_fx_add).
+// A converged warp's rows added to their slots' float sum s (vq_w_fx_add;
+// flags: finite, signed).
 void emit_warp_sum(std::ostringstream& os, const Plan& p, size_t s, const std::string& in, const std::string& flags, const std::string& on,
                    const std::string& slot, const std::string& value) {
     const std::string at = std::to_string(p.slot_pos[s]) + " * ((long long)P.cap + 1)";
-    os << in << "vq_w_fx_add" << flags << "(" << on << ", " << slot << ", P.cap, P.acc_fx + " << at << " * 4, P.special + " << at << ", "
+    os << in << "vq_w_fx_add<" << flags << ">(" << on << ", " << slot << ", P.acc_fx + " << at << " * 4, P.special + " << at << ", "
        << value << ", P.fx_lsb[" << p.slot_pos[s] << "], P.error);\n";
 }
 
@@ -1604,9 +1605,9 @@ CacheField cache_fields(const Plan& p) {
 }
 std::string cache_word(int k) { return "vq_a4 + " + std::to_string(k) + "u * vq_s4"; }
 
-// Template arguments of float sum s's adds (up: the last one, "" none).
-std::string fx_flags(const Plan& p, size_t s, const std::string& up = "") {
-    return std::string("<") + (slot_finite(p, s) ? "true" : "false") + ", " + (slot_signed(p, s) ? "true" : "false") + (up.empty() ? "" : ", " + up) + ">";
+// Template arguments of float sum s's adds: finite, signed.
+std::string fx_flags(const Plan& p, size_t s) {
+    return std::string(slot_finite(p, s) ? "true" : "false") + ", " + (slot_signed(p, s) ? "true" : "false");
 }
 // The limbs' window lies in the digits' window so that both end where the values do.
 std::string limbs_up(const Plan& p) { return std::to_string(VQ_FX_HEAD - p.fx_head); }
@@ -1656,7 +1657,7 @@ void emit_cache_update(std::ostringstream& os, const Plan& p, const std::string&
             case S_NN: os << in << iff << "vq_s_add(" << w << ", 1u);\n"; break;
             case S_ISUM: os << in << iff << "vq_s_add64(" << w << ", " << cache_word(F.at[s] + 1) << ", (unsigned long long)" << SV << ");\n"; break;
             case S_FSUM:
-                os << in << iff << "vq_s_fx_add" << fx_flags(p, s, limbs_up(p)) << "(" << w << ", vq_s4, " << SV << ", P.fx_lsb[" << p.slot_pos[s] << "], P.error);\n";
+                os << in << iff << "vq_s_fx_add<" << fx_flags(p, s) << ", " << limbs_up(p) << ">(" << w << ", vq_s4, " << SV << ", P.fx_lsb[" << p.slot_pos[s] << "], P.error);\n";
                 break;
             default: break;
         }
@@ -1704,7 +1705,7 @@ void emit_table_update(std::ostringstream& os, const Plan& p, const std::string&
             case S_FMAX: os << in << "if (sok" << S << " && !isnan(" << SV << ")) atomicMax(" << aiu << ", vq_fkey(" << SV << "));\n"; break;
             case S_FSUM:
                 if (!sums) break;
-                os << in << iff << "vq_g_fx_add" << fx_flags(p, s, p.path == AggPath::Dense ? limbs_up(p) : "0") << "(P.acc_fx + ((long long)" << pos << " * stride + (long long)slot) * 4, P.special + (long long)"
+                os << in << iff << "vq_g_fx_add<" << fx_flags(p, s) << ", " << (p.path == AggPath::Dense ? limbs_up(p) : "0") << ">(P.acc_fx + ((long long)" << pos << " * stride + (long long)slot) * 4, P.special + (long long)"
                    << pos << " * stride + slot, " << SV << ", P.fx_lsb[" << pos << "], P.error);\n";
                 break;
         }
@@ -1847,8 +1848,10 @@ std::string seg_lookup(const std::string& c, const std::string& s0, const std::s
 
 // block_steps (a kernel with the group cache): every warp of the block walks the
 // same number of steps, counted in vq_step, the ones past the last chunk
-// without a row, so the block can meet between them.
-void chunk_loop_open(std::ostringstream& os, const Plan& p, const Table* t, const std::set<int>& cols, bool block_steps = false) {
+// without a row, so the block can meet between them. last_step: every warp walks
+// one step more, without a row (vq_more is false in it), for what its queue holds.
+void chunk_loop_open(std::ostringstream& os, const Plan& p, const Table* t, const std::set<int>& cols, bool block_steps = false,
+                     bool last_step = false) {
     os << "    const int lane = threadIdx.x & 31;\n"
           "    const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;\n"
           "    long long c = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;\n";
@@ -1856,8 +1859,9 @@ void chunk_loop_open(std::ostringstream& os, const Plan& p, const Table* t, cons
         os << "    int vq_step = 0;\n"
               "    const long long vq_cb = ((long long)blockIdx.x * blockDim.x) >> 5;\n";
     const std::string loop = block_steps ? "    for (long long cb = vq_cb; cb < P.nchunks; cb += nw, c += nw, vq_step++) {\n"
-                                         : "    for (; c < P.nchunks; c += nw) {\n";
-    const std::string row = block_steps ? "        if (c < P.nchunks) {\n" : "";
+                           : last_step ? "    for (bool vq_more = true; vq_more; c += nw) {\n        vq_more = c < P.nchunks;\n"
+                                       : "    for (; c < P.nchunks; c += nw) {\n";
+    const std::string row = block_steps ? "        if (c < P.nchunks) {\n" : last_step ? "        if (vq_more) {\n" : "";
     if (!p.pipeline) {
         os << loop << row << "        long long s0 = 0, s1 = 0, r0 = 0;\n        " << seg_lookup("c", "s0", "s1", "r0");
         emit_loads(os, p, t, cols, "cv", "cm", "r0", "        ", true);
@@ -1990,15 +1994,15 @@ void staged_loop_close(std::ostringstream& os, const StageLayout& L, const std::
 }
 
 // Closes the chunk loop: in the pipelined one the prefetched chunk becomes the
-// current one. With block_steps the caller emits what the block does between
-// steps and the loop's closing brace.
-void chunk_loop_close(std::ostringstream& os, const Plan& p, const Table* t, const std::set<int>& cols, bool block_steps = false) {
-    if (block_steps) os << "        }\n";
+// current one. With rest (block_steps, last_step) the caller emits what follows a
+// step's rows and the loop's closing brace.
+void chunk_loop_close(std::ostringstream& os, const Plan& p, const Table* t, const std::set<int>& cols, bool rest = false) {
+    if (rest) os << "        }\n";
     if (p.pipeline) {
         emit_copy_regs(os, t, cols, "        ");
         os << "        s0 = ns0; s1 = ns1; r0 = nr0;\n";
     }
-    if (!block_steps) os << "    }\n";
+    if (!rest) os << "    }\n";
 }
 
 
@@ -2096,7 +2100,7 @@ struct ScanLoop {
     AsyncLayout A;
     std::string issue;
     bool staged;
-    bool block_steps = false;  // chunk loop of a kernel with the group cache (chunk_loop_open)
+    bool block_steps = false, last_step = false;  // chunk loop of a kernel with the group cache, with a queue (chunk_loop_open)
     int async_n = 0;
     int warps = 8;
     ScanLoop(const Plan& pp, const Table* tt, const std::set<int>& cc, int block, const std::string& name, bool allow_async = false)
@@ -2110,6 +2114,7 @@ struct ScanLoop {
             A = async_layout(t, cols);
         }
     }
+    bool chunks() const { return !staged && async_n == 0; }  // the chunk loop
     int tile_rows() const { return staged ? L.T : 128; }
     // lane l holds rows l + 32k of a chunk (the cp.async pipeline) rather than 4l + k
     bool strided() const { return !staged && async_n > 0; }
@@ -2121,12 +2126,12 @@ struct ScanLoop {
     void open(std::ostringstream& os) const {
         if (staged) staged_loop_open(os, t, cols, L, issue);
         else if (async_n) async_loop_open(os, t, cols, A, async_n, issue);
-        else chunk_loop_open(os, p, t, cols, block_steps);
+        else chunk_loop_open(os, p, t, cols, block_steps, last_step);
     }
     void close(std::ostringstream& os) const {
         if (staged) staged_loop_close(os, L, issue);
         else if (async_n) async_loop_close(os);
-        else chunk_loop_close(os, p, t, cols, block_steps);
+        else chunk_loop_close(os, p, t, cols, block_steps || last_step);
     }
 };
 
@@ -2280,9 +2285,6 @@ static void emit_hash_rows(std::ostringstream& os, Plan& p, const std::vector<in
     Gen g(p, os);
     emit_hash_update(os, p, g, "            ");
     os << "        }\n";
-    os << "        while (vq_qn >= 32) {\n";
-    emit_hash_take(os, p);
-    os << "        }\n";
 }
 
 // Generates the aggregate scan kernel (table → filter → project → aggregate).
@@ -2302,16 +2304,26 @@ static std::string gen_agg_kernel(Plan& p, const std::vector<int>& key_nodes, in
     if (p.path == AggPath::Regs) emit_regs_decl(os, p);
     if (p.smem_groups > 0) emit_cache_init(os, p);
     if (hash_queue(p, block)) emit_hash_queue_decl(os, block);
-    loop.block_steps = p.smem_groups > 0;
-    loop.open(os);
     const bool queue = hash_queue(p, block);
+    loop.block_steps = p.smem_groups > 0;
+    loop.last_step = queue && loop.chunks();
+    loop.open(os);
+    auto take = [&](const std::string& until) {
+        os << "        while (vq_qn >= " << until << ") {\n";
+        emit_hash_take(os, p);
+        os << "        }\n";
+    };
     if (queue) emit_hash_rows(os, p, key_nodes);
     else emit_agg_rows(os, p, key_nodes, p.smem_groups > 0, loop.strided());
+    // (one loop takes the queue in the last step too: the update behind it is
+    // long, and compiling it a second time took 0.1 to 0.3 s of a plan's 0.4 to 1.3)
+    if (queue && !loop.last_step) take("32");
     loop.close(os);
-    if (queue) {
-        os << "    while (vq_qn > 0) {\n";
-        emit_hash_take(os, p);
+    if (loop.last_step) {
+        take("(vq_more ? 32 : 1)");
         os << "    }\n";
+    } else if (queue) {
+        take("1");
     }
     if (loop.block_steps) {
         emit_cache_norm(os, p, block, "vq_step");
@@ -2798,7 +2810,7 @@ static void emit_probe_matches(std::ostringstream& os, Plan& p, const std::vecto
     os << "                } while (false);\n";
     for (size_t s = 0; s < p.slots.size(); s++)
         if (p.slots[s].kind == S_FSUM)
-            emit_warp_sum(os, p, s, "                ", "<false, true>", "vq_o" + std::to_string(s), "vq_t", "vq_v" + std::to_string(s));
+            emit_warp_sum(os, p, s, "                ", "false, true", "vq_o" + std::to_string(s), "vq_t", "vq_v" + std::to_string(s));
     os << "            }\n";
 }
 

@@ -309,13 +309,13 @@ __device__ __forceinline__ void vq_g_fx_add(vq_i64* c, unsigned* sp, double x, i
 // top digits in one instruction: they lie in one 16-byte half of a sector, and
 // the L2 adds both in the time of one (4.0M rows, random slots: one counter a row
 // 27 us, two by the same lane 50, two by neighbouring lanes 27). The window ends
-// where the largest values do, so the top 11 binades have no other digit.
+// where the largest values do, so the top 11 binades have no other digit. A
+// kernel for tables of VQ_WIDE_SLOTS slots or more is compiled with VQ_WIDE.
 template <bool kFinite, bool kSigned>
-__device__ __forceinline__ void vq_w_fx_add(bool on, vq_u64 slot, vq_u64 cap, vq_i64* c, unsigned* sp, double x, int lsb, int* err) {
-    if (cap >= 0x7FFFFFFFull) {  // slot and sign do not fit a word
-        if (on) vq_g_fx_add<kFinite, kSigned, 0>(c + slot * 4, sp + slot, x, lsb, err);
-        return;
-    }
+__device__ __forceinline__ void vq_w_fx_add(bool on, vq_u64 slot, vq_i64* c, unsigned* sp, double x, int lsb, int* err) {
+#ifdef VQ_WIDE
+    if (on) vq_g_fx_add<kFinite, kSigned, 0>(c + slot * 4, sp + slot, x, lsb, err);
+#else
     unsigned mh = 0u, lo = 0u, special = 0u;
     int sh = 0;
     if (on && !vq_fx_image<kFinite, VQ_FX_WINDOW>(x, lsb, mh, lo, sh, special, err)) {
@@ -340,6 +340,7 @@ __device__ __forceinline__ void vq_w_fx_add(bool on, vq_u64 slot, vq_u64 cap, vq
         if (b1) atomicAdd(q + 1, neg ? 0ull - b1 : (vq_u64)b1);
         if (b0) atomicAdd(q, neg ? 0ull - b0 : (vq_u64)b0);
     }
+#endif
 }
 
 __device__ __host__ inline int vq_clz64(vq_u64 x) {

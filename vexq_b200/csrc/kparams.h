@@ -8,6 +8,7 @@
 #define VQ_FX_DIGITS 4  // 32-bit digits of the exact fixed-point float sums
 #define VQ_FX_WINDOW 128  // bits of a group table's window: |x| < 2^(lsb + 128)
 #define VQ_FX_HEAD 31     // bits left free above the largest values where more than 2^31 rows may meet in a sum
+#define VQ_WIDE_SLOTS 0x7FFFFFFFll  // slots from which a slot and a sign do not fit a word (vq_w_fx_add)
 #define VQ_MAXLITS 32   // numeric literals passed at launch (raw 8-byte images)
 #define VQ_RADIX_CAP 4096      // radix join: build entries of one partition held in shared memory
 #define VQ_RADIX_MAX_BITS 12   // radix join: at most 4,096 partitions

@@ -250,6 +250,7 @@ struct Plan {
     ScanMemo build_memo;                   // join build side's pruning (whole table), until its zone maps change
     long long hash_groups_seen = -1;       // hash path: groups the last run found (sizes the next table)
     long long hash_rows_seen = 0;          //   and the rows that run scanned
+    bool wide_slots = false;               // the main kernel is the one for tables of VQ_WIDE_SLOTS slots or more (widen_slots)
     // group tables assembled on the device (assemble.cu)
     OutPool out_pool;
     DevBuf d_asm, asm_bits, asm_scr;       // descriptor and columns; first-row bitmap; positions
@@ -338,6 +339,10 @@ struct SelectLease {
     void done();
 };
 void ensure_events(Plan& p);
+// Compiles the plan's main kernel anew for group tables of VQ_WIDE_SLOTS slots
+// or more. Held in every kernel beside the other, the code for them was a third
+// of what a hashed plan compiles (0.86 against 1.26 s, 7 float sums).
+void widen_slots(Plan& p);
 // Copies the plan's launch-time constants (literals, float-sum windows, cache size) into P.
 void set_plan_constants(const Plan& p, VQParams& P);
 // Fails when a table the plan reads was re-filled with values outside the

@@ -1224,6 +1224,13 @@ static void compact_table(RunCtx& rc, Compacted& c) {
     if (!P.clk) VQ_CUDA(cudaEventRecord(p.ev[3], rc.s));
 }
 
+void widen_slots(Plan& p) {
+    const std::string src = "#define VQ_WIDE 1\n" + p.src_main;
+    p.k_main = jit_get(src, "vq_agg", p.block, p.smem);
+    p.src_main = src;
+    p.wide_slots = true;
+}
+
 // A deferred run (defer set) launches the scan and returns without waiting or
 // compacting: the caller's top-k launches read the table where it lies, and
 // their output brings the group count and the error word.
@@ -1306,6 +1313,7 @@ Compacted run_atomic(RunCtx& rc, VQParams& P, long long nchunks, long long estim
         launch_check(rc.s, "k_init_table");
         bind_distinct(p, P, nchunks * 128, rc.s);
         VQ_CUDA(cudaGetLastError());
+        if (nslots >= VQ_WIDE_SLOTS && !p.wide_slots && !rc.k) widen_slots(p);
         const JitKernel& K = rc.k ? *rc.k : p.k_main;
         int grid = rc.k ? rc.grid : grid_for(p.k_main, nchunks, p.staged);
         mark(p.ev[1]);
