@@ -91,7 +91,7 @@ int64_t probe_out_pool(int n, int64_t bytes, int64_t lend_most, int32_t* lent) {
         for (int i = 0; i < n; i++) {
             bool lend = false;
             std::shared_ptr<OutBlock> b = pool.acquire((size_t)bytes, lend);
-            if (lend) {
+            if (b && lend) {
                 held.push_back(b);
                 ++*lent;
             }

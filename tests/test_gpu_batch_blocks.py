@@ -1,5 +1,6 @@
-"""GPU tests of the pinned blocks batches write their group tables' columns to:
-above a size one block serves every execution and results copy their rows."""
+"""GPU tests of the pinned blocks the device writes result columns to: above a
+size a batch keeps one for every execution and its results copy their rows, and a
+block that cannot be pinned is no error."""
 from __future__ import annotations
 
 import numpy as np
@@ -43,3 +44,11 @@ def test_results_of_a_large_batch_held_over_executions(gpu_lib):
             assert [tuple(r) for r in res.rows()] == rows
     for x in ops + tables:
         x.close()
+
+
+def test_a_block_that_cannot_be_pinned_is_none(gpu_lib, tmp_path):
+    # the caller then takes the way that needs no block (2^46 bytes: more than the address space holds)
+    probe = Probe(str(tmp_path))
+    assert probe.out_pool(2, 1 << 46, 1 << 62) == (0, 0)
+    assert probe.out_pool(2, 1 << 20, 1 << 62)[1] == 2
+    probe.close()

@@ -569,7 +569,7 @@ struct Batch {
         blk.reset();
         pool.lend_most = kLendMost;
         blk = pool.acquire(asm_bytes, blk_lend);
-        if (!blk) fail(VEXQ_EDEVICE, "pinned host memory has no device address");
+        if (!blk) fail(VEXQ_ENOMEM, "no pinned host memory with a device address for the batch's results");
         if (blk->dev == blk_sent) return;
         h2d((char*)dev.p + a_outp, &blk->dev, 8, s);
         blk_sent = blk->dev;

@@ -131,8 +131,8 @@ struct OutPool {
     size_t lend_most = ~(size_t)0;
     std::vector<std::shared_ptr<OutBlock>> lent;
     std::shared_ptr<OutBlock> stage;
-    // A block of at least `bytes`, null where pinned memory has no device
-    // address; lend tells whether the result may keep it.
+    // A block of at least `bytes`, null where none can be pinned or pinned memory
+    // has no device address; lend tells whether the result may keep it.
     std::shared_ptr<OutBlock> acquire(size_t bytes, bool& lend);
     void trim(size_t most);  // drops blocks of more than `most` bytes (a result that holds one keeps it)
     size_t bytes() const;    // of its blocks, lent or not

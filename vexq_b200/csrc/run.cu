@@ -810,7 +810,12 @@ std::shared_ptr<OutBlock> OutPool::acquire(size_t bytes, bool& lend) {
     auto fit = [&](OutBlock& b) {
         if (b.pin.n >= bytes) return;
         b.dev = nullptr;
-        b.pin.ensure(bytes);
+        try {
+            b.pin.ensure(bytes);
+        } catch (const Status&) {  // no such block to be had: the result goes the way that needs none
+            (void)cudaGetLastError();
+            return;
+        }
         void* d = nullptr;
         if (cudaHostGetDevicePointer(&d, b.pin.p, 0) == cudaSuccess) b.dev = (char*)d;
         else (void)cudaGetLastError();
