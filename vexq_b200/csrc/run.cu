@@ -176,7 +176,9 @@ __global__ void k_finalize(const unsigned long long* keys, const long long* firs
         if (occ) finalize_write(i, pos, keys, first, acc_i, acc_fx, special, nslots, ni, nf, fx_lsb, hash, o_key, o_first,
                                 o_i, o_f, cap_out, kst);
     }
-    if (clk && threadIdx.x == 0) atomicMax(clk + VQ_CLK_END, vq_clock());
+    if (!clk) return;
+    __syncthreads();  // the block's last writes are in its end
+    if (threadIdx.x == 0) atomicMax(clk + VQ_CLK_END, vq_clock());
 }
 
 // Batched group tables: global slot g belongs to the table whose slot0 is the
