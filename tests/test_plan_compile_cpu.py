@@ -2,10 +2,16 @@
 compiled for sm_100a as on a GPU host and not loaded."""
 from __future__ import annotations
 
+import os
+import subprocess
+import sys
+
 import pytest
 
 from tests.plan_probe import Probe, abi, column, lsb
 from vexq_b200 import plan as P
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
 @pytest.fixture(scope="module")
@@ -79,3 +85,22 @@ def test_a_hashed_kernel_holds_its_update_twice(probe, monkeypatch, tune, places
     plan = P.AggPlan(P.col(1) < 5.0, [0], [P.sum_(P.col(1), "s"), P.count_star("n")])
     assert f"warp_sums={places} " in probe.agg(t, plan)
     assert f"warp_sums={places} " in probe.agg_wide(t, plan)
+
+
+def test_float_min_max_plans_stay_in_their_arrays(tmp_path):
+    # in a process of its own whose allocator checks every block it frees
+    code = f"""
+from tests.plan_probe import Probe, abi, column
+from vexq_b200 import plan as P
+probe = Probe({str(tmp_path)!r})
+cols = [column(abi.TYPE_INT64, lo=0, hi=999)] + [column(abi.TYPE_FLOAT64, lo=-9, hi=9) for _ in range(6)]
+t = probe.table(cols, 100_000)
+for k in range(1, 7):
+    aggs = [f(P.col(1 + i), f"a{{i}}{{f.__name__}}") for i in range(k) for f in (P.min_, P.max_)]
+    assert "path=dense" in probe.agg(t, P.AggPlan(None, [0], aggs))
+    assert "path=dense" in probe.agg(t, P.AggPlan(None, [0], aggs + [P.sum_(P.col(1), "s")]))
+print("fine")
+"""
+    env = dict(os.environ, VEXQ_JIT_CACHE=str(tmp_path / "jit"), LD_PRELOAD="libc_malloc_debug.so.0", MALLOC_CHECK_="3")
+    r = subprocess.run([sys.executable, "-c", code], env=env, capture_output=True, text=True, cwd=ROOT)
+    assert r.returncode == 0 and "fine" in r.stdout, (r.returncode, r.stderr[-500:])

@@ -3251,7 +3251,8 @@ static std::string gen_kind_tables(const Plan& p, const std::string& prefix) {
     for (size_t s = 0; s < p.slots.size(); s++) {
         int k = p.slots[s].kind;
         int code = (k == S_IMIN || k == S_FMIN) ? 1 : (k == S_IMAX || k == S_FMAX) ? 2 : 0;
-        if (p.slots[s].is_float()) fk[p.slot_pos[s]] = code;
+        // (a group table keeps float MIN and MAX in its integer bank, as order keys)
+        if (p.path == AggPath::Regs ? p.slots[s].is_float() : p.slots[s].kind == S_FSUM) fk[p.slot_pos[s]] = code;
         else ik[p.slot_pos[s]] = code;
     }
     ik[p.ni] = 1;  // first-occurrence key: min
