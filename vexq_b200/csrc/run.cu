@@ -979,7 +979,7 @@ static RegsPending regs_launch(RunCtx& rc, VQParams& P, long long nchunks, bool 
         P.merr_out = err_out;
         P.mdone = p.mdone.as<unsigned>();
     }
-    bind_distinct(p, P, nchunks * 128, rc.s);
+    bind_distinct(p, P, nchunks * p.tile, rc.s);
     // the run's launches: the scan, which stamps the device clock; or a start
     // event, the scan, its merge and an end event (recorded as external nodes
     // when captured, so a replayed graph still times them; plain records when
@@ -1318,7 +1318,7 @@ Compacted run_atomic(RunCtx& rc, VQParams& P, long long nchunks, long long estim
         k_init_table<<<ig, 256, 0, rc.s>>>(P.keys, P.first, P.acc_i, ni, d_iv, P.acc_fx, P.special, nf, nslots, hash, P.ngroups,
                                           P.error, n_out, P.clk);
         launch_check(rc.s, "k_init_table");
-        bind_distinct(p, P, nchunks * 128, rc.s);
+        bind_distinct(p, P, nchunks * p.tile, rc.s);
         VQ_CUDA(cudaGetLastError());
         if (nslots >= VQ_WIDE_SLOTS && !p.wide_slots && !rc.k) widen_slots(p);
         const JitKernel& K = rc.k ? *rc.k : p.k_main;
