@@ -203,7 +203,9 @@ def batch_leg(nplans, steps, warmup, peak, cpu=True):
     """One step = every plan of the batching workload. The batched arm (one
     persistent launch per path class, graph replay, autotuned) against the
     same plans one by one through vexq_plan_run; device time is the kernels
-    alone (the device clock inside the library, before the copy back). The CPU
+    alone: the batch's graph between CUDA events on its stream, with the group
+    tables' results written over PCIe and before the copy back of the rest; the
+    plans one by one by the device clock inside their kernels. The CPU
     figure is one pass of the C++ restatement of ParallelHashAggregate over
     every plan on all host threads."""
     from vexq_b200 import exec as X

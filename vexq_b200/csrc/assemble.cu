@@ -271,9 +271,12 @@ bool asm_plan_ok(const Plan& p) {
 }
 
 // Tables of up to 2^20 slots and scans of up to 2^28 rows: one cluster passes
-// over the slots twice and over a bit a row three times, about 10 us at either
-// limit; above them the compaction over the whole GPU and the host's ordering
-// stay.
+// over the slots twice and over a bit a row three times. 1,000,000 groups take 634
+// us behind the scan, most of it their way over PCIe (a run 0.70 ms; 120 ms with
+// the compaction over the whole GPU and the host's ordering). 4,000 groups of 2^24,
+// 2^26 and 2^28 rows take 29, 74 and 242 us (runs 74, 191 and 631; by the other
+// way 424, 473 and 754): about where one cluster's passes over the bits cost what
+// they save.
 bool asm_run_ok(const Plan& p, long long nslots, long long row0, long long row1) {
     return asm_plan_ok(p) && nslots <= (1LL << 20) + 1 && row1 - row0 <= (1LL << 28);
 }

@@ -3302,6 +3302,12 @@ static void choose_tunables(Plan& p) {
     // warps as three 128-thread blocks, a third of the partials) gave 63.2-63.7
     // against 64.2-65.1 us in one process and 67 against 63 us in the bench
     // loop; it stays a tunable (block=384)
+    // 4M Zipf(1.1) rows, scan us with 48 / 96 / 160 / 190 KB of cache. SUM COUNT MIN MAX
+    // AVG: 4,000 groups 44.4 / 42.9 / 44.0 / 43.8, 20,000 82.9 / 46.8 / 48.1 / 48.6,
+    // 65,536 71.0 / 59.8 / 51.8 / 52.4; SUM COUNT: 34.5 / 30.1 / 29.2 / 29.2, 39.9 / 31.9 /
+    // 34.2 / 35.2, 40.6 / 33.9 / 35.0 / 35.7 (1,000 groups fit 96 KB: 33.3 and 22.3).
+    // More entries than the frequent groups need cost their set-up and flush in
+    // every block; a batch, whose blocks take several units a plan, has 190
     int cache_kb = 96;
     if (const char* e = std::getenv("VEXQ_TUNE")) {
         std::string s(e);
