@@ -2508,6 +2508,7 @@ vexq_result_s* run_plan(Plan& p, int rg_start, int rg_end) {
                     std::vector<long long> soff(nlong);
                     long long tot = 0;
                     for (int i = 0; i < nlong; i++) {
+                        chain_most = std::max(chain_most, (double)lst[i].y);
                         long long m = 1;
                         while (m < lst[i].y) m <<= 1;
                         soff[i] = tot;
@@ -2520,6 +2521,7 @@ vexq_result_s* run_plan(Plan& p, int rg_start, int rg_end) {
                     launch_check(rc.s, "k_sort_long");
                     rc.launches += 1;
                 }
+                chain_most = std::max(chain_most, (double)kShortChain);  // of the chains not in the list
                 rc.launches += 5;
             }
             k_pack_slots<<<(int)std::min<long long>((nslots + 1023) / 1024, (long long)sm_count() * 16), 256, 0, rc.s>>>(
@@ -2542,7 +2544,6 @@ vexq_result_s* run_plan(Plan& p, int rg_start, int rg_end) {
             p.gid_groups = join_keys;
             p.join_keys_seen = join_keys;
             p.join_rows_seen = bs.rows;
-            if (!unique) chain_most = (double)(ntot - nk + 1);
         }
         break;
         }
