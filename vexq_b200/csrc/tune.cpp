@@ -122,7 +122,7 @@ extern "C" int32_t vexq_plan_autotune(vexq_plan_t plan, uint32_t flags, int32_t*
             cands = {0, 6, 8, 10, 12};
             if (!p.radix) cands = {0};
         } else if (p.path == AggPath::Dense) {
-            cands = {0, 48, 96, 160};
+            cands = {0, 48, 96, 160};  // (160 and 190 KB measure alike, choose_tunables)
         } else {
             if (out_choice) *out_choice = -1;  // nothing launch-time to choose on this path
             if (out_ms) *out_ms = 0;
